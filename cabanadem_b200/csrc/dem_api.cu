@@ -104,6 +104,7 @@ struct dem_solver {
     bool coop_refused = false;                  // a cooperative launch of the step loop was refused
     bool coop_ran = false;                      // the last run's steps ran in cooperative launches
     unsigned long long *d_coop = nullptr;       // kCoopScratch words: barrier counter and slots
+    RefTables ref{};                            // cell tables of the rebuild-every-step loop
 };
 
 struct dem_bonds {
@@ -1418,6 +1419,9 @@ extern "C" int dem_solver_destroy(dem_solver *s) {
     cudaFree(B.part_sums);
     cudaFree(s->d_epart); cudaFree(s->d_eout);
     cudaFree(s->d_coop);
+    cudaFree(s->ref.count);
+    cudaFree(s->ref.item);
+    cudaFree(s->ref.key);
     free_mesh(s);
     delete s;
     return DEM_OK;
@@ -1565,6 +1569,71 @@ bool coop_loop(const dem_solver *s) {
            s->loop && !ref_mode(s);
 }
 
+// The rebuild-every-step mode's run in one cooperative launch (dem_refloop.cuh): the one-kernel
+// step of a small system without batched scenes, static walls, no mesh.
+bool ref_loop(const dem_solver *s) {
+    return ref_mode(s) && s->sp.cooperative_loop != 2 && !s->coop_refused && s->fc.all == 1 &&
+           s->p->P.n <= kCoopMaxN && s->loop && !s->fc.mwalls && s->mesh_nt == 0 && !s->p->P.scene && s->nscenes == 0 &&
+           s->p->P.mc <= kCoopSlots;
+}
+
+int ensure_ref_tables(dem_solver *s) {
+    if (s->ref.count) return DEM_OK;
+    dem_ctx *ctx = s->ctx;
+    RefTables &R = s->ref;
+    R.grid = s->B.grid;
+    R.total = s->B.total;
+    R.codes = s->B.cell_cap;
+    CK(dalloc(&R.item, 3 * (size_t)R.codes * kRefCell));
+    CK(dalloc(&R.key, 3 * (size_t)s->p->P.cap));
+    CK(dalloc(&R.count, 3 * (size_t)R.codes));
+    return DEM_OK;
+}
+
+// Steps of a run in the rebuild-every-step mode, as many as the cooperative launch takes.
+// *left: steps the graph of build and step kernels has to do.
+int run_ref_loop(dem_solver *s, int nsteps, bool *left) {
+    dem_ctx *ctx = s->ctx;
+    cudaStream_t st = ctx->stream;
+    *left = true;
+    int e = ensure_ref_tables(s);
+    if (e) return e;
+    if (!s->d_coop) CK(dalloc(&s->d_coop, (size_t)kCoopScratch));
+    s->ref.grid = s->B.grid;
+    for (int done = 0;;) {
+        launch_ref_grid(s->p->P, s->B, s->p->ctl, s->sp.delta, s->sp.skin, st);
+        const cudaError_t le = launch_steps_ref(s->p->P, s->L, s->p->ctl, s->fc, s->d_pp, s->d_pw, s->d_walls, s->ref,
+                                                s->sp.delta, s->sp.skin, nsteps, s->d_coop, st);
+        if (le != cudaSuccess) {   // not resident at once (or refused): the graph from here on
+            (void)cudaGetLastError();
+            s->coop_refused = true;
+            return DEM_OK;
+        }
+        s->launches += 6;
+        const Ctl c = read_ctl(s);
+        CK(cudaGetLastError());
+        if (c.status & DEM_ERR_TIMEOUT) return fail(ctx, DEM_ERR_TIMEOUT, "a bounded device wait gave up");
+        if (c.steps_done > done) s->coop_ran = true;
+        if (c.status & DEM_ERR_NEIGHBOR_OVERFLOW) {   // the step was done, its list did not fit
+            if (c.max_nbr > 128) return fail(ctx, DEM_ERR_NEIGHBOR_OVERFLOW, "more than 128 neighbours");
+            e = alloc_lists(s, std::min(std::max(2 * s->L.maxnb, c.max_nbr + 8), 128));
+            if (e) return e;
+            k_clear_status<<<1, 32, 0, st>>>(s->p->ctl, DEM_ERR_NEIGHBOR_OVERFLOW);
+            if (c.steps_done >= c.target) {   // the lists of the last step, in full
+                launch_build(s->p->P, s->p->alt, s->L, s->B, s->p->ctl, s->sp.delta, s->sp.skin, false, true, st);
+                s->launches += build_kernel_count(false);
+                CK(cudaGetLastError());
+            }
+        }
+        if (c.steps_done >= c.target) {
+            *left = false;
+            return DEM_OK;
+        }
+        if (c.steps_done == done) return DEM_OK;   // no progress on a fresh grid: the graph
+        done = c.steps_done;
+    }
+}
+
 extern "C" int dem_solver_run(dem_solver *s, int nsteps) {
     if (!s) return DEM_ERR_INVALID;
     if (nsteps <= 0) return DEM_OK;
@@ -1614,9 +1683,15 @@ extern "C" int dem_solver_run(dem_solver *s, int nsteps) {
                                : s->graph_nodes;
         steps_before = c.steps_done;
     };
+    bool graph_steps = ref_mode(s);
+    if (graph_steps) s->coop_ran = false;
+    if (ref_loop(s)) {
+        const int e = run_ref_loop(s, nsteps, &graph_steps);
+        if (e) return e;
+    }
     if (ref_mode(s)) {
         // rebuild before every force pass, inside the graph (no re-sort)
-        for (;;) {
+        while (graph_steps) {
             {
                 int e = ensure_graph();
                 if (e) return e;

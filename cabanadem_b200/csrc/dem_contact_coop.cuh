@@ -28,15 +28,37 @@ __device__ __forceinline__ int nth_high_bit(unsigned b, int r) {
     return 31 - __clz(b);
 }
 
+// Where a particle's list comes from: the solver's list arrays, read once through the read-only
+// path (a launch that does one step), or a list the group holds in shared memory, with the
+// particle's own arrays read by plain loads (a launch whose earlier steps wrote them).
+struct GlobalList {
+    static constexpr bool kOneStep = true;
+    const NbrList &L;
+    const int cap;
+    __device__ __forceinline__ int count(int i) const { return ld_early_i(L.nn + i); }
+    __device__ __forceinline__ int at(int i, int k) const { return L.idx[(long)k * cap + i]; }
+};
+struct GroupList {
+    static constexpr bool kOneStep = false;
+    const int *list;
+    const int n;
+    __device__ __forceinline__ int count(int) const { return n; }
+    __device__ __forceinline__ int at(int, int k) const { return list[k]; }
+};
+
 // Warp-collective: all 32 lanes call it; the groups of lanes [g NL, g NL + NL) each take one
 // particle i (i < 0: no particle, the group still takes part in the warp's shuffles).  t is
 // the particle's deferred slot.  s_tidx / s_h are the group's shared slots.
-template <int NL, bool MIXED, bool MESH = false>
-__device__ __forceinline__ void particle_coop(const Particles &P, const NbrList &L, const ForceConsts &fc,
+// List entries are taken from `list`; new u and omega go to vn, wn at t.  pn_out (may be null)
+// receives the particle's new position on the group's first lane.
+template <int NL, bool MIXED, bool MESH, class LIST>
+__device__ __forceinline__ void particle_coop(const Particles &P, const LIST &list, const ForceConsts &fc,
                                               const PairConst *__restrict__ pp, const PairConst *__restrict__ pw,
                                               const WallGeom *__restrict__ walls, const int cur, const int nxt,
                                               const int vcur, const int last, const int i, const int t,
-                                              int *s_tidx, double *s_h, double &vmax2, int &status) {
+                                              int *s_tidx, double *s_h, double *vn, double *wn, double &vmax2,
+                                              int &status, D4 *pn_out = nullptr) {
+    constexpr bool ONE = LIST::kOneStep;
     constexpr unsigned FULL = 0xffffffffu;
     constexpr unsigned GLOW = NL == 32 ? 0xffffffffu : ((1u << NL) - 1u);
     const int lane = threadIdx.x & 31, gl = lane % NL, gbase = lane - gl;
@@ -51,24 +73,24 @@ __device__ __forceinline__ void particle_coop(const Particles &P, const NbrList 
     const double mu_pp = scn ? scn->mu_pp : fc.mu_pp, mu_pw = scn ? scn->mu_pw : fc.mu_pw;
     const int wall0 = fc.wps ? scene_i * fc.wps : 0;
     const int nwall = act ? (fc.wps ? fc.wps : fc.nwall) : 0;
-    const double4 *__restrict__ pc = P.pos[cur];
-    const double *__restrict__ vc = P.vel[vcur];
-    const double *__restrict__ wc = P.omg[vcur];
+    const double4 *pc = P.pos[cur];
+    const double *vc = P.vel[vcur];
+    const double *wc = P.omg[vcur];
     D4 pi = {0., 0., 0., 0.};
     double ui0 = 0., ui1 = 0., ui2 = 0., wi0 = 0., wi1 = 0., wi2 = 0.;
     double2 mIi = make_double2(0., 0.);
     int mi = 0, cs0 = 0, nn = 0;
     if (act) {
-        pi = ld4_early(pc, i);
-        ui0 = ld_early(vc + i);
-        ui1 = ld_early(vc + cap + i);
-        ui2 = ld_early(vc + 2 * cap + i);
-        wi0 = ld_early(wc + i);
-        wi1 = ld_early(wc + cap + i);
-        wi2 = ld_early(wc + 2 * cap + i);
+        pi = ONE ? ld4_early(pc, i) : ld4(pc, i);
+        ui0 = ONE ? ld_early(vc + i) : vc[i];
+        ui1 = ONE ? ld_early(vc + cap + i) : vc[cap + i];
+        ui2 = ONE ? ld_early(vc + 2 * cap + i) : vc[2 * cap + i];
+        wi0 = ONE ? ld_early(wc + i) : wc[i];
+        wi1 = ONE ? ld_early(wc + cap + i) : wc[cap + i];
+        wi2 = ONE ? ld_early(wc + 2 * cap + i) : wc[2 * cap + i];
         mIi = make_double2(ld_early(P.mI + i), ld_early(P.mI + cap + i));
-        cs0 = ld_early_i(P.cstate + i);
-        nn = ld_early_i(L.nn + i);
+        cs0 = ONE ? ld_early_i(P.cstate + i) : P.cstate[i];
+        nn = list.count(i);
         mi = fc.nmat > 1 ? (int)P.mat[i] : 0;
     }
     const int cnt0 = cs0 & 0xff;
@@ -170,7 +192,7 @@ __device__ __forceinline__ void particle_coop(const Particles &P, const NbrList 
         D4 pj = {0., 0., 0., 0.};
         double px = 0., py = 0., pz = 0., rij = 0., overlap = 0.;
         if (kk < nn) {
-            j = L.idx[(long)kk * cap + i];
+            j = list.at(i, kk);
             pj = ld4(pc, j);
             px = pi.x - pj.x;
             py = pi.y - pj.y;
@@ -351,7 +373,7 @@ __device__ __forceinline__ void particle_coop(const Particles &P, const NbrList 
         vmax2 = dadd(dadd(dmul(ui0, ui0), dmul(ui1, ui1)), dmul(ui2, ui2));
     }
     st4(P.pos[nxt], i, pn);
-    double *vn = L.defer_v, *wn = L.defer_w;
+    if (pn_out) *pn_out = pn;
     vn[t] = ui0;
     vn[cap + t] = ui1;
     vn[2 * cap + t] = ui2;
@@ -390,8 +412,8 @@ __global__ void __launch_bounds__(kBlock, MINB) k_contact_coop(Particles P, NbrL
         const int t = base + grp;
         const int i = t < nd ? L.defer[t] : -1;
         double v2 = 0.0;
-        particle_coop<NL, MIXED, MESH>(P, L, fc, pp, pw, walls, cur, cur ^ 1, vcur, last, i, t, s_tidx[sg], s_h[sg], v2,
-                                 status);
+        particle_coop<NL, MIXED, MESH>(P, GlobalList{L, P.cap}, fc, pp, pw, walls, cur, cur ^ 1, vcur, last, i, t,
+                                       s_tidx[sg], s_h[sg], L.defer_v, L.defer_w, v2, status);
         vmax2 = fmax(vmax2, v2);
     }
     warp_vmax(ctl, P.vslots, vmax2, status);

@@ -231,6 +231,17 @@ struct BuildBuffers {
 
 constexpr int kPartBlock = 256;   // block size of the re-sort's partition kernels
 
+// Cell tables of the rebuild-every-step loop (dem_refloop.cuh): three of `codes` cells each.
+constexpr int kRefCell = 16;      // particles a cell holds
+struct RefTables {
+    const Grid *grid;             // one scene's grid, from launch_ref_grid
+    const int *total;             // its cell keys
+    int codes;                    // cells a table holds
+    int *count;                   // [3][codes]
+    int *item;                    // [3][codes][kRefCell]
+    int *key;                     // [3][cap] cell of each particle's entry
+};
+
 // Bond slots (bonded DEM), slot-major like the contact history.
 constexpr unsigned BQ10_INDEX_BY_J = 0x01u;   // history(i, partner id), BondedDEM_Force.hpp:207, :231-322
 constexpr unsigned BQ11_HARDCODED_K = 0x02u;  // k from E, G and bond area, BondedDEM_Force.hpp:186-198
@@ -329,6 +340,17 @@ cudaError_t launch_steps_coop(const Particles &P, const NbrList &L, Ctl *ctl, co
 cudaError_t launch_steps_coop_mixed(const Particles &P, const NbrList &L, Ctl *ctl, const ForceConsts &fc,
                                     const PairConst *pp, const PairConst *pw, const WallGeom *walls, int max_steps,
                                     unsigned long long *scratch, cudaStream_t s);
+
+// The rebuild-every-step mode's run in one cooperative launch (dem_refloop.cuh): at most
+// `max_steps` steps, ending at the target, or earlier where the build and step kernels have to go
+// on (a full cell, a full list, a position that is not finite).  launch_ref_grid first.
+void launch_ref_grid(const Particles &P, BuildBuffers &B, Ctl *ctl, double delta, double skin, cudaStream_t s);
+cudaError_t launch_steps_ref(const Particles &P, const NbrList &L, Ctl *ctl, const ForceConsts &fc, const PairConst *pp,
+                             const PairConst *pw, const WallGeom *walls, const RefTables &R, double delta, double skin,
+                             int max_steps, unsigned long long *arrive, cudaStream_t s);
+cudaError_t launch_steps_ref_mixed(const Particles &P, const NbrList &L, Ctl *ctl, const ForceConsts &fc,
+                                   const PairConst *pp, const PairConst *pw, const WallGeom *walls, const RefTables &R,
+                                   double delta, double skin, int max_steps, unsigned long long *arrive, cudaStream_t s);
 
 // dense layers of the surrogate (dem_nn.cu)
 int nn_mlp_forward(const dem_nn_mlp &m, long rows, const dem_nn_rows *src, int nsrc, const void *resid, void *out,

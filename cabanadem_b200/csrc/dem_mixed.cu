@@ -10,6 +10,7 @@
 #include "dem_contact_coop.cuh"
 #include "dem_pairs.cuh"
 #include "dem_persist.cuh"
+#include "dem_refloop.cuh"
 #include "dem_scenes.cuh"
 
 namespace b200dem {
@@ -217,6 +218,14 @@ cudaError_t launch_steps_coop_mixed(const Particles &P, const NbrList &L, Ctl *c
                                     unsigned long long *scratch, cudaStream_t s) {
     return fc.mesh.nt ? steps_coop_t<true, true>(P, L, ctl, fc, pp, pw, walls, max_steps, scratch, s)
                       : steps_coop_t<true, false>(P, L, ctl, fc, pp, pw, walls, max_steps, scratch, s);
+}
+
+cudaError_t launch_steps_ref_mixed(const Particles &P, const NbrList &L, Ctl *ctl, const ForceConsts &fc, const PairConst *pp,
+                             const PairConst *pw, const WallGeom *walls, const RefTables &R, double delta, double skin,
+                             int max_steps, unsigned long long *arrive, cudaStream_t s) {
+    return P.n <= kRefWideMax
+               ? steps_ref_t<32, true>(P, L, ctl, fc, pp, pw, walls, R, delta, skin, max_steps, arrive, s)
+               : steps_ref_t<8, true>(P, L, ctl, fc, pp, pw, walls, R, delta, skin, max_steps, arrive, s);
 }
 
 void launch_scene_steps_mixed(const Particles &P, const NbrList &L, Ctl *ctl, const ForceConsts &fc,

@@ -13,6 +13,7 @@
 // Built with --fmad=false so that the distance test matches the oracle's.
 #include "dem_internal.cuh"
 #include "b200dem.h"
+#include "dem_cells.cuh"
 
 namespace b200dem {
 
@@ -35,30 +36,6 @@ __device__ __forceinline__ unsigned long long ord(double x) {
 __device__ __forceinline__ double unord(unsigned long long o) {
     const unsigned long long b = (o & 0x8000000000000000ull) ? (o & 0x7fffffffffffffffull) : ~o;
     return __longlong_as_double((long long)b);
-}
-
-__device__ __forceinline__ unsigned part1by2(unsigned x) {
-    x &= 0x3ff;
-    x = (x | (x << 16)) & 0x030000FF;
-    x = (x | (x << 8)) & 0x0300F00F;
-    x = (x | (x << 4)) & 0x030C30C3;
-    x = (x | (x << 2)) & 0x09249249;
-    return x;
-}
-
-__device__ __forceinline__ int cell_key(const Grid &g, int cx, int cy, int cz) {
-    if (g.bits > 0)
-        return g.base + (int)(part1by2((unsigned)cx) | (part1by2((unsigned)cy) << 1) | (part1by2((unsigned)cz) << 2));
-    return g.base + (cz * g.dims[1] + cy) * g.dims[0] + cx;
-}
-
-__device__ __forceinline__ void cell_of(const Grid &g, const D4 &p, int c[3]) {
-    const double xs[3] = {p.x, p.y, p.z};
-    for (int d = 0; d < 3; ++d) {
-        int v = (int)floor((xs[d] - g.lo[d]) * g.inv_cell);
-        v = v < 0 ? 0 : (v >= g.dims[d] ? g.dims[d] - 1 : v);
-        c[d] = v;
-    }
 }
 
 __device__ __forceinline__ int scene_of(const Particles &P, int i) { return P.scene ? P.scene[i] : 0; }
@@ -730,6 +707,15 @@ __global__ void k_build_end(Ctl *ctl) {
 }
 
 }  // namespace
+
+// The grid alone (one scene), for the rebuild-every-step loop's cell tables.
+void launch_ref_grid(const Particles &P, BuildBuffers &B, Ctl *ctl, double delta, double skin, cudaStream_t s) {
+    const int blocks = (P.n + kB - 1) / kB;
+    k_build_begin<<<1, 32, 0, s>>>(ctl);
+    k_bbox_init<<<1, 256, 0, s>>>(B.bbox, 1);
+    k_bbox<<<blocks < 148 * 8 ? blocks : 148 * 8, kB, 0, s>>>(P, ctl, B.bbox);
+    k_grid<<<1, 256, 0, s>>>(B.bbox, B.grid, B.total, 1, B.cell_cap, delta, skin, ctl);
+}
 
 void launch_build(const Particles &P, Particles &alt, const NbrList &L, BuildBuffers &B, Ctl *ctl, double delta,
                   double skin, bool resort, bool check_run, cudaStream_t s, bool classes) {

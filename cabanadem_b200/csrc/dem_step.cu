@@ -20,6 +20,7 @@
 #include "dem_contact_coop.cuh"
 #include "dem_pairs.cuh"
 #include "dem_persist.cuh"
+#include "dem_refloop.cuh"
 #include "dem_scenes.cuh"
 
 namespace b200dem {
@@ -905,6 +906,16 @@ cudaError_t launch_steps_coop(const Particles &P, const NbrList &L, Ctl *ctl, co
     if (fc.mixed) return launch_steps_coop_mixed(P, L, ctl, fc, pp, pw, walls, max_steps, scratch, s);
     return fc.mesh.nt ? steps_coop_t<false, true>(P, L, ctl, fc, pp, pw, walls, max_steps, scratch, s)
                       : steps_coop_t<false, false>(P, L, ctl, fc, pp, pw, walls, max_steps, scratch, s);
+}
+
+cudaError_t launch_steps_ref(const Particles &P, const NbrList &L, Ctl *ctl, const ForceConsts &fc, const PairConst *pp,
+                             const PairConst *pw, const WallGeom *walls, const RefTables &R, double delta, double skin,
+                             int max_steps, unsigned long long *arrive, cudaStream_t s) {
+    if (fc.mixed)
+        return launch_steps_ref_mixed(P, L, ctl, fc, pp, pw, walls, R, delta, skin, max_steps, arrive, s);
+    return P.n <= kRefWideMax
+               ? steps_ref_t<32, false>(P, L, ctl, fc, pp, pw, walls, R, delta, skin, max_steps, arrive, s)
+               : steps_ref_t<8, false>(P, L, ctl, fc, pp, pw, walls, R, delta, skin, max_steps, arrive, s);
 }
 
 void launch_step(const Particles &P, const NbrList &L, Ctl *ctl, const ForceConsts &fc, const PairConst *pp,
