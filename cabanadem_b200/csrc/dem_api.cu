@@ -1569,6 +1569,12 @@ bool coop_loop(const dem_solver *s) {
            s->loop && !ref_mode(s);
 }
 
+// Whether the cooperative launches keep each particle in a thread's registers (dem_live.cuh):
+// static walls, no mesh, at most the threads resident at once.
+bool live_form(const dem_solver *s) {
+    return !s->fc.mwalls && s->mesh_nt == 0 && s->p->P.n <= live_capacity(s->fc.mixed != 0);
+}
+
 // The rebuild-every-step mode's run in one cooperative launch (dem_refloop.cuh): the one-kernel
 // step of a small system without batched scenes, static walls, no mesh.
 bool ref_loop(const dem_solver *s) {
@@ -1736,8 +1742,12 @@ extern "C" int dem_solver_run(dem_solver *s, int nsteps) {
             if (coop_loop(s)) {   // every step until the target or a stale list in one launch
                 if (!s->d_coop) CK(dalloc(&s->d_coop, (size_t)kCoopScratch));
                 CK(cudaEventRecord(s->ev0, st));
-                const cudaError_t le = launch_steps_coop(s->p->P, s->L, s->p->ctl, s->fc, s->d_pp, s->d_pw, s->d_walls,
-                                                         nsteps, s->d_coop, st);
+                const bool live = live_form(s);
+                const cudaError_t le =
+                    live ? launch_steps_live(s->p->P, s->L, s->p->ctl, s->fc, s->d_pp, s->d_pw, s->d_walls, s->p->P.n,
+                                             nsteps, s->d_coop, 0, st)
+                         : launch_steps_coop(s->p->P, s->L, s->p->ctl, s->fc, s->d_pp, s->d_pw, s->d_walls, nsteps,
+                                             s->d_coop, st);
                 if (le != cudaSuccess) {   // not resident at once (or refused): graph replays from here on
                     (void)cudaGetLastError();
                     s->coop_refused = true;

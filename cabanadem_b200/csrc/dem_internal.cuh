@@ -49,6 +49,12 @@ struct Ctl {
     int loop_iter;            // iterations of the step loop in the current graph replay
     long long wfar_build;     // value of `rebuilds` when NbrList::wfar was last computed
     unsigned gen;             // step generation of the cooperative step loop (dem_persist.cuh)
+    // quiet systems (dem_flight.cuh)
+    double clear_until;       // displacement bound up to which the particles [0, nlone + nclear) are clear
+    unsigned long long vq2;   // bound on |u|^2 of the quiet particles (double bits)
+    int flight_cur;           // position buffer the quiet particles are in
+    int flight_steps;         // steps the others were advanced from there
+    int flight_last;          // 1: the last of them was the run's last
 };
 
 struct Particles {
@@ -340,6 +346,17 @@ cudaError_t launch_steps_coop(const Particles &P, const NbrList &L, Ctl *ctl, co
 cudaError_t launch_steps_coop_mixed(const Particles &P, const NbrList &L, Ctl *ctl, const ForceConsts &fc,
                                     const PairConst *pp, const PairConst *pw, const WallGeom *walls, int max_steps,
                                     unsigned long long *scratch, cudaStream_t s);
+// The same with each particle in a thread's registers (dem_live.cuh): static walls, no mesh, `count`
+// particles, at most live_capacity.  quiet: the particles [nlone + nclear, n) only (dem_flight.cuh).
+// scratch 16-byte aligned.
+int live_capacity(bool mixed);
+cudaError_t launch_steps_live(const Particles &P, const NbrList &L, Ctl *ctl, const ForceConsts &fc, const PairConst *pp,
+                              const PairConst *pw, const WallGeom *walls, int count, int max_steps,
+                              unsigned long long *scratch, int quiet, cudaStream_t s);
+int live_capacity_mixed();
+cudaError_t launch_steps_live_mixed(const Particles &P, const NbrList &L, Ctl *ctl, const ForceConsts &fc,
+                                    const PairConst *pp, const PairConst *pw, const WallGeom *walls, int count,
+                                    int max_steps, unsigned long long *scratch, int quiet, cudaStream_t s);
 
 // The rebuild-every-step mode's run in one cooperative launch (dem_refloop.cuh): at most
 // `max_steps` steps, ending at the target, or earlier where the build and step kernels have to go

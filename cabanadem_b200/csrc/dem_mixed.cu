@@ -10,6 +10,7 @@
 #include "dem_contact_coop.cuh"
 #include "dem_pairs.cuh"
 #include "dem_persist.cuh"
+#include "dem_live.cuh"
 #include "dem_refloop.cuh"
 #include "dem_scenes.cuh"
 
@@ -218,6 +219,14 @@ cudaError_t launch_steps_coop_mixed(const Particles &P, const NbrList &L, Ctl *c
                                     unsigned long long *scratch, cudaStream_t s) {
     return fc.mesh.nt ? steps_coop_t<true, true>(P, L, ctl, fc, pp, pw, walls, max_steps, scratch, s)
                       : steps_coop_t<true, false>(P, L, ctl, fc, pp, pw, walls, max_steps, scratch, s);
+}
+
+int live_capacity_mixed() { return live_threads<true>(); }
+
+cudaError_t launch_steps_live_mixed(const Particles &P, const NbrList &L, Ctl *ctl, const ForceConsts &fc, const PairConst *pp,
+                              const PairConst *pw, const WallGeom *walls, int count, int max_steps,
+                              unsigned long long *scratch, int quiet, cudaStream_t s) {
+    return steps_live_t<true>(P, L, ctl, fc, pp, pw, walls, count, max_steps, scratch, quiet, s);
 }
 
 cudaError_t launch_steps_ref_mixed(const Particles &P, const NbrList &L, Ctl *ctl, const ForceConsts &fc, const PairConst *pp,

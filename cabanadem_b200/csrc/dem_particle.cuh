@@ -263,6 +263,37 @@ __device__ __forceinline__ void block_vmax(Ctl *ctl, unsigned long long *slots, 
 }
 
 
+// The step of particle i without pair force and torque, as particle_full takes it: external force,
+// the hooks, stage3 of this step and stage1 + stage2 of the next (or F and tau stored after a run's
+// last step).  u and pn in and out; omega stays (no torque).  Returns |u|^2 of the drift.
+__device__ __forceinline__ double free_step(const Particles &P, const ForceConsts &fc, const int i, const int last,
+                                            const double m, double (&u)[3], D4 &pn) {
+    const int cap = P.cap;
+    double F[3] = {0., 0., 0.};
+    for (int d = 0; d < 3; ++d) {
+        if (fc.has_ext) F[d] = dadd(F[d], P.ext[d * cap + i]);
+        if (fc.has_gravity) F[d] = dadd(F[d], dmul(m, fc.g[d]));
+    }
+    if (fc.has_fix && (P.fix[i] & DEM_FIX_FORCE)) F[0] = F[1] = F[2] = 0.;
+    const double m_inverse = 1. / m;
+    double x[3] = {pn.x, pn.y, pn.z};
+    for (int d = 0; d < 3; ++d) {
+        const double a = dmul(dmul(fc.half_dt, F[d]), m_inverse);
+        u[d] = dadd(u[d], a);
+        if (last) {
+            P.force[d * cap + i] = F[d];
+            P.torque[d * cap + i] = 0.;
+        } else {
+            u[d] = dadd(u[d], a);
+            x[d] = dadd(x[d], dmul(fc.dt, u[d]));
+        }
+    }
+    pn.x = x[0];
+    pn.y = x[1];
+    pn.z = x[2];
+    return last ? 0.0 : dadd(dadd(dmul(u[0], u[0]), dmul(u[1], u[1])), dmul(u[2], u[2]));
+}
+
 // One particle-particle contact of i with partner j at overlap > 0 (Force.hpp:73-329): Hertz
 // normal force with damping, Mindlin tangential force with the Coulomb limit.  h is the
 // tangential history (in and out); cf receives the contribution to F (0..2) and tau (3..5) of i,

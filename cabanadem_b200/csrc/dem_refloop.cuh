@@ -105,39 +105,6 @@ __device__ __forceinline__ bool ref_barrier(Ctl *ctl, unsigned long long *arrive
     return s_go != 0;
 }
 
-// The step of a particle without pair force and torque: external force, the hooks, stage3 of this
-// step and stage1 + stage2 of the next, into the other buffers (omega as it is: no torque).
-__device__ __forceinline__ void ref_free_step(const Particles &P, const ForceConsts &fc, const int i, const int nxt,
-                                              const int vnxt, const int last, const double m_i, double (&u)[3],
-                                              const double (&w)[3], D4 &pn) {
-    const int cap = P.cap;
-    double F[3] = {0., 0., 0.};
-    for (int d = 0; d < 3; ++d) {
-        if (fc.has_ext) F[d] = dadd(F[d], P.ext[d * cap + i]);
-        if (fc.has_gravity) F[d] = dadd(F[d], dmul(m_i, fc.g[d]));
-    }
-    if (fc.has_fix && (P.fix[i] & DEM_FIX_FORCE)) F[0] = F[1] = F[2] = 0.;
-    const double m_inverse = 1. / m_i;
-    double x[3] = {pn.x, pn.y, pn.z};
-    for (int d = 0; d < 3; ++d) {
-        const double a = dmul(dmul(fc.half_dt, F[d]), m_inverse);
-        u[d] = dadd(u[d], a);
-        if (last) {
-            P.force[d * cap + i] = F[d];
-            P.torque[d * cap + i] = 0.;
-        } else {
-            u[d] = dadd(u[d], a);
-            x[d] = dadd(x[d], dmul(fc.dt, u[d]));
-        }
-        P.vel[vnxt][d * cap + i] = u[d];
-        P.omg[vnxt][d * cap + i] = w[d];
-    }
-    pn.x = x[0];
-    pn.y = x[1];
-    pn.z = x[2];
-    st4(P.pos[nxt], i, pn);
-}
-
 struct RefGroup {   // a group's share of the block's shared memory
     double h[3 * kCoopSlots + 1];
     int tidx[kCoopSlots + 1];
@@ -278,7 +245,12 @@ __global__ void __launch_bounds__(RefShape<NL>::block, RefShape<NL>::min_blocks)
                                                 status, &pn);
             } else if (i >= 0 && gl == 0) {
                 // nothing touches this particle: the step of particle_coop without contacts
-                ref_free_step(P, fc, i, cur ^ 1, vcur ^ 1, last, m_i, u, w, pn);
+                free_step(P, fc, i, last, m_i, u, pn);
+                st4(P.pos[cur ^ 1], i, pn);
+                for (int d = 0; d < 3; ++d) {
+                    P.vel[vcur ^ 1][d * cap + i] = u[d];
+                    P.omg[vcur ^ 1][d * cap + i] = w[d];
+                }
             }
             if (i >= 0 && gl == 0) {
                 if (k > 0) R.count[(long)tz * R.codes + R.key[(long)tz * cap + i]] = 0;

@@ -20,6 +20,7 @@
 #include "dem_contact_coop.cuh"
 #include "dem_pairs.cuh"
 #include "dem_persist.cuh"
+#include "dem_live.cuh"
 #include "dem_refloop.cuh"
 #include "dem_scenes.cuh"
 
@@ -906,6 +907,16 @@ cudaError_t launch_steps_coop(const Particles &P, const NbrList &L, Ctl *ctl, co
     if (fc.mixed) return launch_steps_coop_mixed(P, L, ctl, fc, pp, pw, walls, max_steps, scratch, s);
     return fc.mesh.nt ? steps_coop_t<false, true>(P, L, ctl, fc, pp, pw, walls, max_steps, scratch, s)
                       : steps_coop_t<false, false>(P, L, ctl, fc, pp, pw, walls, max_steps, scratch, s);
+}
+
+int live_capacity(bool mixed) { return mixed ? live_capacity_mixed() : live_threads<false>(); }
+
+cudaError_t launch_steps_live(const Particles &P, const NbrList &L, Ctl *ctl, const ForceConsts &fc, const PairConst *pp,
+                              const PairConst *pw, const WallGeom *walls, int count, int max_steps,
+                              unsigned long long *scratch, int quiet, cudaStream_t s) {
+    if (fc.mixed)
+        return launch_steps_live_mixed(P, L, ctl, fc, pp, pw, walls, count, max_steps, scratch, quiet, s);
+    return steps_live_t<false>(P, L, ctl, fc, pp, pw, walls, count, max_steps, scratch, quiet, s);
 }
 
 cudaError_t launch_steps_ref(const Particles &P, const NbrList &L, Ctl *ctl, const ForceConsts &fc, const PairConst *pp,
