@@ -104,6 +104,9 @@ struct dem_solver {
     bool coop_refused = false;                  // a cooperative launch of the step loop was refused
     bool coop_ran = false;                      // the last run's steps ran in cooperative launches
     unsigned long long *d_coop = nullptr;       // kCoopScratch words: barrier counter and slots
+    bool quiet = false;                         // the current list's build found a quiet system
+    int rest = 0;                               // its particles that are not quiet
+    int quiet_wait = 0;                         // builds until quiet classes are tried again
     RefTables ref{};                            // cell tables of the rebuild-every-step loop
 };
 
@@ -938,7 +941,8 @@ int prepare(dem_solver *s) {
     CK(cudaMemcpyAsync(s->d_pp, pp.data(), pp.size() * sizeof(PairConst), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(s->d_pw, pw.data(), pw.size() * sizeof(PairConst), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(s->d_walls, wg.data(), wg.size() * sizeof(WallGeom), cudaMemcpyHostToDevice, st));
-    // the wall-gap flags of the last build were taken against the previous walls
+    // the wall-gap flags and the quiet classes of the last build were taken against the previous walls
+    s->quiet = false;
     CK(cudaMemsetAsync(&p->ctl->wfar_build, 0xff, sizeof(long long), st));
     // mesh: particle materials against the mesh's, in the plane walls' expression order
     cudaFree(s->d_mesh_pm);
@@ -1134,6 +1138,15 @@ int check_walls(dem_solver *s) {
                 "dem_solver_set_scenes) or too few walls for the scenes");
 }
 
+// Quiet systems (dem_flight.cuh).  The gap that makes a particle quiet, in skins: a larger one keeps
+// the classes valid longer (a build is needed when the displacement bound reaches half of it), a
+// smaller one leaves fewer particles to step one by one.
+constexpr double kQuietGap = 0.25;
+constexpr int kQuietMinSteps = 64;   // steps a build has to last to be worth its classes
+constexpr int kQuietRetry = 16;      // builds until a system found not quiet is looked at again
+constexpr int kFlightSteps = 64;     // steps of the others per flight of the quiet ones
+constexpr int kFlightBatch = 16;     // flights queued before the host reads the control word
+
 // kernels issued by one launch_build (see dem_nbr.cu)
 long build_kernel_count(bool resort) { return 13 + (resort ? 7 : 0); }
 
@@ -1141,13 +1154,41 @@ long build_kernel_count(bool resort) { return 13 + (resort ? 7 : 0); }
 int build_with(dem_solver *s, bool resort, double delta, double skin);
 int build_now(dem_solver *s, bool resort) { return build_with(s, resort, s->sp.delta, s->sp.skin); }
 
+// Whether a build should look for a quiet system: the three-kernel step's sizes and settings, where
+// a quiet particle's free steps can be taken many at a time.
+bool quiet_possible(const dem_solver *s) {
+    return !ref_mode(s) && s->sp.delta <= 0.0 && s->sp.skin > 0.0 && s->loop && s->sp.cooperative_loop != 2 &&
+           !s->coop_refused && s->sp.contact_lanes == 0 && s->sp.dense_form == 0 && s->sp.stream_split == 0 &&
+           s->p->P.n > live_capacity(s->fc.mixed != 0) && !s->fc.mwalls && s->mesh_nt == 0 && !s->p->P.ext && !s->p->has_bonds &&
+           (s->fc.nwall == 0 || s->d_walls);
+}
+
 int build_with(dem_solver *s, bool resort, double delta, double skin) {
     dem_ctx *ctx = s->ctx;
     s->scenes_ready = false;   // this build's order partitions the storage by class, not by scene
+    s->quiet = false;
     if (s->p->has_bonds) resort = false;
     for (int attempt = 0; attempt < 8; ++attempt) {
-        launch_build(s->p->P, s->p->alt, s->L, s->B, s->p->ctl, delta, skin, resort, false, ctx->stream);
+        // a solver's run list: with quiet classes (dem_flight.cuh) where those may pay
+        ClassSpec cc;
+        cc.gap = 0.5 * skin;
+        bool quiet = false;
+        if (resort && delta == s->sp.delta && skin == s->sp.skin && quiet_possible(s)) {
+            quiet = s->quiet_wait == 0;
+            if (!quiet) --s->quiet_wait;
+        }
+        if (quiet) {
+            cc.gap = kQuietGap * skin;
+            cc.walls = s->d_walls;
+            cc.nwall = s->fc.nwall;
+            cc.wps = s->fc.wps;
+        }
+        launch_build(s->p->P, s->p->alt, s->L, s->B, s->p->ctl, delta, skin, resort, false, ctx->stream, cc);
         s->launches += build_kernel_count(resort);
+        if (quiet) {
+            launch_quiet_begin(s->p->P, s->p->ctl, ctx->stream);
+            s->launches += 1;
+        }
         if (resort && s->mesh_nt > 0) {   // tracked triangle contacts follow the re-sort (B.key: new <- old)
             const size_t cap = (size_t)s->p->P.cap;
             const MeshDev &M = s->mesh, &A = s->mesh_alt;
@@ -1177,6 +1218,15 @@ int build_with(dem_solver *s, bool resort, double delta, double skin) {
             }
             s->built = true;
             s->p->dirty = false;
+            if (quiet) {
+                double vq2;
+                std::memcpy(&vq2, &c.vq2, sizeof vq2);
+                const int rest = s->p->P.n - c.nlone - c.nclear;
+                s->quiet = rest <= live_capacity(s->fc.mixed != 0) &&
+                           kQuietMinSteps * s->sp.dt * std::sqrt(vq2) < 0.5 * cc.gap;
+                s->rest = rest;
+                if (!s->quiet) s->quiet_wait = kQuietRetry;
+            }
             return DEM_OK;
         }
         const int want = std::min(std::max(2 * s->L.maxnb, c.max_nbr + 8), 128);
@@ -1516,7 +1566,9 @@ int run_scenes(dem_solver *s, int nsteps) {
     if (!s->scenes_ready || s->p->dirty) {
         // re-sort in plain cell order (scene-major keys): every scene contiguous
         for (int attempt = 0;; ++attempt) {
-            launch_build(s->p->P, s->p->alt, s->L, s->B, s->p->ctl, s->sp.delta, s->sp.skin, true, false, st, false);
+            ClassSpec plain;
+            plain.on = false;
+            launch_build(s->p->P, s->p->alt, s->L, s->B, s->p->ctl, s->sp.delta, s->sp.skin, true, false, st, plain);
             s->launches += build_kernel_count(true);
             const Ctl c = read_ctl(s);
             if (!(c.status & DEM_ERR_NEIGHBOR_OVERFLOW)) break;
@@ -1739,6 +1791,43 @@ extern "C" int dem_solver_run(dem_solver *s, int nsteps) {
         }
         s->coop_ran = false;
         for (int guard = 0;; ++guard) {
+            if (s->quiet) {   // the few that can touch something step by step, the quiet ones in flights
+                if (!s->d_coop) CK(dalloc(&s->d_coop, (size_t)kCoopScratch));
+                const int done_before = s->graph_done_mark, left = nsteps - done_before;
+                CK(cudaEventRecord(s->ev0, st));
+                for (int b = 0; b < kFlightBatch && b * kFlightSteps < left; ++b) {
+                    const cudaError_t le = launch_steps_live(s->p->P, s->L, s->p->ctl, s->fc, s->d_pp, s->d_pw,
+                                                             s->d_walls, s->rest, kFlightSteps, s->d_coop, 1, st);
+                    if (le != cudaSuccess) {
+                        (void)cudaGetLastError();
+                        s->coop_refused = true;
+                        s->quiet = false;
+                        break;
+                    }
+                    launch_flight(s->p->P, s->p->ctl, s->fc, st);
+                    s->launches += 2;
+                }
+                CK(cudaEventRecord(s->ev1, st));
+                const Ctl c = read_ctl(s);
+                CK(cudaGetLastError());
+                if (c.status & DEM_ERR_TIMEOUT) return fail(ctx, DEM_ERR_TIMEOUT, "a bounded device wait gave up");
+                if (c.steps_done > done_before) {
+                    s->coop_ran = true;
+                    float ms = 0.f;
+                    CK(cudaEventElapsedTime(&ms, s->ev0, s->ev1));
+                    s->graph_ms += ms;
+                    s->graph_steps_run += c.steps_done - done_before;
+                    s->graph_done_mark = c.steps_done;
+                    steps_before = c.steps_done;
+                }
+                if (c.steps_done >= c.target) break;
+                if (s->quiet && !(c.disp < std::min(c.half_skin, c.clear_until))) {
+                    int e = build_now(s, true);
+                    if (e) return e;
+                }
+                if (guard > 4 * (nsteps + 4)) return fail(ctx, DEM_ERR_CUDA, "solver made no progress");
+                continue;
+            }
             if (coop_loop(s)) {   // every step until the target or a stale list in one launch
                 if (!s->d_coop) CK(dalloc(&s->d_coop, (size_t)kCoopScratch));
                 CK(cudaEventRecord(s->ev0, st));

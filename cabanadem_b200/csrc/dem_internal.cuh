@@ -44,7 +44,7 @@ struct Ctl {
     int nlone;                // particles [0, nlone) had no listed neighbour at the last build
                               // (placed first by the re-sort; 0 when the build did not re-sort)
     int nclear;               // particles [nlone, nlone + nclear): every listed neighbour's gap
-                              // exceeded skin/2 at the last build (placed second)
+                              // exceeded 2 clear_until at the last build (placed second)
     int npairs;               // contact work items of the current step (pair-parallel dense step)
     int loop_iter;            // iterations of the step loop in the current graph replay
     long long wfar_build;     // value of `rebuilds` when NbrList::wfar was last computed
@@ -318,10 +318,20 @@ void launch_energy(const Particles &P, const NbrList &L, Ctl *ctl, const ForceCo
 // ---- launchers (dem_nbr.cu) -------------------------------------------------------
 // Builds the neighbour list of the current order; with `resort` the particles are first
 // re-ordered by Morton cell key (state permuted, contact partners remapped).
-// classes = false: a re-sort keeps the plain cell order (scene-major for batched scenes), without
-// the partition into particles with no listed neighbour, clear ones and the rest.
+// `cc`: the re-sort's partition into particles with no listed neighbour, clear ones and the rest;
+// off keeps the plain cell order (scene-major for batched scenes).
+struct ClassSpec {
+    bool on = true;
+    double gap = 0.0;                 // a clear particle's listed neighbours all keep a larger gap
+    const struct WallGeom *walls = nullptr;   // quiet classes: tracked contacts and near walls count too
+    int nwall = 0, wps = 0;
+};
 void launch_build(const Particles &P, Particles &alt, const NbrList &L, BuildBuffers &B, Ctl *ctl, double delta,
-                  double skin, bool resort, bool check_run, cudaStream_t s, bool classes = true);
+                  double skin, bool resort, bool check_run, cudaStream_t s, const ClassSpec &cc = ClassSpec());
+// Quiet systems (dem_flight.cuh), static walls, no mesh, no external forces: after a build with
+// quiet classes, launch_quiet_begin; after each launch_steps_live with quiet 1, launch_flight.
+void launch_quiet_begin(const Particles &P, Ctl *ctl, cudaStream_t s);
+void launch_flight(const Particles &P, Ctl *ctl, const ForceConsts &fc, cudaStream_t s);
 // Batched small scenes in one persistent launch per run (dem_scenes.cuh): the scene table of
 // the current storage (false when some scene is not contiguous or exceeds the block), and the
 // run's steps.

@@ -461,80 +461,21 @@ __global__ void __launch_bounds__(128) k_list(Particles P, NbrList L, Ctl *ctl, 
     }
 }
 
-// Re-sort partition, pass 1: class of cell slot s (cell order of the old storage): 0 when its
-// particle has no neighbour within the list cutoff (the predicate of k_list: its list will be
-// empty), 1 when, in the Verlet-skin mode, every listed neighbour's gap |x_i - x_j| - r_i - r_j
-// exceeds skin/2 (no contact possible while twice the displacement bound stays below skin/2),
-// else 2.  Per-block counts of classes 0 and 1 into sums[0][b], sums[1][b].
-__global__ void __launch_bounds__(kPartBlock) k_part_flag(Particles P, const Ctl *ctl, const Grid *g, const int *start,
-                                                          const int *items, double delta, double skin, int *cls,
-                                                          int *sums, int nb, int classes) {
-    const int cur = ctl->cur, n = P.n;
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    int c_s = 2;
-    if (s < n && classes && !(ctl->status & DEM_ERR_NAN)) {
-        const int q = items[s];
-        const Grid G = g[scene_of(P, q)];
-        const double4 *pc = P.pos[cur];
-        const D4 pi = ld4(pc, q);
-        const bool skin_mode = !(delta > 0.0) && skin > 0.0;
-        int c[3];
-        cell_of(G, pi, c);
-        bool any = false, near = false;
-        for (int dz = -1; dz <= 1 && !near; ++dz) {
-            const int z = c[2] + dz;
-            if (z < 0 || z >= G.dims[2]) continue;
-            for (int dy = -1; dy <= 1 && !near; ++dy) {
-                const int y = c[1] + dy;
-                if (y < 0 || y >= G.dims[1]) continue;
-                for (int dx = -1; dx <= 1 && !near; ++dx) {
-                    const int x = c[0] + dx;
-                    if (x < 0 || x >= G.dims[0]) continue;
-                    const int key = cell_key(G, x, y, z);
-                    const int e = start[key + 1];
-                    for (int t = start[key]; t < e; ++t) {
-                        const int j = items[t];
-                        if (j == q) continue;
-                        const D4 pj = ld4(pc, j);
-                        const double px = pi.x - pj.x, py = pi.y - pj.y, pz = pi.z - pj.z;
-                        const double r2 = px * px + py * py + pz * pz;
-                        const double cut = delta > 0.0 ? delta : pi.w + pj.w + skin;
-                        if (r2 <= cut * cut) {
-                            any = true;
-                            if (!skin_mode || !(sqrt(r2) - (pi.w + pj.w) > 0.5 * skin)) {
-                                near = true;
-                                break;
-                            }
-                        }
-                    }
-                }
-            }
-        }
-        c_s = !any ? 0 : (near ? 2 : 1);
-    }
-    if (s < n) cls[s] = c_s;
-    __shared__ int cnt[2];
-    if (threadIdx.x < 2) cnt[threadIdx.x] = 0;
-    __syncthreads();
-    const int w0 = __popc(__ballot_sync(0xffffffffu, s < n && c_s == 0));
-    const int w1 = __popc(__ballot_sync(0xffffffffu, s < n && c_s == 1));
-    if ((threadIdx.x & 31) == 0) {
-        if (w0) atomicAdd(&cnt[0], w0);
-        if (w1) atomicAdd(&cnt[1], w1);
-    }
-    __syncthreads();
-    if (threadIdx.x < 2) sums[threadIdx.x * (nb + 1) + blockIdx.x] = cnt[threadIdx.x];
-}
-
-// Re-sort partition, pass 1 with the lists: the class of cell slot s as k_part_flag gives it,
-// from the full list search of k_list done here, in the old storage order -- the list of the
+// Re-sort partition, pass 1, with the lists: the class of cell slot s (cell order of the old
+// storage): 0 when its particle has no neighbour within the list cutoff (its list is empty), 1 when,
+// in the Verlet-skin mode, every listed neighbour's gap |x_i - x_j| - r_i - r_j exceeds `cc.gap` (no
+// contact possible while twice the displacement bound stays below it), else 2.  With cc.walls also 2
+// when the particle tracks a contact or wall history, or when a wall of its scene is not farther than
+// cc.gap: classes 0 and 1 are then the particles that nothing can touch until then (quiet,
+// dem_flight.cuh).  Per-block counts of classes 0 and 1 into sums[0][b], sums[1][b].
+// The full list search of k_list is done here, in the old storage order -- the list of the
 // particle q = items[s] goes to nn_old[q], idx_old[k][q] (old indices, ascending caller index),
 // and k_list_remap re-indexes it into the new order after the permutation, instead of a second
 // 27-cell search over the permuted storage.  Same candidates, same order, same overflow rule as
 // k_list (kMaxCand kept, DEM_ERR_NEIGHBOR_OVERFLOW when a list exceeds the capacity).
 __global__ void __launch_bounds__(kPartBlock) k_part_list(Particles P, NbrList L, Ctl *ctl, const Grid *g,
                                                           const int *start, const int *items, double delta,
-                                                          double skin, int *cls, int *sums, int nb, int classes) {
+                                                          double skin, int *cls, int *sums, int nb, ClassSpec cc) {
     const int cur = ctl->cur, n = P.n, cap = P.cap;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     const bool invalid = (ctl->status & DEM_ERR_NAN) != 0;
@@ -570,7 +511,7 @@ __global__ void __launch_bounds__(kPartBlock) k_part_list(Particles P, NbrList L
                         const double r2 = px * px + py * py + pz * pz;
                         const double cut = delta > 0.0 ? delta : pi.w + pj.w + skin;
                         if (r2 <= cut * cut) {
-                            if (!skin_mode || !(sqrt(r2) - (pi.w + pj.w) > 0.5 * skin)) near = true;
+                            if (!skin_mode || !(sqrt(r2) - (pi.w + pj.w) > cc.gap)) near = true;
                             if (count < kMaxCand) {
                                 // insertion by caller index
                                 const int kj = P.perm[j];
@@ -593,7 +534,17 @@ __global__ void __launch_bounds__(kPartBlock) k_part_list(Particles P, NbrList L
         const int keep = count < lim ? count : lim;
         for (int k = 0; k < keep; ++k) L.idx_old[(long)k * cap + q] = cand[k];
         L.nn_old[q] = keep;
-        c_s = !classes ? 2 : count == 0 ? 0 : (near ? 2 : 1);
+        if (cc.walls) {
+            near = near || P.cstate[q] != 0;
+            const int w0 = cc.wps ? scene_of(P, q) * cc.wps : 0, w1 = cc.wps ? w0 + cc.wps : cc.nwall;
+            for (int w = w0; w < w1; ++w) {
+                const WallGeom &g = cc.walls[w];
+                const double at = (pi.x - g.x[0]) * g.n[0] + (pi.y - g.x[1]) * g.n[1] + (pi.z - g.x[2]) * g.n[2];
+                near = near || !(at - pi.w > cc.gap);
+            }
+        }
+        // without the walls' part a particle near a wall can still be lone: the streaming pass tests its walls
+        c_s = !cc.on ? 2 : (cc.walls && near) ? 2 : count == 0 ? 0 : (near ? 2 : 1);
     }
     if (s < n) cls[s] = c_s;
     __shared__ int cnt[2];
@@ -693,15 +644,17 @@ __global__ void __launch_bounds__(kPartBlock) k_part_place(int n, const int *cls
 
 __global__ void k_build_begin(Ctl *ctl) {
     if (threadIdx.x == 0) {
+        ctl->vq2 = 0ull;
         ctl->max_nbr = 0;
         ctl->nlone = 0;
         ctl->nclear = 0;
     }
 }
 
-__global__ void k_build_end(Ctl *ctl) {
+__global__ void k_build_end(Ctl *ctl, double clear_until) {
     if (threadIdx.x == 0) {
         ctl->disp = 0.0;
+        ctl->clear_until = clear_until;
         ctl->rebuilds += 1;
     }
 }
@@ -718,7 +671,7 @@ void launch_ref_grid(const Particles &P, BuildBuffers &B, Ctl *ctl, double delta
 }
 
 void launch_build(const Particles &P, Particles &alt, const NbrList &L, BuildBuffers &B, Ctl *ctl, double delta,
-                  double skin, bool resort, bool check_run, cudaStream_t s, bool classes) {
+                  double skin, bool resort, bool check_run, cudaStream_t s, const ClassSpec &cc) {
     (void)check_run;
     const int n = P.n;
     const int gs = 148 * 8;
@@ -741,12 +694,8 @@ void launch_build(const Particles &P, Particles &alt, const NbrList &L, BuildBuf
         // particles whose listed neighbours all keep a gap above skin/2, and the rest, so that
         // the streaming kernel's leading warps load no list and the next ones no partner
         const int nb = (n + kPartBlock - 1) / kPartBlock;
-        if (L.idx_old)   // the lists too, in the old order (re-indexed below)
-            k_part_list<<<nb, kPartBlock, 0, s>>>(P, L, ctl, B.grid, B.cell_fill, B.cell_items, delta, skin, B.src,
-                                                  B.part_sums, nb, classes ? 1 : 0);
-        else
-            k_part_flag<<<nb, kPartBlock, 0, s>>>(P, ctl, B.grid, B.cell_fill, B.cell_items, delta, skin, B.src,
-                                                  B.part_sums, nb, classes ? 1 : 0);
+        k_part_list<<<nb, kPartBlock, 0, s>>>(P, L, ctl, B.grid, B.cell_fill, B.cell_items, delta, skin, B.src,
+                                              B.part_sums, nb, cc);
         k_part_scan<<<1, 1024, 0, s>>>(B.part_sums, nb, ctl);
         k_part_place<<<nb, kPartBlock, 0, s>>>(n, B.src, B.part_sums, nb, ctl, B.cell_items, B.key);
         k_make_dst<<<gs, kB, 0, s>>>(n, B.key, B.dst);
@@ -764,11 +713,11 @@ void launch_build(const Particles &P, Particles &alt, const NbrList &L, BuildBuf
         if (P.scene) cudaMemcpyAsync(P.scene, alt.scene, cap * sizeof(int), cudaMemcpyDeviceToDevice, s);
         k_flip<<<1, 32, 0, s>>>(ctl);
     }
-    if (resort && L.idx_old)
+    if (resort)
         k_list_remap<<<gs, kB, 0, s>>>(n, P.cap, L, B.key, B.dst);
     else
         k_list<<<(n + 127) / 128, 128, 0, s>>>(P, L, ctl, B.grid, B.cell_fill, B.cell_items, delta, skin);
-    k_build_end<<<1, 32, 0, s>>>(ctl);
+    k_build_end<<<1, 32, 0, s>>>(ctl, 0.5 * cc.gap);
 }
 
 }  // namespace b200dem

@@ -21,6 +21,7 @@
 #include "dem_pairs.cuh"
 #include "dem_persist.cuh"
 #include "dem_live.cuh"
+#include "dem_flight.cuh"
 #include "dem_refloop.cuh"
 #include "dem_scenes.cuh"
 
@@ -70,9 +71,9 @@ __device__ __forceinline__ StreamCtl stream_ctl(const Ctl *ctl, int n) {
     c.cur = ctl->cur;
     c.vcur = ctl->vcur;
     c.nlone = ctl->nlone;
-    // particles [nlone, nclear_end) had every listed neighbour at a gap above skin/2: while
-    // twice the displacement bound stays below skin/2 none of them can touch
-    c.nclear_end = (2.0 * ctl->disp < ctl->half_skin) ? c.nlone + ctl->nclear : c.nlone;
+    // particles [nlone, nclear_end) had every listed neighbour at a gap above 2 clear_until: while
+    // the displacement bound stays below clear_until none of them can touch
+    c.nclear_end = ctl->disp < ctl->clear_until ? c.nlone + ctl->nclear : c.nlone;
     c.wfar = ctl->wfar_build == ctl->rebuilds && 2.0 * ctl->disp < ctl->half_skin;
     c.last = ctl->steps_done + 1 >= ctl->target;
     c.n = n;
@@ -543,8 +544,8 @@ __global__ void __launch_bounds__(kApplyBlock) k_apply(Particles P, NbrList L, C
 // one block per 128 particles (15,625 on the 2M lattice) would queue as many atomics on one word.
 __global__ void __launch_bounds__(kBlock) k_prologue(Particles P, Ctl *ctl, ForceConsts fc) {
     const int cur = ctl->cur, nxt = cur ^ 1, vcur = ctl->vcur;
-    const int cap = P.cap;
-    double vmax2 = 0.0;
+    const int cap = P.cap, nq = ctl->nlone + ctl->nclear;
+    double vmax2 = 0.0, vq2 = 0.0;   // of all; of the quiet ones (dem_flight.cuh)
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P.n; i += gridDim.x * blockDim.x) {
         const double m_inverse = 1. / P.mI[i], h = fc.half_dt;
         double *vc = P.vel[vcur], *wc = P.omg[vcur];
@@ -566,9 +567,12 @@ __global__ void __launch_bounds__(kBlock) k_prologue(Particles P, Ctl *ctl, Forc
         p.x += fc.dt * u[0];
         p.y += fc.dt * u[1];
         p.z += fc.dt * u[2];
-        vmax2 = fmax(vmax2, u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
+        const double v2 = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
+        vmax2 = fmax(vmax2, v2);
+        if (i < nq) vq2 = fmax(vq2, v2);
         st4(P.pos[nxt], i, p);
     }
+    fold_vq2(ctl, vq2);
     finish_step(ctl, P.vslots, vmax2, fc.dt, 0, false, false, &fc);
 }
 
