@@ -119,6 +119,8 @@ struct dem_bonds {
     int graph_steps = 0;
     long graph_version = -1;
     bool set_up = false;
+    int slots = -1;          // largest bond count of a particle, -1 when bonds changed since it was read
+    bool loop_refused = false;
 };
 
 namespace {
@@ -369,6 +371,12 @@ __global__ void k_loop_ctl(Ctl *ctl, cudaGraphConditionalHandle h, int n, int de
     if (threadIdx.x != 0) return;
     ++ctl->loop_iter;
     cudaGraphSetConditional(h, loop_go(ctl, n, dense, min_left) ? 1u : 0u);
+}
+__global__ void k_max_i(const int *v, int n, int *out) {
+    int m = 0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) m = max(m, v[i]);
+    m = (int)__reduce_max_sync(0xffffffffu, (unsigned)m);
+    if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(out, m);
 }
 __global__ void k_invalidate(Ctl *ctl) {
     if (threadIdx.x == 0) ctl->disp = 1e300;
@@ -2199,6 +2207,7 @@ extern "C" int dem_bonds_setup(dem_bonds *b, double factor, double search_cutoff
     p->has_bonds = true;
     s->built = false;   // the list was built with the bond search cutoff
     b->set_up = true;
+    b->slots = -1;
     Ctl c = read_ctl(s);
     return c.status & DEM_ERR_BOND_OVERFLOW;
 }
@@ -2287,6 +2296,7 @@ extern "C" int dem_bonds_set(dem_bonds *b, int field, const void *host, long cou
         // bonds given by the caller define the particle order from now on, as setupBonds does
         s->p->has_bonds = true;
         b->set_up = true;
+        b->slots = -1;
     }
     return DEM_OK;
 }
@@ -2349,6 +2359,21 @@ extern "C" int dem_bonds_broken(dem_bonds *b, long *count) {
     return DEM_OK;
 }
 
+// b->slots: the largest bond count of a particle, read after the bonds changed.
+static int bond_slots(dem_bonds *b) {
+    if (b->slots >= 0) return DEM_OK;
+    dem_ctx *ctx = b->s->ctx;
+    int *out = reinterpret_cast<int *>(b->d_count), most = 0;
+    CK(cudaMemsetAsync(out, 0, sizeof(int), ctx->stream));
+    k_max_i<<<kGS, kTB, 0, ctx->stream>>>(b->B.count, b->s->p->P.n, out);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(&most, out, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    if (most != b->slots) b->graph_version = -1;   // the captured step holds the old one
+    b->slots = most;
+    return DEM_OK;
+}
+
 extern "C" int dem_bonded_run(dem_bonds *b, int nsteps) {
     if (!b) return DEM_ERR_INVALID;
     if (nsteps <= 0) return DEM_OK;
@@ -2366,6 +2391,23 @@ extern "C" int dem_bonded_run(dem_bonds *b, int nsteps) {
     launch_prologue(s->p->P, s->p->ctl, s->fc, st);
     s->launches += 2;
     CK(cudaGetLastError());
+    const int sst = bond_slots(b);
+    if (sst) return sst;
+    // small specimens: the run in one cooperative launch
+    if (s->loop && s->sp.cooperative_loop != 2 && !b->loop_refused && s->p->P.n <= bond_loop_capacity(b->B, b->bc, b->slots)) {
+        if (!s->d_coop) CK(dalloc(&s->d_coop, (size_t)kCoopScratch));
+        if (launch_bond_loop(s->p->P, b->B, s->p->ctl, s->fc, b->bc, nsteps, s->d_coop, st) != cudaSuccess) {
+            (void)cudaGetLastError();   // not resident at once, or refused: the step graph
+            b->loop_refused = true;
+        } else {
+            s->launches += 1;
+            const Ctl c = read_ctl(s);
+            CK(cudaGetLastError());
+            if (c.status & DEM_ERR_TIMEOUT) return fail(ctx, DEM_ERR_TIMEOUT, "a bounded device wait gave up");
+            if (c.steps_done >= c.target) return c.status & (DEM_ERR_BOND_OVERFLOW | DEM_ERR_NAN);
+            return fail(ctx, DEM_ERR_CUDA, "dem_bonded_run made no progress");
+        }
+    }
     const int chunk = s->sp.steps_per_launch;
     if (!b->graph || b->graph_version != s->version || b->graph_steps != chunk) {
         if (b->graph) {
@@ -2376,7 +2418,7 @@ extern "C" int dem_bonded_run(dem_bonds *b, int nsteps) {
             cudaGraph_t g = nullptr;
             cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
             if (e != cudaSuccess) return e;
-            for (int k = 0; k < chunk; ++k) launch_bond_step(s->p->P, b->B, s->p->ctl, s->fc, b->bc, st);
+            for (int k = 0; k < chunk; ++k) launch_bond_step(s->p->P, b->B, s->p->ctl, s->fc, b->bc, b->slots, st);
             e = cudaStreamEndCapture(st, &g);
             if (e != cudaSuccess) return e;
             e = cudaGraphInstantiate(&b->graph, g, 0);
@@ -2398,6 +2440,7 @@ extern "C" int dem_bonded_run(dem_bonds *b, int nsteps) {
         CK(cudaGraphLaunch(b->graph, st));
         s->launches += chunk;
         Ctl c = read_ctl(s);
+        if (c.status & DEM_ERR_TIMEOUT) return fail(ctx, DEM_ERR_TIMEOUT, "a bounded device wait gave up");
         if (c.steps_done >= c.target) return c.status & (DEM_ERR_BOND_OVERFLOW | DEM_ERR_NAN);
     }
     return fail(ctx, DEM_ERR_CUDA, "dem_bonded_run made no progress");

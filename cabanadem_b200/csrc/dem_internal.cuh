@@ -271,8 +271,13 @@ struct BondConsts {
 
 // ---- launchers (dem_bonded.cu) ----------------------------------------------------
 void launch_bond_setup(const Particles &P, const NbrList &L, const Bonds &B, Ctl *ctl, double factor, cudaStream_t s);
-void launch_bond_step(const Particles &P, const Bonds &B, Ctl *ctl, const ForceConsts &fc, const BondConsts &bc,
+void launch_bond_step(const Particles &P, const Bonds &B, Ctl *ctl, const ForceConsts &fc, const BondConsts &bc, int slots,
                       cudaStream_t s);
+// A run of at most bond_loop_capacity particles in one cooperative launch (scratch as for
+// launch_steps_live).
+int bond_loop_capacity(const Bonds &B, const BondConsts &bc, int slots);
+cudaError_t launch_bond_loop(const Particles &P, const Bonds &B, Ctl *ctl, const ForceConsts &fc, const BondConsts &bc,
+                             int max_steps, unsigned long long *scratch, cudaStream_t s);
 void launch_bond_broken_count(const Bonds &B, int n, unsigned long long *out, cudaStream_t s);
 void launch_bond_force(const Particles &P, const Bonds &B, Ctl *ctl, const BondConsts &bc, double dt, cudaStream_t s);
 void launch_add_ext_force(const Particles &P, cudaStream_t s);

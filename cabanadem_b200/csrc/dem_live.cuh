@@ -16,12 +16,6 @@
 // instructions of a contact, staged through shared memory, where a thread has its own state at hand.
 // What bounds it: the barrier (1.2 us) and the chain of one contact's divisions and square roots.
 //
-// Barrier: three rotating 16-byte words (scratch, zeroed before the launch): arrivals and the
-// step's count of particles in contact, and the bits of the step's largest |u|^2.  A block folds
-// its maximum, then arrives with a release; one atomic 16-byte acquire load polls both (bounded).
-// Block 0 clears the word of step k + 1 during step k: its last pollers (step k - 2) have arrived
-// at the barrier of step k - 1.  Every block takes the same decisions from those words.
-//
 // Velocities alternate between two buffers, since a contact reads its partner's velocities of the
 // step; only particles in contact are read, so a free particle's spin, which does not change, is
 // copied over only in the step after a contact.
@@ -31,8 +25,8 @@
 // afterwards by the steps taken.  The second buffer is then the deferred-velocity arrays, and the
 // bound on the quiet ones' speed enters the displacement bound.
 #pragma once
+#include "dem_gridstep.cuh"
 #include "dem_particle.cuh"
-#include "dem_persist.cuh"
 
 namespace b200dem {
 namespace {
@@ -231,38 +225,13 @@ __device__ __forceinline__ void live_contact(const Particles &P, const NbrList &
     }
 }
 
-__device__ __forceinline__ void ld_acquire_b128(const void *p, unsigned long long &lo, unsigned long long &hi) {
-    asm volatile(
-        "{\n\t"
-        ".reg .b128 t;\n\t"
-        "ld.acquire.gpu.global.b128 t, [%2];\n\t"
-        "mov.b128 {%0, %1}, t;\n\t"
-        "}\n"
-        : "=l"(lo), "=l"(hi)
-        : "l"(p)
-        : "memory");
-}
-
-// Largest of the warp's non-negative doubles, exactly: the high words, then the low words of those
-// that share the largest high word.
-__device__ __forceinline__ unsigned long long warp_max_bits(double v) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-    const unsigned hi = (unsigned)(b >> 32);
-    const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
-    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)b : 0u);
-    return ((unsigned long long)mh << 32) | ml;
-}
-
 template <bool MIXED>
 __global__ void __launch_bounds__(kBlock, 3) k_steps_live(Particles P, NbrList L, Ctl *ctl, ForceConsts fc,
                                                           const PairConst *__restrict__ pp,
                                                           const PairConst *__restrict__ pw,
                                                           const WallGeom *__restrict__ walls, int max_steps,
                                                           unsigned long long *scratch, int quiet) {
-    constexpr int W = kBlock / 32;
-    __shared__ unsigned long long s_vmax[W], s_arr, s_v2;
-    __shared__ int s_cnt[W];
-    const int G = gridDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ GridStep<kBlock> bar;
     const int n = P.n, cap = P.cap;
     const int cur0 = ctl->cur, vcur0 = ctl->vcur, target = ctl->target;
     const int first = quiet ? ctl->nlone + ctl->nclear : 0;
@@ -359,44 +328,11 @@ __global__ void __launch_bounds__(kBlock, 3) k_steps_live(Particles P, NbrList L
             }
         }
         const unsigned busy = __ballot_sync(0xffffffffu, full);
-        if (lane == 0) s_cnt[warp] = __popc(busy);
         if (status) atomicOr(&ctl->status, status);
-        const unsigned long long vb = warp_max_bits(v2);
-        if (lane == 0) s_vmax[warp] = vb;
-        __syncthreads();
-        unsigned long long *slot = scratch + 2 * (k % 3);
-        if (threadIdx.x == 0) {
-            unsigned long long vm = s_vmax[0];
-            int c = s_cnt[0];
-            for (int q = 1; q < W; ++q) {
-                vm = s_vmax[q] > vm ? s_vmax[q] : vm;
-                c += s_cnt[q];
-            }
-            if (blockIdx.x == 0) {
-                unsigned long long *nxt = scratch + 2 * ((k + 1) % 3);
-                nxt[0] = 0ull;
-                nxt[1] = 0ull;
-            }
-            if (vm) atomicMax(&slot[1], vm);
-            // the block's writes before its arrival
-            asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(slot), "l"(1ull + ((unsigned long long)c << 32))
-                         : "memory");
-            unsigned long long arr, big;
-            int p = 0;
-            do ld_acquire_b128(slot, arr, big);
-            while ((unsigned)arr < (unsigned)G && ++p < kCoopWaitPolls);
-            if (p == kCoopWaitPolls) {
-                atomicOr(&ctl->status, DEM_ERR_TIMEOUT);
-                arr = ~0ull;
-            }
-            s_arr = arr;
-            s_v2 = big;
-        }
-        __syncthreads();   // every block has arrived (or this one gave up)
-        ok = s_arr != ~0ull;
+        unsigned long long big;
+        ok = grid_step<kBlock>(bar, ctl, scratch, k, v2, __popc(busy), big, ncon);
         if (!ok) break;
-        ncon = (int)(s_arr >> 32);
-        double v = sqrt(__longlong_as_double((long long)s_v2));
+        double v = sqrt(__longlong_as_double((long long)big));
         if (quiet) v = fmax(v, vq + (k + 1) * fc.dt * ga * (1.0 + 1e-9));
         disp = disp + fc.dt * v * (1.0 + 1e-9);
         cur ^= 1;
