@@ -69,16 +69,36 @@ __global__ void k_bbox(Particles P, const Ctl *ctl, unsigned long long *bb) {
         else if (threadIdx.x < 7) atomicMax(&bb[threadIdx.x], s[threadIdx.x]);
         return;
     }
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P.n; i += gridDim.x * blockDim.x) {
-        const D4 p = ld4(P.pos[cur], i);
-        unsigned long long *w = bb + 8L * P.scene[i];
-        atomicMin(&w[0], ord(p.x));
-        atomicMin(&w[1], ord(p.y));
-        atomicMin(&w[2], ord(p.z));
-        atomicMax(&w[3], ord(p.x));
-        atomicMax(&w[4], ord(p.y));
-        atomicMax(&w[5], ord(p.z));
-        atomicMax(&w[6], ord(p.w));
+    // many scenes: a warp whose particles share one (the usual case in storage order) reduces before
+    // its seven atomics; one per particle queued 40,000 on a word at 4 scenes (178 us, now 5)
+    for (int i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); i0 < P.n; i0 += gridDim.x * blockDim.x) {
+        const int i = i0 + (threadIdx.x & 31);
+        const bool in = i < P.n;
+        const int s = in ? P.scene[i] : -1;
+        const D4 p = in ? ld4(P.pos[cur], i) : D4{0., 0., 0., 0.};
+        const unsigned long long v[4] = {ord(p.x), ord(p.y), ord(p.z), ord(p.w)};
+        const int s0 = __shfl_sync(0xffffffffu, s, 0);
+        if (__all_sync(0xffffffffu, s == s0 || !in)) {
+            for (int k = 0; k < 4; ++k) {
+                unsigned long long lo = in ? v[k] : ~0ull, hi = in ? v[k] : 0ull;
+                for (int o = 16; o > 0; o >>= 1) {
+                    const unsigned long long a = __shfl_xor_sync(0xffffffffu, lo, o), b = __shfl_xor_sync(0xffffffffu, hi, o);
+                    lo = a < lo ? a : lo;
+                    hi = b > hi ? b : hi;
+                }
+                if ((threadIdx.x & 31) == 0) {
+                    unsigned long long *w = bb + 8L * s0;
+                    if (k < 3) atomicMin(&w[k], lo);
+                    atomicMax(&w[3 + k], hi);
+                }
+            }
+        } else if (in) {
+            unsigned long long *w = bb + 8L * s;
+            for (int k = 0; k < 4; ++k) {
+                if (k < 3) atomicMin(&w[k], v[k]);
+                atomicMax(&w[3 + k], v[k]);
+            }
+        }
     }
 }
 

@@ -570,6 +570,21 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_wgrad(WgradArgs a) {
     tc_teardown(tm, TC, ok, a.err, mbar, phase);
 }
 
+// p[0] + p[stride] + ... over the blocks in order, eight loads in flight.
+__device__ __forceinline__ float sum_blocks(const float *p, long stride, int nblocks) {
+    float s = 0.f;
+    int b = 0;
+    for (; b + 8 <= nblocks; b += 8) {
+        float v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = p[(b + k) * stride];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s += v[k];
+    }
+    for (; b < nblocks; ++b) s += p[b * stride];
+    return s;
+}
+
 // Sum the per-CTA partials in block order and add them to the gradient buffers:
 // g_w1t [128][KIN], g_b1 [128], g_w2t [NOUT][128], g_b2 [NOUT].
 __global__ void k_wgrad_reduce(const float *part, int nblocks, int kin, int nout, float *g_w1t, int ld_w1, float *g_b1,
@@ -578,8 +593,7 @@ __global__ void k_wgrad_reduce(const float *part, int nblocks, int kin, int nout
     const int nc = kin + nw2 + 2;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < kRows * nc; e += gridDim.x * blockDim.x) {
         const int r = e / nc, c = e % nc;
-        float s = 0.f;
-        for (int b = 0; b < nblocks; ++b) s += part[((long)b * kRows + r) * nc + c];
+        const float s = sum_blocks(part + (long)r * nc + c, (long)kRows * nc, nblocks);
         if (c < kin) g_w1t[(long)r * ld_w1 + c] += s;
         else if (c < kin + nw2) {
             const int cc = c - kin;
@@ -1037,9 +1051,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_linear_wgrad(LinWgradArgs a) {
 __global__ void k_linw_reduce(const float *part, int nblocks, float *g, int ld, int col0) {
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < kRows * 256; e += gridDim.x * blockDim.x) {
         const int o = e / 256, c = e % 256;
-        float s = 0.f;
-        for (int b = 0; b < nblocks; ++b) s += part[((long)b * kRows + o) * 256 + c];
-        g[(long)o * ld + col0 + c] += s;
+        g[(long)o * ld + col0 + c] += sum_blocks(part + (long)o * 256 + c, kRows * 256L, nblocks);
     }
 }
 
@@ -1132,7 +1144,9 @@ int nn_mlp_backward(const dem_nn_mlp &m, long rows, const dem_nn_rows *src, int 
     B200_NN_SHAPES(X)
 #undef X
     if (st != DEM_OK || rows <= 0) return st;
-    k_wgrad_reduce<<<64, 256, 0, s>>>(part, nblocks, m.kin, m.nout, g_w1t, ld_w1, g_b1, g_w2t, g_b2);
+    // a thread per element: 64 blocks that looped over them took 62 us on average
+    const int nc = m.kin + (m.nout == kHidden ? kHidden : m.nout) + 2;
+    k_wgrad_reduce<<<(kRows * nc + 127) / 128, 128, 0, s>>>(part, nblocks, m.kin, m.nout, g_w1t, ld_w1, g_b1, g_w2t, g_b2);
     return cudaGetLastError() == cudaSuccess ? DEM_OK : DEM_ERR_CUDA;
 }
 
@@ -1156,7 +1170,7 @@ int nn_linear_pq_wgrad(long rows, const void *dpq, const void *h, float *g_w1t, 
     const int st = launch_tc(k_linear_wgrad, linw_smem(), 256, rows, a, s);
     if (st) return st;
     const long ntiles = (rows + kRows - 1) / kRows;
-    k_linw_reduce<<<64, 256, 0, s>>>(part, (int)(ntiles < 148 ? ntiles : 148), g_w1t, ld, col0);
+    k_linw_reduce<<<kRows * 256 / 128, 128, 0, s>>>(part, (int)(ntiles < 148 ? ntiles : 148), g_w1t, ld, col0);
     return cudaGetLastError() == cudaSuccess ? DEM_OK : DEM_ERR_CUDA;
 }
 

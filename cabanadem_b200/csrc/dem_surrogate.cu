@@ -239,23 +239,36 @@ __global__ void k_segsum(int n, const int *offs, const bf16 *ev, bf16 *agg) {
     }
 }
 
-// de[e] (=|+=) dn[recv[e]][c0:c0+128]
-__global__ void k_edge_from_node(int ne, const int *recv, const float *dn, int ld, int c0, float *de, int accumulate) {
+// One pass over the edges' gradient between two layers of the backward pass: de (0 when `first`) +
+// dxe, the input gradient of the message layer above (null: none), + the receiver's aggregate gradient
+// dn[recv[e]][128:256] (null: none), in that order; stored in FP32 (unless it is the last pass) and as
+// the BF16 upstream gradient of the next layer.
+__global__ void k_edge_grad(int ne, const int *recv, const float *dn, const float *dxe, float *de, bf16 *dyb, int first) {
     for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < (long)ne * (kH / 4); q += (long)gridDim.x * blockDim.x) {
         const long e = q / (kH / 4);
         const int c = (int)(q % (kH / 4)) * 4;
-        const float4 a = *reinterpret_cast<const float4 *>(dn + (long)recv[e] * ld + c0 + c);
-        float4 *d = reinterpret_cast<float4 *>(de + e * kH + c);
-        if (accumulate) {
-            float4 v = *d;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!first) v = *reinterpret_cast<const float4 *>(de + e * kH + c);
+        if (dxe) {
+            const float4 a = *reinterpret_cast<const float4 *>(dxe + e * kH + c);
             v.x += a.x;
             v.y += a.y;
             v.z += a.z;
             v.w += a.w;
-            *d = v;
-        } else {
-            *d = a;
         }
+        if (dn) {
+            const float4 a = *reinterpret_cast<const float4 *>(dn + (long)recv[e] * 2 * kH + kH + c);
+            v.x += a.x;
+            v.y += a.y;
+            v.z += a.z;
+            v.w += a.w;
+            *reinterpret_cast<float4 *>(de + e * kH + c) = v;
+        }
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+        uint2 o;
+        o.x = *reinterpret_cast<const uint32_t *>(&lo);
+        o.y = *reinterpret_cast<const uint32_t *>(&hi);
+        *reinterpret_cast<uint2 *>(dyb + e * kH + c) = o;
     }
 }
 
@@ -281,7 +294,7 @@ __global__ void k_f2bf(long count, const float *src, bf16 *dst) {
 }
 
 // ---- loss: mean over nodes and the 2 components of (a - target)^2 ----
-constexpr int kLossBlocks = 256;
+constexpr int kLossBlocks = 256;   // at most kTB (k_sum_parts)
 __global__ void k_loss(int n, const float *out, const double4 *pk, const double2 *disp, const double *next,
                        double inv_sa, bf16 *dout, double *part) {
     __shared__ double s[kTB];
@@ -305,12 +318,16 @@ __global__ void k_loss(int n, const float *out, const double4 *pk, const double2
     }
     if (threadIdx.x == 0) part[blockIdx.x] = s[0] * scale;
 }
+// The sum of nb <= kTB partials, in a fixed tree (one block).
 __global__ void k_sum_parts(int nb, const double *part, double *out) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double s = 0.0;
-        for (int b = 0; b < nb; ++b) s += part[b];
-        *out = s;
+    __shared__ double s[kTB];
+    s[threadIdx.x] = threadIdx.x < nb ? part[threadIdx.x] : 0.0;
+    __syncthreads();
+    for (int o = kTB / 2; o > 0; o >>= 1) {
+        if (threadIdx.x < o) s[threadIdx.x] += s[threadIdx.x + o];
+        __syncthreads();
     }
+    if (threadIdx.x == 0) *out = s[0];
 }
 
 // ---- Adam + BF16 refresh ----
@@ -772,7 +789,7 @@ int build_graph(dem_surrogate *sg, int n, const int *frame, int nframes, bool tr
     int st = ensure_edges(sg, total, training);
     if (st) return st;
     k_csr_fill<<<kGS, kTB, 0, s>>>(n, sg->cap, sg->L.nn, sg->L.idx, sg->offs, sg->recv, sg->send);
-    k_csr_rev<<<kGS, kTB, 0, s>>>(total, sg->recv, sg->send, sg->offs, sg->rev);
+    if (training) k_csr_rev<<<kGS, kTB, 0, s>>>(total, sg->recv, sg->send, sg->offs, sg->rev);   // the backward pass's
     SCK(cudaGetLastError());
     *ne_out = total;
     return DEM_OK;
@@ -892,7 +909,6 @@ int backward(dem_surrogate *sg, int n, long ne) {
         dem_nn_rows ds{sg->h[3], nullptr, kH};
         SG(mlp_bwd(sg, L_DEC, n, &ds, 1, sg->dout, sg->dh));
     }
-    SCK(cudaMemsetAsync(sg->de, 0, sizeof(float) * (size_t)std::max<long>(ne, 1) * kH, s));
     for (int l = 2; l >= 0; --l) {
         // h_{l+1} = h_l + Upd[h_l, agg_l]
         k_f2bf<<<kGS, kTB, 0, s>>>((long)n * kH, sg->dh, sg->dyb);
@@ -900,16 +916,14 @@ int backward(dem_surrogate *sg, int n, long ne) {
         SG(mlp_bwd(sg, L_UPD(l), n, us, 2, sg->dyb, sg->dxn));
         k_add_cols<<<kGS, kTB, 0, s>>>(n, sg->dxn, 256, 0, sg->dh);            // dh_l = dh_{l+1} + dUpd/dh_l
         if (ne > 0) {
-            // agg_l = sum over edges of e_{l+1}: de_{l+1} += dagg[recv]
-            k_edge_from_node<<<kGS, kTB, 0, s>>>((int)ne, sg->recv, sg->dxn, 256, 128, sg->de, 1);
-            // e_{l+1} = e_l + Msg[e_l, h_l[recv], h_l[send]]
-            k_f2bf<<<kGS, kTB, 0, s>>>(ne * kH, sg->de, sg->dyb);
+            // agg_l = sum over edges of e_{l+1}: de_{l+1} += dagg[recv], after the layer above's
+            // de_{l+1} += dMsg/de_{l+1}; then e_{l+1} = e_l + Msg[e_l, h_l[recv], h_l[send]]
+            k_edge_grad<<<kGS, kTB, 0, s>>>((int)ne, sg->recv, sg->dxn, l < 2 ? sg->dxe : nullptr, sg->de, sg->dyb, l == 2);
             SG(msg_bwd(sg, L_MSG(l), n, ne, sg->h[l], sg->e[l], sg->dyb, sg->dh));   // dh += dMsg/dh_l
-            k_add_cols<<<kGS, kTB, 0, s>>>(ne, sg->dxe, kH, 0, sg->de);       // de_l = de_{l+1} + dMsg/de_l
         }
     }
     if (ne > 0) {
-        k_f2bf<<<kGS, kTB, 0, s>>>(ne * kH, sg->de, sg->dyb);
+        k_edge_grad<<<kGS, kTB, 0, s>>>((int)ne, sg->recv, nullptr, sg->dxe, sg->de, sg->dyb, 0);
         dem_nn_rows xe{sg->xe, nullptr, kF};
         SG(mlp_bwd(sg, L_ENC_E, ne, &xe, 1, sg->dyb, nullptr));
     }
@@ -938,7 +952,7 @@ int loss_grad(dem_surrogate *sg, int n, const double *prev, const double *cur, c
     SG(forward(sg, n, ne, true));
     cudaStream_t s = ctx_stream(sg->ctx);
     k_loss<<<kLossBlocks, kTB, 0, s>>>(n, sg->out, sg->packed, sg->disp, next, 1.0 / sg->prm.sigma_a, sg->dout, sg->part);
-    k_sum_parts<<<1, 32, 0, s>>>(kLossBlocks, sg->part, sg->d_loss);
+    k_sum_parts<<<1, kTB, 0, s>>>(kLossBlocks, sg->part, sg->d_loss);
     SG(backward(sg, n, ne));
     SCK(cudaMemcpyAsync(loss, sg->d_loss, sizeof(double), cudaMemcpyDeviceToHost, s));
     SCK(cudaStreamSynchronize(s));
@@ -948,6 +962,22 @@ int loss_grad(dem_surrogate *sg, int n, const double *prev, const double *cur, c
     int e = 0;
     SCK(cudaMemcpy(&e, err, sizeof(int), cudaMemcpyDeviceToHost));
     if (e) return sg_fail(sg, e, "surrogate: tensor-core kernel gave up waiting");
+    return DEM_OK;
+}
+
+// Caller-order scratch of the rollout (and, of it, predict's projection), kept between calls.
+int ensure_rollout(dem_surrogate *sg, int n) {
+    if (sg->roll_n < n) {
+        cudaFree(sg->x_prev); cudaFree(sg->x_cur); cudaFree(sg->x_next); cudaFree(sg->x_tmp); cudaFree(sg->rad);
+        cudaFree(sg->mass);
+        SCK(dmalloc(&sg->x_prev, 3 * (size_t)n));
+        SCK(dmalloc(&sg->x_tmp, 3 * (size_t)n));
+        SCK(dmalloc(&sg->x_cur, 3 * (size_t)n));
+        SCK(dmalloc(&sg->x_next, 3 * (size_t)n));
+        SCK(dmalloc(&sg->rad, n));
+        SCK(dmalloc(&sg->mass, n));
+        sg->roll_n = n;
+    }
     return DEM_OK;
 }
 
@@ -1164,15 +1194,9 @@ extern "C" int dem_surrogate_predict(dem_surrogate *sg, int n, const double *pos
     cudaStream_t s = ctx_stream(sg->ctx);
     k_integrate<<<kGS, kTB, 0, s>>>(n, sg->packed, sg->disp, sg->out, sg->prm.sigma_a, sg->fc, pos_cur, pos_next);
     if (sg->prm.project_iters > 0) {
-        double *tmp = nullptr, *w = nullptr;
-        SCK(dmalloc(&tmp, 3 * (size_t)n));
-        SCK(dmalloc(&w, (size_t)n));
-        k_rad3<<<kGS, kTB, 0, s>>>(n, rad, w);   // mass weights of equal-density particles
-        const int st = project(sg, n, pos_next, tmp, rad, w);
-        SCK(cudaStreamSynchronize(s));
-        cudaFree(tmp);
-        cudaFree(w);
-        if (st) return st;
+        SG(ensure_rollout(sg, n));
+        k_rad3<<<kGS, kTB, 0, s>>>(n, rad, sg->mass);   // mass weights of equal-density particles
+        SG(project(sg, n, pos_next, sg->x_tmp, rad, sg->mass));
     }
     SCK(cudaGetLastError());
     SCK(cudaStreamSynchronize(s));
@@ -1189,17 +1213,7 @@ extern "C" int dem_surrogate_rollout(dem_surrogate *sg, dem_solver *solver, int 
     SG(ensure_nodes(sg, n, 1));
     cudaStream_t s = ctx_stream(sg->ctx);
     if (V.stream != s) return sg_fail(sg, DEM_ERR_INVALID, "dem_surrogate_rollout: solver and surrogate need one context");
-    if (sg->roll_n < n) {
-        cudaFree(sg->x_prev); cudaFree(sg->x_cur); cudaFree(sg->x_next); cudaFree(sg->x_tmp); cudaFree(sg->rad);
-        cudaFree(sg->mass);
-        SCK(dmalloc(&sg->x_prev, 3 * (size_t)n));
-        SCK(dmalloc(&sg->x_tmp, 3 * (size_t)n));
-        SCK(dmalloc(&sg->x_cur, 3 * (size_t)n));
-        SCK(dmalloc(&sg->x_next, 3 * (size_t)n));
-        SCK(dmalloc(&sg->rad, n));
-        SCK(dmalloc(&sg->mass, n));
-        sg->roll_n = n;
-    }
+    SG(ensure_rollout(sg, n));
     const int steps = sg->prm.steps_per_stride;
     const double T = steps * sg->prm.dt;
     auto dem_stride = [&]() -> int {
