@@ -815,33 +815,99 @@ __global__ void __launch_bounds__(kFwdThreads, 2) k_edge_fwd(EdgeArgs a) {
 }
 
 // The same layer with its row tiles brought in by the tensor copy engine and the hidden tile
-// kept in tensor memory, so that the next tile's input is in flight during this tile's
-// products and epilogues.  Per CTA (two per SM, 256 threads): the e tile of 128 rows arrives as
+// kept in tensor memory.  One CTA of 512 threads per SM: two groups of 256, each with a tile of its
+// own in flight (its e tile, accumulator, barriers), share the weights.  Per tile the e rows arrive as
 // two 64-feature boxes of a tiled tensor copy in the 128-byte swizzle layout (one elected thread
 // issues them on an mbarrier, one tile ahead: as soon as the first product of the current tile
 // has read the buffer); the first product reads it from shared memory; the epilogue writes the
 // hidden activations as BF16 pairs into tensor memory (tcgen05.st), which is the A operand of
-// the second product; the second epilogue stores each thread's half row straight to global
-// memory.  Same arithmetic, in the same order, as k_edge_fwd.
-constexpr size_t edge_tma_smem() { return 1024 + 3 * (size_t)kRows * kHidden * 2 + 64; }
+// the second product.  Same arithmetic, in the same order, as k_edge_fwd.
+//
+// Rows reach and leave the threads through a 4 KB buffer per warp: eight lanes read or write one
+// row's 128 bytes in global memory, and a thread takes its own row's eight chunks from the buffer
+// (chunks XOR-swizzled by the row, no bank conflicts).  A thread reading its own row directly touched
+// 32 lines per instruction: P, Q, residual and output rows then cost 1,024 L1 wavefronts per warp and
+// tile, and two CTAs per SM spent three quarters of their time on them; now 384.  1.2 M edges (B200):
+// see nn_edge_forward.
+constexpr int kEdgeThreads = 512, kEdgeGroup = 256;
+constexpr size_t edge_tma_smem() {
+    return 1024 + 4 * (size_t)kRows * kHidden * 2 + (size_t)(kEdgeThreads / 32) * 4096 + 128;
+}
 
-__global__ void __launch_bounds__(kFwdThreads, 2) k_edge_fwd_tma(const __grid_constant__ CUtensorMap tm_e, EdgeArgs a) {
+// Barrier of one group of 256 threads (ids 1 and 2), and the same with a vote.
+__device__ __forceinline__ void group_sync(int id) { asm volatile("bar.sync %0, 256;" ::"r"(id) : "memory"); }
+__device__ __forceinline__ bool group_and(int id, bool p) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t"
+        ".reg .pred a, b;\n\t"
+        "setp.ne.u32 a, %1, 0;\n\t"
+        "bar.red.and.pred b, %2, 256, a;\n\t"
+        "selp.u32 %0, 1, 0, b;\n\t"
+        "}\n"
+        : "=r"(r)
+        : "r"(p ? 1u : 0u), "r"(id)
+        : "memory");
+    return r != 0;
+}
+
+// A warp's 32 half rows of 64 features, row r of lane r: coalesced between global memory and the
+// buffer (row_in_lane: the row, of the lane's 4 k + lane / 8, chunk lane % 8), own rows between the
+// buffer and registers.
+__device__ __forceinline__ unsigned char *warp_chunk(unsigned char *buf, int row, int c) {
+    return buf + row * 128 + ((c ^ (row & 7)) << 4);
+}
+__device__ __forceinline__ void warp_rows_issue(const bf16 *base, long stride, int own_row, uint4 v[8]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const long r = __shfl_sync(0xffffffffu, own_row, 4 * k + (lane >> 3));
+        v[k] = *reinterpret_cast<const uint4 *>(base + r * stride + (lane & 7) * 8);
+    }
+}
+__device__ __forceinline__ void warp_rows_take(unsigned char *buf, const uint4 v[8], uint4 own[8]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) *reinterpret_cast<uint4 *>(warp_chunk(buf, 4 * k + (lane >> 3), lane & 7)) = v[k];
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < 8; ++c) own[c] = *reinterpret_cast<const uint4 *>(warp_chunk(buf, lane, c));
+    __syncwarp();
+}
+__device__ __forceinline__ void warp_rows_store(unsigned char *buf, const uint4 own[8], bf16 *g, long row0, long rows) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4 *>(warp_chunk(buf, lane, c)) = own[c];
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const int row = 4 * k + (lane >> 3);
+        if (row0 + row < rows)
+            *reinterpret_cast<uint4 *>(g + (row0 + row) * kHidden + (lane & 7) * 8) =
+                *reinterpret_cast<const uint4 *>(warp_chunk(buf, row, lane & 7));
+    }
+    __syncwarp();
+}
+
+__global__ void __launch_bounds__(kEdgeThreads, 1) k_edge_fwd_tma(const __grid_constant__ CUtensorMap tm_e, EdgeArgs a) {
     // 1,024-byte alignment by hand: an extern array declared with it would raise the alignment of
     // every kernel's dynamic shared memory in this file (and their static padding with it)
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr uint32_t T = (uint32_t)kRows * kHidden * 2;   // one 128 x 128 BF16 tile
-    unsigned char *sE = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);   // 1,024-byte aligned
-    unsigned char *sW1 = sE + T;   // W1e^T 128 x 128 (row tile)
-    unsigned char *sW2 = sW1 + T;  // W2^T 128 x 128 (row tile)
-    uint64_t *bar_mma = reinterpret_cast<uint64_t *>(sW2 + T);
-    uint64_t *bar_e = bar_mma + 1;
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(bar_e + 1);
+    unsigned char *sE0 = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);   // 1,024-byte aligned
+    unsigned char *sW1 = sE0 + 2 * T;   // W1e^T 128 x 128 (row tile), after the groups' e tiles
+    unsigned char *sW2 = sW1 + T;       // W2^T 128 x 128 (row tile)
+    unsigned char *sBuf = sW2 + T;      // 4 KB per warp
+    uint64_t *bars = reinterpret_cast<uint64_t *>(sBuf + (kEdgeThreads / 32) * 4096);
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(bars + 4);
     __shared__ float s_b1[kHidden], s_b2[kHidden];
-    const int tid = threadIdx.x;
+    const int group = threadIdx.x / kEdgeGroup, tid = threadIdx.x % kEdgeGroup, bid = 1 + group;
     const int t = tid & (kRows - 1);   // tile row (TMEM lane)
     const int half = tid >> 7;         // features [64 half, 64 half + 64)
-    if (half == 0) s_b1[t] = a.b1[t];
-    else s_b2[t] = a.b2[t];
+    unsigned char *sE = sE0 + group * T, *buf = sBuf + (threadIdx.x >> 5) * 4096;
+    uint64_t *bar_mma = bars + 2 * group, *bar_e = bar_mma + 1;
+    if (threadIdx.x < kHidden) s_b1[threadIdx.x] = a.b1[threadIdx.x];
+    else if (threadIdx.x < 2 * kHidden) s_b2[threadIdx.x - kHidden] = a.b2[threadIdx.x - kHidden];
     stage_dense(sW1, a.w1e_t, kHidden, kHidden, 0, kHidden);
     stage_dense(sW2, a.w2t, kHidden, kHidden, 0, kHidden);
     cp_wait_all();
@@ -850,8 +916,8 @@ __global__ void __launch_bounds__(kFwdThreads, 2) k_edge_fwd_tma(const __grid_co
         tc::mbar_init(bar_e, 1);
         tc::mbar_init_fence();
     }
-    if (tid < 32) {
-        tc::tmem_alloc(tslot, 256);
+    if (threadIdx.x < 32) {
+        tc::tmem_alloc(tslot, 512);
         tc::tmem_relinquish();
     }
     tc::fence_async_smem();   // the weight tiles, complete, visible to the tensor core
@@ -859,40 +925,49 @@ __global__ void __launch_bounds__(kFwdThreads, 2) k_edge_fwd_tma(const __grid_co
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tm = *tslot;
-    const uint32_t tacc = tm;         // accumulator, 128 columns (both products)
-    const uint32_t ta = tm + 128;     // hidden tile as the second product's A operand, 64 columns
+    const uint32_t tacc = tm + 256u * group;   // accumulator, 128 columns (both products)
+    const uint32_t ta = tacc + 128;            // hidden tile as the second product's A operand, 64 columns
     const uint32_t aE = tc::smem_u32(sE), aW1 = tc::smem_u32(sW1), aW2 = tc::smem_u32(sW2);
     constexpr uint32_t id = tc::idesc_bf16(kRows, kHidden, false, false);
-    const long ntiles = (a.rows + kRows - 1) / kRows;
-    auto issue_e = [&](long tile) {   // thread 0: the tile's two feature boxes
+    const long ntiles = (a.rows + kRows - 1) / kRows, step = 2L * gridDim.x;
+    auto issue_e = [&](long tile) {   // the group's thread 0: the tile's two feature boxes
         tc::mbar_arrive_expect(bar_e, T);
         tc::tma_load_2d(sE, &tm_e, 0, (int)(tile * kRows), bar_e);
         tc::tma_load_2d(sE + T / 2, &tm_e, 64, (int)(tile * kRows), bar_e);
     };
     uint32_t ph_mma = 0, ph_e = 0;
-    bool ok = true, e_pending = false;   // e_pending: thread 0 has a tile copy not yet waited for
-    if (tid == 0 && (long)blockIdx.x < ntiles) {
-        issue_e(blockIdx.x);
+    bool ok = true, e_pending = false, mma_pending = false;   // of thread 0: not yet waited for
+    const long tile0 = 2L * blockIdx.x + group;
+    if (tid == 0 && tile0 < ntiles) {
+        issue_e(tile0);
         e_pending = true;
     }
-    for (long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const long row0 = tile * kRows, grow = row0 + t;
+    auto wait_mma = [&]() {
+        const bool w = tc::mbar_wait(bar_mma, ph_mma, g_tc_wait_limit);
+        const bool all = group_and(bid, w);
+        if (all) {
+            ph_mma ^= 1u;
+            mma_pending = false;
+        }
+        tc::fence_after_sync();
+        return all;
+    };
+    for (long tile = tile0; tile < ntiles; tile += step) {
+        const long row0 = tile * kRows, grow = row0 + t, wrow0 = row0 + (t & ~31);   // the warp's first row
         const bool live = grow < a.rows;
         uint4 p[8], q[8];
         {
-            const long r = live ? a.recv[grow] : 0, c = live ? a.send[grow] : 0;
-            const uint4 *ps = reinterpret_cast<const uint4 *>(a.pq + r * 2 * kHidden + half * 64);
-            const uint4 *qs = reinterpret_cast<const uint4 *>(a.pq + c * 2 * kHidden + kHidden + half * 64);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                p[k] = ps[k];
-                q[k] = qs[k];
-            }
+            const int r = live ? a.recv[grow] : 0, c = live ? a.send[grow] : 0;
+            uint4 vp[8], vq[8];
+            warp_rows_issue(a.pq + half * 64, 2 * kHidden, r, vp);
+            warp_rows_issue(a.pq + kHidden + half * 64, 2 * kHidden, c, vq);
+            warp_rows_take(buf, vp, p);
+            warp_rows_take(buf, vq, q);
         }
-        // the e tile; the block barrier also orders every thread's reads of the previous tile's
+        // the e tile; the group's barrier also orders every thread's reads of the previous tile's
         // accumulator before this tile's first product
         const bool e_ok = tc::mbar_wait(bar_e, ph_e, g_tc_wait_limit);
-        if (!__syncthreads_and(e_ok)) {
+        if (!group_and(bid, e_ok)) {
             ok = false;
             break;
         }
@@ -904,14 +979,16 @@ __global__ void __launch_bounds__(kFwdThreads, 2) k_edge_fwd_tma(const __grid_co
                 mma_issue(tacc, tc::sdesc_sw128(aE + (uint32_t)(ks >> 2) * (T / 2) + (uint32_t)(ks & 3) * 32u),
                           tc::kmajor_desc(aW1, kHidden, ks), id, ks > 0);
             mma_commit_issue(bar_mma);
+            mma_pending = true;
         }
-        ok = mma_wait(bar_mma, ph_mma);
+        ok = wait_mma();
         if (!ok) break;
         // the first product has read the e tile: the next tile's copy goes into its buffer
-        if (tid == 0 && tile + gridDim.x < ntiles) {
-            issue_e(tile + gridDim.x);
+        if (tid == 0 && tile + step < ntiles) {
+            issue_e(tile + step);
             e_pending = true;
         }
+        uint4 hv[8];   // the thread's hidden half row
 #pragma unroll
         for (int b = 0; b < 2; ++b) {   // two batches of 32 columns keep the P/Q registers live
             float w[32];
@@ -938,30 +1015,29 @@ __global__ void __launch_bounds__(kFwdThreads, 2) k_edge_fwd_tma(const __grid_co
                 hw[8 * c2 + 5] = hi.y;
                 hw[8 * c2 + 6] = hi.z;
                 hw[8 * c2 + 7] = hi.w;
-                if (a.h1 && live) {
-                    uint4 *dst = reinterpret_cast<uint4 *>(a.h1 + grow * kHidden + c * 16);
-                    dst[0] = lo;
-                    dst[1] = hi;
-                }
+                hv[2 * cc] = lo;
+                hv[2 * cc + 1] = hi;
             }
             // features [64 half + 32 b, + 32) as 16 columns of BF16 pairs
             tc::tmem_st16(tc::tmem_warp_addr(ta, half * 32 + b * 16), hw);
         }
         tc::tmem_wait_st();
         tc::fence_before_sync();
-        __syncthreads();
+        group_sync(bid);
         if (tid == 0) {
             tc::fence_after_sync();
             for (int ks = 0; ks < kHidden / 16; ++ks)
                 mma_issue_tmem_a(tacc, ta + (uint32_t)ks * 8u, tc::kmajor_desc(aW2, kHidden, ks), id, ks > 0);
             mma_commit_issue(bar_mma);
+            mma_pending = true;
         }
-        {   // residual half row while the second product runs
-            const uint4 *es = reinterpret_cast<const uint4 *>(a.e + (live ? grow : 0) * kHidden + half * 64);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) p[k] = es[k];
+        {   // hidden rows out (training) and the residual half row in, while the second product runs
+            uint4 v[8];
+            warp_rows_issue(a.e + half * 64, kHidden, live ? (int)grow : 0, v);
+            if (a.h1) warp_rows_store(buf, hv, a.h1 + half * 64, wrow0, a.rows);
+            warp_rows_take(buf, v, p);
         }
-        ok = mma_wait(bar_mma, ph_mma);
+        ok = wait_mma();
         if (!ok) break;
         {
             float w[64];
@@ -979,17 +1055,20 @@ __global__ void __launch_bounds__(kFwdThreads, 2) k_edge_fwd_tma(const __grid_co
                 o[2 * cc] = tc::pack8(v);
                 o[2 * cc + 1] = tc::pack8(v + 8);
             }
-            if (live) {
-                uint4 *dst = reinterpret_cast<uint4 *>(a.out + grow * kHidden + half * 64);
-#pragma unroll
-                for (int k = 0; k < 8; ++k) dst[k] = o[k];
-            }
+            warp_rows_store(buf, o, a.out + half * 64, wrow0, a.rows);
         }
         tc::fence_before_sync();
     }
-    // a wait gave up with a tile copy in flight: let it land before the block's memory goes
+    // a wait gave up: let the group's copy and product in flight land before the block's memory goes
     if (tid == 0 && e_pending) (void)tc::mbar_wait(bar_e, ph_e, g_tc_wait_limit);
-    tc_teardown(tm, 256, ok, a.err, bar_mma, ph_mma);
+    if (tid == 0 && mma_pending) (void)tc::mbar_wait(bar_mma, ph_mma, g_tc_wait_limit);
+    tc::fence_before_sync();
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        tc::fence_after_sync();
+        tc::tmem_dealloc(tm, 512);
+    }
+    if (!ok && tid == 0 && a.err) atomicOr(a.err, DEM_ERR_TIMEOUT);
 }
 
 // dW^T [256][128] partials: D_half[o][k] = sum_rows A[row][128 half + o] B[row][k]
@@ -1227,8 +1306,8 @@ int nn_edge_forward(long rows, const void *e, const void *pq, const int *recv, c
         int sms = 148, dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const long ntiles = (rows + kRows - 1) / kRows, cap = 2L * (sms > 0 ? sms : 148);   // two CTAs per SM
-        k_edge_fwd_tma<<<(int)(ntiles < cap ? ntiles : cap), kFwdThreads, smem, s>>>(m, a);
+        const long pairs = ((rows + kRows - 1) / kRows + 1) / 2, cap = sms > 0 ? sms : 148;   // a CTA steps two tiles
+        k_edge_fwd_tma<<<(int)(pairs < cap ? pairs : cap), kEdgeThreads, smem, s>>>(m, a);
         return cudaGetLastError() == cudaSuccess ? DEM_OK : DEM_ERR_CUDA;
     }
     return launch_tc(k_edge_fwd, edge_smem(), 128, rows, a, s, 0, kFwdThreads);
