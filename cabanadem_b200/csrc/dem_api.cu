@@ -107,6 +107,7 @@ struct dem_solver {
     bool quiet = false;                         // the current list's build found a quiet system
     int rest = 0;                               // its particles that are not quiet
     int quiet_wait = 0;                         // builds until quiet classes are tried again
+    bool live_off = false;                      // the last step was too dense for several particles per thread
     RefTables ref{};                            // cell tables of the rebuild-every-step loop
 };
 
@@ -1621,18 +1622,31 @@ int run_scenes(dem_solver *s, int nsteps) {
 }
 }  // namespace
 
+// Whether the cooperative launches keep each particle in a thread's registers (dem_live.cuh):
+// static walls, no mesh, at most the threads resident at once.
+bool live_form(const dem_solver *s) {
+    const int one = live_capacity(s->fc.mixed != 0);
+    return !s->fc.mwalls && s->mesh_nt == 0 &&
+           (s->p->P.n <= one || (s->p->P.n <= kLiveMany * one && !s->live_off));
+}
+// Particles in contact above which a step is not taken from memory by several per thread: their contacts
+// would follow one another in a thread.  Below it the loop is the faster one at every size it takes (device
+// us per step, three kernels / this loop, 176,000 spheres in scenes 25 / 14.4); a column with nearly all of
+// 65,000 disks in contact takes 54 us in one kernel per step and 66 with several per thread.
+int live_dense(const dem_solver *s) { return s->p->P.n / 16; }
+
 // The run's steps in cooperative launches (dem_persist.cuh) rather than graph replays: the
 // one-kernel step of a small system in the Verlet-skin mode, with the step loop in while-loop
 // graphs (steps_per_launch 0, so no profiler asked for fixed graphs).
 bool coop_loop(const dem_solver *s) {
-    return s->sp.cooperative_loop != 2 && !s->coop_refused && s->fc.all == 1 && s->p->P.n <= kCoopMaxN &&
-           s->loop && !ref_mode(s);
-}
-
-// Whether the cooperative launches keep each particle in a thread's registers (dem_live.cuh):
-// static walls, no mesh, at most the threads resident at once.
-bool live_form(const dem_solver *s) {
-    return !s->fc.mwalls && s->mesh_nt == 0 && s->p->P.n <= live_capacity(s->fc.mixed != 0);
+    if (s->sp.cooperative_loop == 2 || s->coop_refused || !s->loop || ref_mode(s)) return false;
+    if (s->fc.all == 1 && s->p->P.n <= kCoopMaxN) {
+        // dense and larger than one particle per resident thread: one kernel per step in a graph (a
+        // column of 65,000 disks, FP64 / FP32 forces: 54 / 32 us per step, 66 / 51 in one cooperative launch)
+        return s->fc.mwalls || s->mesh_nt > 0 || live_form(s);
+    }
+    // larger sparse systems, several particles per thread (dem_live.cuh)
+    return s->sp.contact_lanes == 0 && s->sp.dense_form == 0 && s->sp.stream_split == 0 && !s->fc.dense && live_form(s);
 }
 
 // The rebuild-every-step mode's run in one cooperative launch (dem_refloop.cuh): the one-kernel
@@ -1805,7 +1819,8 @@ extern "C" int dem_solver_run(dem_solver *s, int nsteps) {
                 CK(cudaEventRecord(s->ev0, st));
                 for (int b = 0; b < kFlightBatch && b * kFlightSteps < left; ++b) {
                     const cudaError_t le = launch_steps_live(s->p->P, s->L, s->p->ctl, s->fc, s->d_pp, s->d_pw,
-                                                             s->d_walls, s->rest, kFlightSteps, s->d_coop, 1, st);
+                                                             s->d_walls, s->rest, kFlightSteps, s->d_coop, 1,
+                                                             s->p->P.n, st);
                     if (le != cudaSuccess) {
                         (void)cudaGetLastError();
                         s->coop_refused = true;
@@ -1842,7 +1857,7 @@ extern "C" int dem_solver_run(dem_solver *s, int nsteps) {
                 const bool live = live_form(s);
                 const cudaError_t le =
                     live ? launch_steps_live(s->p->P, s->L, s->p->ctl, s->fc, s->d_pp, s->d_pw, s->d_walls, s->p->P.n,
-                                             nsteps, s->d_coop, 0, st)
+                                             nsteps, s->d_coop, 0, live_dense(s), st)
                          : launch_steps_coop(s->p->P, s->L, s->p->ctl, s->fc, s->d_pp, s->d_pw, s->d_walls, nsteps,
                                              s->d_coop, st);
                 if (le != cudaSuccess) {   // not resident at once (or refused): graph replays from here on
@@ -1862,10 +1877,16 @@ extern "C" int dem_solver_run(dem_solver *s, int nsteps) {
                 s->graph_ms += ms;
                 s->graph_steps_run += c.steps_done - done_before;
                 s->graph_done_mark = c.steps_done;
+                steps_before = c.steps_done;
+                if (live) s->live_off = c.last_ndefer > live_dense(s);
+                else if (c.last_ndefer < live_dense(s) / 4) s->live_off = false;
+                adapt_density(s, c);
                 if (c.steps_done >= c.target) break;
                 if (!(c.disp < c.half_skin)) {
                     int e = build_now(s, true);
                     if (e) return e;
+                } else if (s->live_off && !live_form(s)) {
+                    // the other forms from here on, until a step of theirs is sparse again
                 } else if (c.steps_done == done_before) {
                     return fail(ctx, DEM_ERR_CUDA, "solver made no progress");
                 }
@@ -1885,6 +1906,7 @@ extern "C" int dem_solver_run(dem_solver *s, int nsteps) {
             count_launches(c);
             if (c.status & DEM_ERR_TIMEOUT) return fail(ctx, DEM_ERR_TIMEOUT, "a bounded device wait gave up");
             adapt_density(s, c);
+            if (c.last_ndefer < live_dense(s) / 4) s->live_off = false;
             {
                 float ms = 0.f;
                 CK(cudaEventElapsedTime(&ms, s->ev0, s->ev1));

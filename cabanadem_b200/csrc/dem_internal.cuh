@@ -352,8 +352,8 @@ constexpr int kSceneMaxParticles = 64;   // largest scene of the persistent form
 // steps, ending at the target, a stale list or a stop bit.  An error when the launch is refused
 // (e.g. the grid cannot be resident at once).
 constexpr int kCoopMaxN = 65536;   // largest system the cooperative step loop takes
-// scratch: kCoopScratch words of device memory for the symmetric barrier (static walls, no
-// moving mesh).
+// scratch: kCoopScratch words of device memory for the symmetric barrier (static walls, a
+// mesh at rest).
 constexpr int kCoopScratch = 1 + 4 * (kCoopMaxN / 128);
 cudaError_t launch_steps_coop(const Particles &P, const NbrList &L, Ctl *ctl, const ForceConsts &fc, const PairConst *pp,
                               const PairConst *pw, const WallGeom *walls, int max_steps, unsigned long long *scratch,
@@ -362,16 +362,18 @@ cudaError_t launch_steps_coop_mixed(const Particles &P, const NbrList &L, Ctl *c
                                     const PairConst *pp, const PairConst *pw, const WallGeom *walls, int max_steps,
                                     unsigned long long *scratch, cudaStream_t s);
 // The same with each particle in a thread's registers (dem_live.cuh): static walls, no mesh, `count`
-// particles, at most live_capacity.  quiet: the particles [nlone + nclear, n) only (dem_flight.cuh).
-// scratch 16-byte aligned.
+// particles, at most live_capacity; up to kLiveMany times as many from memory, then ending also once
+// more than `dense` particles of a step were in contact.  quiet: the particles [nlone + nclear, n) only
+// (dem_flight.cuh).  scratch 16-byte aligned.
+constexpr int kLiveMany = 4;
 int live_capacity(bool mixed);
 cudaError_t launch_steps_live(const Particles &P, const NbrList &L, Ctl *ctl, const ForceConsts &fc, const PairConst *pp,
                               const PairConst *pw, const WallGeom *walls, int count, int max_steps,
-                              unsigned long long *scratch, int quiet, cudaStream_t s);
+                              unsigned long long *scratch, int quiet, int dense, cudaStream_t s);
 int live_capacity_mixed();
 cudaError_t launch_steps_live_mixed(const Particles &P, const NbrList &L, Ctl *ctl, const ForceConsts &fc,
                                     const PairConst *pp, const PairConst *pw, const WallGeom *walls, int count,
-                                    int max_steps, unsigned long long *scratch, int quiet, cudaStream_t s);
+                                    int max_steps, unsigned long long *scratch, int quiet, int dense, cudaStream_t s);
 
 // The rebuild-every-step mode's run in one cooperative launch (dem_refloop.cuh): at most
 // `max_steps` steps, ending at the target, or earlier where the build and step kernels have to go

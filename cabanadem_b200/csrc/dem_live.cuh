@@ -10,8 +10,8 @@
 //
 // k_steps_coop_lean (dem_persist.cuh) reloads each particle's state and runs the full body in every
 // thread.  Measured (B200, device us per step, that form / this one): 4,096 spheres, no pair in
-// contact 6.6 / 4.8, some 9.0 / 6.5; 30,011 spheres 11.0 / 6.9, FP32 forces 9.8 / 6.3; 200 spheres
-// 7.5 / 5.4; a column of disks with most in contact, 5,000 29.5 / 26.8, 56,000 36.0 / 32.8.  Contacts
+// contact 6.6 / 4.8, some 9.0 / 6.5; 30,011 spheres 11.0 / 6.9, FP32 forces 9.8 / 6.2; 200 spheres
+// 7.5 / 5.4; a column of disks with most in contact, 5,000 29.5 / 26.3, 56,000 36.0 / 32.6.  Contacts
 // by eight lanes each (particle_coop) instead took 11.2 us on the 4,096: some 1,400 dependent
 // instructions of a contact, staged through shared memory, where a thread has its own state at hand.
 // What bounds it: the barrier (1.2 us) and the chain of one contact's divisions and square roots.
@@ -225,6 +225,41 @@ __device__ __forceinline__ void live_contact(const Particles &P, const NbrList &
     }
 }
 
+// List entries of particle i at x that may overlap (bit kk, 31 for all from 31 on; the exact early-out
+// of the contact loop) and walls it may touch (bit lw; a margin above the law's own test).
+__device__ __forceinline__ void live_marks(const NbrList &L, const int cap, const WallGeom *__restrict__ walls,
+                                           const double4 *pc, const D4 &x, const int i, const int nn, const int j0,
+                                           const int j1, const int wall0, const int wall1, unsigned &pairs,
+                                           unsigned &near) {
+    auto touches = [&](const D4 &pj) {
+        const double px = dadd(x.x, -pj.x), py = dadd(x.y, -pj.y), pz = dadd(x.z, -pj.z);
+        const double r2 = dadd(dadd(dmul(px, px), dmul(py, py)), dmul(pz, pz));
+        const double sr = dadd(x.w, pj.w);
+        return !(r2 >= dmul(dmul(sr, sr), 1.0000000001));
+    };
+    pairs = near = 0u;
+    if (nn > 0) {
+        const D4 pa = ld4(pc, j0), pb = ld4(pc, nn > 1 ? j1 : j0);
+        pairs = (touches(pa) ? 1u : 0u) | (nn > 1 && touches(pb) ? 2u : 0u);
+        for (int k0 = 2; k0 < nn; k0 += 4) {   // four entries' indices, then their positions, in flight
+            int j[4];
+            D4 p[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) j[c] = L.idx[(long)min(k0 + c, nn - 1) * cap + i];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) p[c] = ld4(pc, j[c]);
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                if (touches(p[c])) pairs |= 1u << min(min(k0 + c, nn - 1), 31);
+        }
+    }
+    for (int q = wall0; q < wall1; ++q) {
+        const WallGeom &g = walls[q];
+        const double at = (x.x - g.x[0]) * g.n[0] + (x.y - g.x[1]) * g.n[1] + (x.z - g.x[2]) * g.n[2];
+        near |= !(at > x.w * 1.000001) ? 1u << (q - wall0) : 0u;
+    }
+}
+
 template <bool MIXED>
 __global__ void __launch_bounds__(kBlock, 3) k_steps_live(Particles P, NbrList L, Ctl *ctl, ForceConsts fc,
                                                           const PairConst *__restrict__ pp,
@@ -285,25 +320,8 @@ __global__ void __launch_bounds__(kBlock, 3) k_steps_live(Particles P, NbrList L
         int status = 0;
         bool full = false;
         if (have) {
-            auto touches = [&](const D4 &pj) {   // the exact early-out of the contact loop
-                const double px = dadd(x.x, -pj.x), py = dadd(x.y, -pj.y), pz = dadd(x.z, -pj.z);
-                const double r2 = dadd(dadd(dmul(px, px), dmul(py, py)), dmul(pz, pz));
-                const double sr = dadd(x.w, pj.w);
-                return !(r2 >= dmul(dmul(sr, sr), 1.0000000001));
-            };
-            unsigned pairs = 0u, near = 0u;
-            if (nn > 0) {
-                const D4 pa = ld4(pc, j0), pb = ld4(pc, nn > 1 ? j1 : j0);
-                pairs = (touches(pa) ? 1u : 0u) | (nn > 1 && touches(pb) ? 2u : 0u);
-                for (int kk = 2; kk < nn; ++kk)
-                    if (touches(ld4(pc, L.idx[(long)kk * cap + i]))) pairs |= 1u << min(kk, 31);
-            }
-            if (!(wfar && far))
-                for (int q = wall0; q < wall1; ++q) {   // a margin above the law's own test
-                    const WallGeom &g = walls[q];
-                    const double at = (x.x - g.x[0]) * g.n[0] + (x.y - g.x[1]) * g.n[1] + (x.z - g.x[2]) * g.n[2];
-                    near |= !(at > x.w * 1.000001) ? 1u << (q - wall0) : 0u;
-                }
+            unsigned pairs, near;
+            live_marks(L, cap, walls, pc, x, i, nn, j0, j1, wall0, wfar && far ? wall0 : wall1, pairs, near);
             full = cs != 0 || pairs != 0u || near != 0u;
             if (!full) {
                 if (last) {
@@ -364,31 +382,173 @@ __global__ void __launch_bounds__(kBlock, 3) k_steps_live(Particles P, NbrList L
     }
 }
 
+// The same loop for up to kLiveMany particles per thread, their state in memory: a thread first takes
+// the free step of those nothing marks, then the warp's threads each take their marked ones, one after
+// another (live_contact), so that particles in contact in different rounds share one pass.  Ends
+// early once more than `dense` particles of a step were in contact.
+//
+// Bounded by the list and position gathers of a thread's rounds and by the barrier.  Measured (B200,
+// device us per step, the three-kernel step in graph replays / this one): 151 scenes of 1,166 spheres
+// in their boxes (176,000, FP32 forces) 25 / 14.4; four entries' gathers in flight at a time instead of
+// one after another 16.6 -> 14.4.
 template <bool MIXED>
-static int live_threads() {   // particles a launch takes: threads resident at once, per host thread
-    static thread_local int fit = 0;
-    if (!fit) {
+__global__ void __launch_bounds__(kBlock, 3) k_steps_live_many(Particles P, NbrList L, Ctl *ctl, ForceConsts fc,
+                                                               const PairConst *__restrict__ pp,
+                                                               const PairConst *__restrict__ pw,
+                                                               const WallGeom *__restrict__ walls, int max_steps,
+                                                               unsigned long long *scratch, int quiet, int dense) {
+    constexpr unsigned FULL = 0xffffffffu;
+    __shared__ GridStep<kBlock> bar;
+    const int n = P.n, cap = P.cap, T = gridDim.x * kBlock;
+    const int cur0 = ctl->cur, vcur0 = ctl->vcur, target = ctl->target;
+    const int first = quiet ? ctl->nlone + ctl->nclear : 0;
+    const bool stopped = (ctl->status & kStopBits) != 0;
+    const double half = ctl->half_skin, until = quiet ? fmin(half, ctl->clear_until) : half;
+    const bool wfar_ok = ctl->wfar_build == ctl->rebuilds;
+    const double vq = quiet ? sqrt(__longlong_as_double((long long)ctl->vq2)) : 0.0;
+    const double ga = sqrt(fc.g[0] * fc.g[0] + fc.g[1] * fc.g[1] + fc.g[2] * fc.g[2]);
+    double disp = ctl->disp;
+    int done = ctl->steps_done, cur = cur0, steps = 0, ncon = 0;
+    double *v0 = P.vel[vcur0], *w0 = P.omg[vcur0];   // velocities of the step, and of the next
+    double *v1 = quiet ? L.defer_v : P.vel[vcur0 ^ 1], *w1 = quiet ? L.defer_w : P.omg[vcur0 ^ 1];
+    const int i0 = first + blockIdx.x * kBlock + threadIdx.x;
+    unsigned spin = 0u;   // bit r: the particle of round r was in contact in the last step
+    for (int i = i0; i < n; i += T)
+        for (int d = 0; d < 3; ++d) w1[d * cap + i] = w0[d * cap + i];
+    bool ok = true;
+    for (int k = 0; k < max_steps; ++k) {
+        // the same in every block
+        if (!(done < target && !stopped && disp < until && ok && ncon <= dense)) break;
+        const int last = done + 1 >= target;
+        const bool wfar = wfar_ok && 2.0 * disp < half;
+        const double4 *pc = P.pos[cur];
+        double vmax = 0.0;
+        int status = 0;
+        unsigned pend = 0u;
+        // particle i's state and marks
+        auto read = [&](const int i, D4 &x, double &m, double (&u)[3], int &cs, int &nn, int &j0, int &j1, int &wall0,
+                        unsigned &pairs, unsigned &near) {
+            x = ld4(pc, i);
+            cs = P.cstate[i];
+            nn = L.nn[i];
+            const bool far = wfar && L.wfar[i];
+            j0 = L.maxnb > 0 ? L.idx[i] : 0;   // used below the list length only
+            j1 = L.maxnb > 1 ? L.idx[cap + i] : 0;
+            m = P.mI[i];
+            for (int d = 0; d < 3; ++d) u[d] = v0[d * cap + i];
+            const int scene_i = P.scene ? P.scene[i] : 0;
+            wall0 = fc.wps ? scene_i * fc.wps : 0;
+            const int wall1 = far ? wall0 : fc.wps ? wall0 + fc.wps : fc.nwall;
+            live_marks(L, cap, walls, pc, x, i, nn, j0, j1, wall0, wall1, pairs, near);
+        };
+        int r = 0;
+        for (int i = i0; i < n; i += T, ++r) {
+            D4 x;
+            double m, u[3];
+            int cs, nn, j0, j1, wall0;
+            unsigned pairs, near;
+            read(i, x, m, u, cs, nn, j0, j1, wall0, pairs, near);
+            if (cs != 0 || pairs != 0u || near != 0u) {
+                pend |= 1u << r;
+                continue;
+            }
+            vmax = fmax(vmax, free_step(P, fc, i, last, m, u, x));
+            st4(P.pos[cur ^ 1], i, x);
+            for (int d = 0; d < 3; ++d) v1[d * cap + i] = u[d];
+            if ((spin >> r) & 1u) {   // the spin a contact wrote last step, in both buffers again
+                for (int d = 0; d < 3; ++d) w1[d * cap + i] = w0[d * cap + i];
+                spin &= ~(1u << r);
+            }
+        }
+        const int busy = (int)__reduce_add_sync(FULL, (unsigned)__popc(pend));
+        spin |= pend;
+        while (__any_sync(FULL, pend != 0u)) {
+            if (pend) {
+                const int i = i0 + (__ffs(pend) - 1) * T;
+                pend &= pend - 1u;
+                D4 x;
+                double m, u[3], v2 = 0.0;
+                int cs, nn, j0, j1, wall0;
+                unsigned pairs, near;
+                read(i, x, m, u, cs, nn, j0, j1, wall0, pairs, near);
+                live_contact<MIXED>(P, L, fc, pp, pw, walls, pc, P.pos[cur ^ 1], v0, w0, v1, w1, last, i, j0, j1, nn,
+                                    pairs, near, wall0, m, x, u, cs, v2, status);
+                vmax = fmax(vmax, v2);
+            }
+        }
+        if (status) atomicOr(&ctl->status, status);
+        unsigned long long big;
+        ok = grid_step<kBlock>(bar, ctl, scratch, k, vmax, busy, big, ncon);
+        if (!ok) break;
+        double v = sqrt(__longlong_as_double((long long)big));
+        if (quiet) v = fmax(v, vq + (k + 1) * fc.dt * ga * (1.0 + 1e-9));
+        disp = disp + fc.dt * v * (1.0 + 1e-9);
+        cur ^= 1;
+        double *tv = v0, *tw = w0;
+        v0 = v1;
+        w0 = w1;
+        v1 = tv;
+        w1 = tw;
+        done += 1;
+        steps += 1;
+    }
+    if (quiet && (steps & 1))   // the velocities back into their arrays
+        for (int i = i0; i < n; i += T)
+            for (int d = 0; d < 3; ++d) {
+                v1[d * cap + i] = v0[d * cap + i];
+                w1[d * cap + i] = w0[d * cap + i];
+            }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {   // as k_steps_live leaves it
+        ctl->cur = cur;
+        if (!quiet) ctl->vcur = vcur0 ^ (steps & 1);
+        ctl->steps_done = done;
+        ctl->total_steps += steps;
+        ctl->disp = disp;
+        if (steps > 0) ctl->last_ndefer = ncon;
+        ctl->ndefer = 0;
+        ctl->npairs = 0;
+        ctl->flight_cur = cur0;
+        ctl->flight_steps = steps;
+        ctl->flight_last = done >= target;
+    }
+}
+
+// Blocks resident at once, per host thread.
+template <bool MIXED>
+static int live_blocks(bool many) {
+    static thread_local int fit[2] = {0, 0};
+    if (!fit[many]) {
         int dev = 0, sms = 0, per = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void *)k_steps_live<MIXED>, kBlock, 0);
-        fit = (sms > 0 ? sms : 148) * (per > 0 ? per : 1) * kBlock;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+            &per, many ? (const void *)k_steps_live_many<MIXED> : (const void *)k_steps_live<MIXED>, kBlock, 0);
+        fit[many] = (sms > 0 ? sms : 148) * (per > 0 ? per : 1);
     }
-    return fit;
+    return fit[many];
 }
+
+template <bool MIXED>
+static int live_threads() { return live_blocks<MIXED>(false) * kBlock; }
 
 template <bool MIXED>
 static cudaError_t steps_live_t(const Particles &P, const NbrList &L, Ctl *ctl, const ForceConsts &fc,
                                 const PairConst *pp, const PairConst *pw, const WallGeom *walls, int count, int max_steps,
-                                unsigned long long *scratch, int quiet, cudaStream_t s) {
-    const int grid = count > 0 ? (count + kBlock - 1) / kBlock : 1;
+                                unsigned long long *scratch, int quiet, int dense, cudaStream_t s) {
+    const int need = count > 0 ? (count + kBlock - 1) / kBlock : 1;
+    const bool many = need > live_blocks<MIXED>(false);
+    // every thread the same number of rounds: the fewest rounds, then no more blocks than those need
+    const int most = live_blocks<MIXED>(true), rounds = (need + most - 1) / most;
+    const int grid = many ? (need + rounds - 1) / rounds : need;
+    if (many && rounds > kLiveMany) return cudaErrorInvalidValue;
     const cudaError_t e = cudaMemsetAsync(scratch, 0, sizeof(unsigned long long) * 6, s);
     if (e != cudaSuccess) return e;
     Particles p = P;
     NbrList l = L;
     ForceConsts f = fc;
-    void *args[] = {&p, &l, &ctl, &f, (void *)&pp, (void *)&pw, (void *)&walls, &max_steps, &scratch, &quiet};
-    return cudaLaunchCooperativeKernel((const void *)k_steps_live<MIXED>, dim3(grid), dim3(kBlock), args, 0, s);
+    void *args[] = {&p, &l, &ctl, &f, (void *)&pp, (void *)&pw, (void *)&walls, &max_steps, &scratch, &quiet, &dense};
+    return cudaLaunchCooperativeKernel(many ? (const void *)k_steps_live_many<MIXED> : (const void *)k_steps_live<MIXED>,
+                                       dim3(grid), dim3(kBlock), args, 0, s);   // k_steps_live takes no `dense`
 }
 
 }  // namespace

@@ -188,8 +188,8 @@ template <bool MIXED, bool MESH>
 static cudaError_t steps_coop_t(const Particles &P, const NbrList &L, Ctl *ctl, const ForceConsts &fc,
                                 const PairConst *pp, const PairConst *pw, const WallGeom *walls, int max_steps,
                                 unsigned long long *scratch, cudaStream_t s) {
-    const bool lean = !fc.mwalls && !fc.mesh_moving && scratch;
-    const void *kernel = lean ? (const void *)k_steps_coop_lean<MIXED, MESH> : (const void *)k_steps_coop<MIXED, MESH>;
+    const bool lean = MESH && !fc.mwalls && !fc.mesh_moving && scratch;
+    const void *kernel = lean ? (const void *)k_steps_coop_lean<MIXED> : (const void *)k_steps_coop<MIXED, MESH>;
     static thread_local int fit[2] = {0, 0};   // resident blocks of each form, per host thread
     if (!fit[lean]) {
         int dev = 0, sms = 0, per = 0;
@@ -225,8 +225,8 @@ int live_capacity_mixed() { return live_threads<true>(); }
 
 cudaError_t launch_steps_live_mixed(const Particles &P, const NbrList &L, Ctl *ctl, const ForceConsts &fc, const PairConst *pp,
                               const PairConst *pw, const WallGeom *walls, int count, int max_steps,
-                              unsigned long long *scratch, int quiet, cudaStream_t s) {
-    return steps_live_t<true>(P, L, ctl, fc, pp, pw, walls, count, max_steps, scratch, quiet, s);
+                              unsigned long long *scratch, int quiet, int dense, cudaStream_t s) {
+    return steps_live_t<true>(P, L, ctl, fc, pp, pw, walls, count, max_steps, scratch, quiet, dense, s);
 }
 
 cudaError_t launch_steps_ref_mixed(const Particles &P, const NbrList &L, Ctl *ctl, const ForceConsts &fc, const PairConst *pp,

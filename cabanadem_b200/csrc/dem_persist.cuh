@@ -1,4 +1,5 @@
-// dem_persist.cuh -- the step loop of a small system in one cooperative launch.
+// dem_persist.cuh -- the step loop of a small system with a mesh or moving walls in one cooperative
+// launch (with static walls and no mesh: dem_live.cuh).
 //
 // Below a few tens of thousands of particles the one-kernel step (k_contact_all) takes a few
 // microseconds, about what a kernel launch and the step's last-block finalisation cost on top.
@@ -123,7 +124,7 @@ __global__ void __launch_bounds__(kBlock) k_steps_coop(Particles P, NbrList L, C
     }
 }
 
-// The same loop with static walls and no moving mesh, where nothing but the particles changes
+// The same loop with static walls and a mesh at rest, where nothing but the particles changes
 // between steps: every block keeps the step counters, the buffer parity and the displacement
 // bound itself, and the barrier is symmetric.  Per step each block stores its largest |u|^2
 // and its in-contact count in its own slot (two sets of slots, by step parity), then arrives on
@@ -136,7 +137,7 @@ __global__ void __launch_bounds__(kBlock) k_steps_coop(Particles P, NbrList L, C
 // counts.
 constexpr int kCoopMaxBlocks = kCoopMaxN / kBlock;
 
-template <bool MIXED, bool MESH>
+template <bool MIXED>
 __global__ void __launch_bounds__(kBlock) k_steps_coop_lean(Particles P, NbrList L, Ctl *ctl, ForceConsts fc,
                                                             const PairConst *__restrict__ pp,
                                                             const PairConst *__restrict__ pw,
@@ -177,7 +178,7 @@ __global__ void __launch_bounds__(kBlock) k_steps_coop_lean(Particles P, NbrList
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P.n; i += gridDim.x * blockDim.x) {
             double v2 = 0.0;
             int a = 0;
-            particle_full<MODE_FUSED_DIRECT, MIXED, MESH>(P, L, fc, pp, pw, walls, cur, cur ^ 1, vcur, last, i, i, v2,
+            particle_full<MODE_FUSED_DIRECT, MIXED, true>(P, L, fc, pp, pw, walls, cur, cur ^ 1, vcur, last, i, i, v2,
                                                           status, &a);
             vmax2 = fmax(vmax2, v2);
             active += a;

@@ -93,3 +93,36 @@ def test_wall_history(quirks):
     sc.gravity = (0.0, 0.0, -9.81)
     a, _ = _same(sc, (61, 140))
     assert np.abs(a.tng_sw_x).max() > 0
+
+
+@pytest.mark.parametrize("precision", [_lib.DEM_FP64, _lib.DEM_MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("n", [57_000, 130_001])
+def test_several_particles_per_thread(n, precision):
+    """More particles than resident threads, few of them in contact, none of them quiet (a thick skin)."""
+    sc = S.hcp_box(n=n, seed=3, vmax=2.0)
+    sc.skin = 4e-4
+    sc.state.omega[:] = np.random.default_rng(3).uniform(-50, 50, sc.state.omega.shape)
+    sc.walls.x[:] += 1.198e-3 * sc.walls.normal
+    out = []
+    for coop in (0, 2):
+        s = api.from_scenario(sc, cooperative_loop=coop, precision=precision)
+        for k in (1, 2, 150, 57):
+            s.run_steps(k)
+        out.append((s.particles.download(), s.stats()))
+    (a, sa), (b, sb) = out
+    for f in FIELDS:
+        assert np.array_equal(getattr(a, f), getattr(b, f)), f
+    assert sa["cooperative_loop"] == 1 and sb["cooperative_loop"] == 0 and a.tng_count.sum() > 50
+
+
+def test_from_sparse_to_dense():
+    """A lattice that is squeezed until its steps are too dense for several particles per thread."""
+    sc = _box(58_001, squeeze=0.9, vmax=0.5)
+    out = []
+    for coop in (0, 2):
+        s = api.from_scenario(sc, cooperative_loop=coop)
+        s.run_steps(60)
+        out.append((s.particles.download(), s.last_status))
+    for f in FIELDS:
+        assert np.array_equal(getattr(out[0][0], f), getattr(out[1][0], f)), f
+    assert out[0][1] == out[1][1] and out[0][0].tng_count.mean() > 1.0
