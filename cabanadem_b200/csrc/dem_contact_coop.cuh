@@ -231,7 +231,7 @@ __device__ __forceinline__ void particle_coop(const Particles &P, const LIST &li
             }
             const int mj = fc.nmat > 1 ? (int)P.mat[j] : 0;
             const PairConst c = pp[mi * fc.nmat + mj];
-            pp_pair<MIXED>(P.mI, vc, wc, cap, q, pi, pj, j, px, py, pz, rij, overlap, ui0, ui1, ui2, wi0, wi1, wi2,
+            pp_pair<MIXED>(load_mate(P.mI, vc, wc, cap, j), q, pi, pj, px, py, pz, rij, overlap, ui0, ui1, ui2, wi0, wi1, wi2,
                            mIi.x, c, K_n_pp, K_t_pp, mu_pp, fc.dt, h0, h1, h2, cf);
             if (found_at >= 0) {
                 const long a = (long)found_at * cap;

@@ -10,8 +10,9 @@
 //
 // k_steps_coop_lean (dem_persist.cuh) reloads each particle's state and runs the full body in every
 // thread.  Measured (B200, device us per step, that form / this one): 4,096 spheres, no pair in
-// contact 6.6 / 4.8, some 9.0 / 6.5; 30,011 spheres 11.0 / 6.9, FP32 forces 9.8 / 6.2; 200 spheres
-// 7.5 / 5.4; a column of disks with most in contact, 5,000 29.5 / 26.3, 56,000 36.0 / 32.6.  Contacts
+// contact 6.6 / 4.8, some 9.0 / 6.0; 30,011 spheres 11.0 / 6.9, FP32 forces 9.8 / 6.1; 200 spheres
+// 7.5 / 5.4; a column of disks with most in contact, 5,000 29.5 / 20.6, 56,000 36.0 / 26.2
+// (some of it the pair law's).  Contacts
 // by eight lanes each (particle_coop) instead took 11.2 us on the 4,096: some 1,400 dependent
 // instructions of a contact, staged through shared memory, where a thread has its own state at hand.
 // What bounds it: the barrier (1.2 us) and the chain of one contact's divisions and square roots.
@@ -103,6 +104,7 @@ __device__ __forceinline__ void live_contact(const Particles &P, const NbrList &
     for (int kk = todo ? __ffs(todo) - 1 : nn; kk < nn;) {
         const int j = kk == 0 ? j0 : kk == 1 ? j1 : L.idx[(long)kk * cap + i];
         const D4 pj = ld4(pc, j);
+        const Mate b = load_mate(P.mI, vc, wc, cap, j);   // most marked entries are in contact
         const double px = x.x - pj.x, py = x.y - pj.y, pz = x.z - pj.z;
         const double r2ij = px * px + py * py + pz * pz;
         const double sr = x.w + pj.w;
@@ -131,7 +133,7 @@ __device__ __forceinline__ void live_contact(const Particles &P, const NbrList &
             const int mj = fc.nmat > 1 ? (int)P.mat[j] : 0;
             const PairConst c = pp[mi * fc.nmat + mj];
             double cf[6];
-            pp_pair<MIXED>(P.mI, vc, wc, cap, q, x, pj, j, px, py, pz, rij, overlap, u[0], u[1], u[2], w[0], w[1], w[2], m,
+            pp_pair<MIXED>(b, q, x, pj, px, py, pz, rij, overlap, u[0], u[1], u[2], w[0], w[1], w[2], m,
                            c, scn ? scn->K_n_pp : fc.K_n_pp, scn ? scn->K_t_pp : fc.K_t_pp, scn ? scn->mu_pp : fc.mu_pp,
                            fc.dt, h0, h1, h2, cf);
             if (found_at >= 0) {

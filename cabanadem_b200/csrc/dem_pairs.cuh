@@ -243,14 +243,10 @@ __device__ __forceinline__ void pairs_item(const Particles &P, const ForceConsts
                        swy, swz, cf);
     } else {
         const D4 pj = ld4(pc, j);
+        const Mate b = load_mate(P.mI, vc, wc, cap, j);
         const double K_n_pp = scn ? scn->K_n_pp : fc.K_n_pp, K_t_pp = scn ? scn->K_t_pp : fc.K_t_pp;
         const double mu_pp = scn ? scn->mu_pp : fc.mu_pp;
         const int mj = fc.nmat > 1 ? (int)P.mat[j] : 0;
-        const double px = pi.x - pj.x, py = pi.y - pj.y, pz = pi.z - pj.z;
-        const double r2ij = px * px + py * py + pz * pz;
-        const double sr = pi.w + pj.w;
-        const double rij = sqrt(r2ij);
-        const double overlap = sr - rij;
         double *hx = P.th + (long)slot * cap + i;
         double *hy = P.th + ((long)P.mc + slot) * cap + i;
         double *hz = P.th + (2L * P.mc + slot) * cap + i;
@@ -260,7 +256,12 @@ __device__ __forceinline__ void pairs_item(const Particles &P, const ForceConsts
             h1 = *hy;
             h2 = *hz;
         }
-        pp_pair<MIXED>(P.mI, vc, wc, cap, q, pi, pj, j, px, py, pz, rij, overlap, ui0, ui1, ui2, wi0, wi1, wi2,
+        const double px = pi.x - pj.x, py = pi.y - pj.y, pz = pi.z - pj.z;
+        const double r2ij = px * px + py * py + pz * pz;
+        const double sr = pi.w + pj.w;
+        const double rij = sqrt(r2ij);
+        const double overlap = sr - rij;
+        pp_pair<MIXED>(b, q, pi, pj, px, py, pz, rij, overlap, ui0, ui1, ui2, wi0, wi1, wi2,
                        m_i, pp[mi * fc.nmat + mj], K_n_pp, K_t_pp, mu_pp, fc.dt, h0, h1, h2, cf);
         if (slot >= 0) {
             *hx = h0;
