@@ -32,12 +32,17 @@ namespace b200dem {
 namespace {
 
 constexpr int kPairsBlock = 128;
-// List entries the contact search tests per round: their index loads, then their position
-// loads, are issued together (B200, dam-break state, FP64 step: 79.2 us with one entry per round,
-// 76.8 us with two, 81.9 us with four -- more registers, fewer resident warps; testing the
-// tracked slots the same way before the compaction, or prefetching the first two tracked
-// partners with the own state, cost more registers than they saved: 82.1 and 83.8 us).
-constexpr int kFindBatch = 2;
+// The contact search is bound by round trips of a thread (index, then position).  It takes a
+// particle's first tracked partners (kFindSlots) and list entries (kFindFirst) together with its own
+// state, tests kFindBatch positions at a time, and knows the tracked slots that stay from the list's
+// contacts: only where a contact has ended are tracked partners' positions read, one by one.  The first
+// kFindKeep contacts' partners wait in shared memory for the items.  Before, the compaction read every
+// tracked partner's position first and the list two entries at a time: a column of disks (B200, one
+// launch at 200,000) 34.8 -> 23.0 us; with k_pairs_eval's items read a round ahead the whole step
+// 69.6 -> 60.4 us, FP32 forces (90,001) 37.0 -> 32.6 us.  Two positions at a time 61.3; a register cap
+// of 80 (six blocks per SM) 60.8, 34.1 against 32.5 on 90,001 in FP32; a block per 128 particles instead
+// of a resident grid 61.3 (and 63.3 with k_pairs_sum so).
+constexpr int kFindSlots = 6, kFindFirst = 8, kFindBatch = 4, kFindKeep = 8;
 // The three kernels are compiled without a register cap: on the dam-break state (B200) caps of
 // 80 / 64 registers for the per-contact and summing kernels (more resident blocks, spills) ran
 // the step in 102.3 us against 95.1 us, and a contact search with 4 or 8 lanes per particle
@@ -52,24 +57,65 @@ __global__ void __launch_bounds__(kPairsBlock) k_pairs_find(Particles P, NbrList
     if (!c.go) return;
     const int cap = P.cap, n = P.n;
     const double4 *__restrict__ pc = P.pos[c.cur];
+    const bool wfar_ok = ctl->wfar_build == ctl->rebuilds && 2.0 * ctl->disp < ctl->half_skin;
+    __shared__ int s_j[kFindKeep][kPairsBlock];   // partners of a thread's first contacts
     int status = 0;
     for (int b = blockIdx.x * kPairsBlock; b < n; b += gridDim.x * kPairsBlock) {   // block-uniform
         const int i = b + threadIdx.x;
         int ncont = 0, nwc = 0, cs0 = 0, cnt = 0, nn = 0, wall0 = 0;
         unsigned cm[4] = {0u, 0u, 0u, 0u};   // contact flags of list entries 0..127
         unsigned wmask = 0u, wtouch = 0u;    // wall history bits; walls in contact this step
+        int tx[kFindSlots];                  // tracked partners of the first slots
         int *tidx = P.tidx + i;
         double *thx = P.th + i;
         double *thy = P.th + (long)P.mc * cap + i;
         double *thz = P.th + 2L * P.mc * cap + i;
-        D4 pi{};
         if (i < n) {
-            pi = ld4(pc, i);
+            // own state, first tracked partners and first list entries in one round trip
+            const D4 pi = ld4(pc, i);
             cs0 = P.cstate[i];
-            cnt = cs0 & 0xff;
             nn = L.nn[i];
-            // ---- update_tangential_contacts (Force.hpp:364-441), as in particle_full
-            if (cnt > 0) {
+            int jn[kFindFirst];
+#pragma unroll
+            for (int s = 0; s < kFindSlots; ++s) tx[s] = s < P.mc ? tidx[(long)s * cap] : -1;
+#pragma unroll
+            for (int u = 0; u < kFindFirst; ++u) jn[u] = u < L.maxnb ? L.idx[(long)u * cap + i] : -1;
+            const bool far = wfar_ok && L.wfar[i] != 0;
+            cnt = cs0 & 0xff;
+            unsigned keep = 0u;   // tracked slots whose partner the list finds in contact
+            // ---- overlap test over the list (the pair loop's early-outs of particle_full)
+            auto test = [&](const int kk, const int j, const D4 &pj) {
+                const double px = pi.x - pj.x, py = pi.y - pj.y, pz = pi.z - pj.z;
+                const double r2ij = px * px + py * py + pz * pz;
+                const double sr = pi.w + pj.w, s2 = sr * sr;
+                // overlap = sr - sqrt(r2) > 0; the root only where the squares are close
+                if (r2ij >= s2 * 1.0000000001) return;
+                if (!(r2ij < s2 * 0.9999999999) && !(sr - sqrt(r2ij) > 0.)) return;
+                cm[kk >> 5] |= 1u << (kk & 31);
+                if (ncont < kFindKeep) s_j[ncont][threadIdx.x] = j;
+                ++ncont;
+#pragma unroll
+                for (int s = 0; s < kFindSlots; ++s) keep |= tx[s] == j ? 1u << s : 0u;
+            };
+#pragma unroll
+            for (int u0 = 0; u0 < kFindFirst; u0 += kFindBatch) {   // kFindBatch positions in flight
+                if (u0 && u0 >= nn) break;
+                D4 pj[kFindBatch];
+#pragma unroll
+                for (int u = 0; u < kFindBatch; ++u) pj[u] = ld4(pc, u0 + u < nn ? jn[u0 + u] : i);
+#pragma unroll
+                for (int u = 0; u < kFindBatch; ++u)
+                    if (u0 + u < nn) test(u0 + u, jn[u0 + u], pj[u]);
+            }
+#pragma unroll 1
+            for (int kk = kFindFirst; kk < nn; ++kk) {
+                const int j = L.idx[(long)kk * cap + i];
+                test(kk, j, ld4(pc, j));
+            }
+            // ---- update_tangential_contacts (Force.hpp:364-441): nothing moves while every tracked
+            // partner is in contact; else the slots the list did not find are tested one by one
+            const unsigned all = (1u << min(cnt, kFindSlots)) - 1u;
+            if (cnt > kFindSlots || (keep & all) != all) {
                 int count = 0, k = 0;
                 const int total = cnt;
                 int last_idx_tmp = cnt - 1;
@@ -105,38 +151,14 @@ __global__ void __launch_bounds__(kPairsBlock) k_pairs_find(Particles P, NbrList
                     }
                     count += 1;
                 }
-            }
-            // ---- overlap test over the list (the pair loop's early-outs of particle_full)
-            // (kFindBatch list entries per round: their index loads, then their position loads)
-#pragma unroll 1
-            for (int k0 = 0; k0 < nn; k0 += kFindBatch) {
-                int jj[kFindBatch];
-                D4 pj[kFindBatch];
 #pragma unroll
-                for (int u = 0; u < kFindBatch; ++u) jj[u] = k0 + u < nn ? L.idx[(long)(k0 + u) * cap + i] : -1;
-#pragma unroll
-                for (int u = 0; u < kFindBatch; ++u)
-                    if (jj[u] >= 0) pj[u] = ld4(pc, jj[u]);
-#pragma unroll
-                for (int u = 0; u < kFindBatch; ++u) {
-                    if (jj[u] < 0) continue;
-                    const int kk = k0 + u;
-                    const double px = pi.x - pj[u].x, py = pi.y - pj[u].y, pz = pi.z - pj[u].z;
-                    const double r2ij = px * px + py * py + pz * pz;
-                    const double sr = pi.w + pj[u].w;
-                    if (r2ij >= sr * sr * 1.0000000001) continue;
-                    const double rij = sqrt(r2ij);
-                    const double overlap = sr - rij;
-                    if (!(overlap > 0.)) continue;
-                    cm[kk >> 5] |= 1u << (kk & 31);
-                    ++ncont;
-                }
+                for (int s = 0; s < kFindSlots; ++s) tx[s] = s < cnt ? tidx[(long)s * cap] : -1;
             }
             // ---- particle-infinite wall overlaps (Force.hpp:475-490, 664-673)
             const int scene_i = P.scene ? P.scene[i] : 0;
             wall0 = fc.wps ? scene_i * fc.wps : 0;
-            const int wall1 = fc.wps ? wall0 + fc.wps : fc.nwall;
             wmask = (unsigned)cs0 >> 8;
+            const int wall1 = far && wmask == 0u ? wall0 : fc.wps ? wall0 + fc.wps : fc.nwall;
             for (int w = wall0; w < wall1; ++w) {
                 const WallGeom *g = walls + w;
                 const int lw = w - wall0;
@@ -169,15 +191,21 @@ __global__ void __launch_bounds__(kPairsBlock) k_pairs_find(Particles P, NbrList
         if (i < n) {
             int t = wbase + incl - ncont - nwc;
             L.prec[i] = make_int4(t, ncont, cs0, nwc);
+            const int cnt0 = cnt;   // a list names a partner once: slots added below match no later entry
+            int nth = 0;
             for (int w = 0; w < 4; ++w) {
                 unsigned bits = cm[w];
                 while (bits) {
                     const int kk = 32 * w + __ffs(bits) - 1;
                     bits &= bits - 1u;
-                    const int j = L.idx[(long)kk * cap + i];
+                    const int j = nth < kFindKeep ? s_j[nth][threadIdx.x] : L.idx[(long)kk * cap + i];
+                    ++nth;
                     // slot lookup / insert (Force.hpp:166-192)
                     int found_at = -1;
-                    for (int s = 0; s < cnt; ++s)
+#pragma unroll
+                    for (int s = 0; s < kFindSlots; ++s)
+                        if (s < cnt0 && tx[s] == j) found_at = s;
+                    for (int s = kFindSlots; s < cnt0; ++s)
                         if (tidx[(long)s * cap] == j) found_at = s;
                     if (found_at < 0) {
                         if (cnt < P.mc) {
@@ -285,9 +313,14 @@ __global__ void __launch_bounds__(kPairsBlock) k_pairs_eval(Particles P, NbrList
     const int vcur = ctl->vcur;
     const double *__restrict__ vc = P.vel[vcur];
     const double *__restrict__ wc = P.omg[vcur];
-    for (int t = blockIdx.x * kPairsBlock + threadIdx.x; t < np; t += gridDim.x * kPairsBlock) {
+    const int stride = gridDim.x * kPairsBlock;
+    int t = blockIdx.x * kPairsBlock + threadIdx.x;
+    int4 it = t < np ? L.pitem[t] : make_int4(0, 0, 0, 0);
+    for (; t < np; t += stride) {
         double cf[6];
-        pairs_item<MIXED>(P, fc, pp, pw, walls, pc, vc, wc, L.pitem[t], cf);
+        const int4 ahead = t < np - stride ? L.pitem[t + stride] : it;   // the next round's item
+        pairs_item<MIXED>(P, fc, pp, pw, walls, pc, vc, wc, it, cf);
+        it = ahead;
         double2 *term = L.pterm + 3L * t;
         term[0] = make_double2(cf[0], cf[1]);
         term[1] = make_double2(cf[2], cf[3]);
