@@ -34,6 +34,7 @@ constexpr int kRows = 128;      // rows per tile (= MMA M)
 constexpr int kHidden = 128;    // hidden width
 constexpr int kThreads = 128;
 constexpr int kFwdThreads = 256;   // forward kernels: warps w and w + 4 split a TMEM lane quarter's columns
+constexpr int kBwdThreads = 512;   // gradient kernels: warps w, w + 4, w + 8 and w + 12 do
 
 struct RowSrc {
     const bf16 *p;
@@ -51,6 +52,36 @@ __device__ __forceinline__ void cp16(void *smem, const void *gmem) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tc::smem_u32(smem)), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// Element q of a tile of R rows (a multiple of 8) and C chunks: eight consecutive threads take eight
+// consecutive rows of one chunk (conflict-free 128-byte runs in shared memory), the warp four chunks of
+// them, so that its access covers whole 32-byte sectors of global memory.
+__device__ __forceinline__ void tile_element(int q, int R, int C, int &row, int &kc) {
+    const int G = C < 4 ? C : 4, rest = (q >> 3) / G;
+    row = (rest % (R / 8)) * 8 + (q & 7);
+    kc = (rest / (R / 8)) * G + (q >> 3) % G;
+}
+
+// Feature f of the concatenated sources: the source's number, and f within it.  (The sources are
+// picked by comparisons: an index into the kernel's argument array would put a copy of it in local memory.)
+__device__ __forceinline__ RowSrc pick_source(const RowSrc *src, int nsrc, int &f, int &s) {
+    RowSrc r = src[0];
+    s = 0;
+    if (nsrc > 1 && f >= r.width) {
+        f -= r.width;
+        r = src[1];
+        s = 1;
+        if (nsrc > 2 && f >= r.width) {
+            f -= r.width;
+            r = src[2];
+            s = 2;
+        }
+    }
+    return r;
+}
 
 // Row indices of the tile's rows for the gathered sources: s_idx[s][row] (one round trip).
 __device__ __forceinline__ void load_row_index(int *s_idx, const RowSrc *src, int nsrc, long row0, long rows) {
@@ -63,26 +94,18 @@ __device__ __forceinline__ void load_row_index(int *s_idx, const RowSrc *src, in
 }
 
 // Queue the copies of rows [row0, row0 + kRows) of the concatenated sources (C chunks of 8
-// features per row) into a row tile of 128 rows; rows past `rows` are zero-filled.  Eight
-// consecutive threads take eight consecutive rows of one chunk (conflict-free 128-byte runs
-// in shared memory).  s_idx must hold the tile's row indices (load_row_index + barrier).
+// features per row) into a row tile of 128 rows; rows past `rows` are zero-filled.
+// s_idx must hold the tile's row indices (load_row_index + barrier).
 __device__ __forceinline__ void stage_gather(unsigned char *tile, const RowSrc *src, int nsrc, int C, long row0,
                                              long rows, const int *s_idx) {
-    const int G = C < 4 ? C : 4;
     for (int q = threadIdx.x; q < kRows * C; q += blockDim.x) {
-        const int i = q & 7;
-        const int g = (q >> 3) % G;
-        const int rest = (q >> 3) / G;
-        const int row = (rest % (kRows / 8)) * 8 + i;
-        const int kc = (rest / (kRows / 8)) * G + g;
+        int row, kc;
+        tile_element(q, kRows, C, row, kc);
         unsigned char *dst = tile + tc::tile_off(kRows, row, kc);
         if (row0 + row < rows) {
-            int f = kc * 8, s = 0;
-            while (s < nsrc - 1 && f >= src[s].width) {
-                f -= src[s].width;
-                ++s;
-            }
-            cp16(dst, src[s].p + (long)s_idx[s * kRows + row] * src[s].width + f);
+            int f = kc * 8, s;
+            const RowSrc r = pick_source(src, nsrc, f, s);
+            cp16(dst, r.p + (long)s_idx[s * kRows + row] * r.width + f);
         } else {
             *reinterpret_cast<uint4 *>(dst) = make_uint4(0, 0, 0, 0);
         }
@@ -94,11 +117,28 @@ __device__ __forceinline__ void stage_gather(unsigned char *tile, const RowSrc *
 __device__ __forceinline__ void stage_dense(unsigned char *tile, const bf16 *g, int R, int F, long row0, long rows) {
     const int C = F / 8;
     for (int q = threadIdx.x; q < R * C; q += blockDim.x) {
-        const int row = q % R, kc = q / R;
+        int row, kc;
+        tile_element(q, R, C, row, kc);
         unsigned char *dst = tile + tc::tile_off(R, row, kc);
         if (row0 + row < rows) cp16(dst, g + (row0 + row) * F + kc * 8);
         else *reinterpret_cast<uint4 *>(dst) = make_uint4(0, 0, 0, 0);
     }
+}
+
+// The same into the swizzled layout (F a multiple of 64): a warp takes whole rows, four lines of global
+// memory, where the layout above makes it touch eight rows: there the copies of a 32 KB tile occupied an
+// SM's load path for some 2,000 cycles, most of the gradient kernels' time.
+__device__ __forceinline__ void stage_sw(unsigned char *tile, const bf16 *g, int R, int F, long row0, long rows) {
+    const int C = F / 8;
+    for (int q = threadIdx.x; q < R * C; q += blockDim.x) {
+        const int row = q / C, c = q % C;
+        unsigned char *dst = tile + tc::sw_off(R, row, c);
+        if (row0 + row < rows) cp16(dst, g + (row0 + row) * F + c * 8);
+        else *reinterpret_cast<uint4 *>(dst) = make_uint4(0, 0, 0, 0);
+    }
+}
+__device__ __forceinline__ unsigned char *align1024(unsigned char *p) {
+    return p + ((1024u - (tc::smem_u32(p) & 1023u)) & 1023u);
 }
 
 // Completes this thread's queued copies and publishes the tiles to the tensor core.
@@ -374,96 +414,152 @@ struct BwdArgs {
     int *err;
 };
 
+// Tiles in flight per CTA (384 inputs leave room for one), and whether the dX rows leave through a
+// buffer of their own (else through the dY tile, which is spent by then).
+template <int KIN>
+__host__ __device__ constexpr int bwd_bufs() { return KIN > 2 * kHidden ? 1 : 2; }
 template <int KIN, int NOUT>
 constexpr size_t bwd_smem() {
-    return (size_t)kHidden * NOUT * 2 + (size_t)KIN * kHidden * 2 + (size_t)kRows * NOUT * 2 +
-           2 * (size_t)kRows * kHidden * 2 + 64;
+    return (size_t)kHidden * NOUT * 2 + (size_t)KIN * kHidden * 2 +
+           bwd_bufs<KIN>() * ((size_t)kRows * NOUT * 2 + (size_t)kRows * kHidden * 2) + (NOUT < kHidden ? 32768 : 0) + 1024 + 64;
 }
 
+// The next tile's dY and H arrive while this one is worked on; dZ takes H's place in the tile (each
+// chunk by the thread that read it) and leaves from there, dX through a 2 KB buffer per warp, both in
+// whole sectors.  One CTA fills an SM's shared memory, so the epilogues' warps are all there is to hide
+// latency: four per scheduler.  With 128 threads, one tile at a time and rows written by the thread that
+// owned them, 240,000 edges took 129 us (B200); with 512 threads and this order 120, in the swizzled layout
+// 74.  HBM: 306 MB, 47 us at the copy rate.
 template <int KIN, int NOUT>
-__global__ void __launch_bounds__(kThreads, 1) k_mlp_bwd(BwdArgs a) {
-    extern __shared__ __align__(128) unsigned char smem[];
+__global__ void __launch_bounds__(kBwdThreads, 1) k_mlp_bwd(BwdArgs a) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    unsigned char *smem = align1024(smem_raw);
+    constexpr int NB = bwd_bufs<KIN>();
+    constexpr uint32_t TY = (uint32_t)kRows * NOUT * 2, TH = (uint32_t)kRows * kHidden * 2;
     unsigned char *sW2 = smem;                                  // W2: 128 rows (in) x NOUT
     unsigned char *sW1 = sW2 + (size_t)kHidden * NOUT * 2;      // W1: KIN rows (in) x 128
-    unsigned char *sY = sW1 + (size_t)KIN * kHidden * 2;        // dY tile: 128 x NOUT
-    unsigned char *sZ = sY + (size_t)kRows * NOUT * 2;          // dZ tile: 128 x 128
-    unsigned char *sH = sZ + (size_t)kRows * kHidden * 2;       // saved hidden tile: 128 x 128
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(sH + (size_t)kRows * kHidden * 2);
+    unsigned char *sIn = sW1 + (size_t)KIN * kHidden * 2;       // per tile in flight: dY 128 x NOUT, H (then dZ) 128 x 128
+    unsigned char *sOut = sIn + (size_t)NB * (TY + TH);         // dX buffers of the warps (NOUT < 128)
+    uint64_t *mbar = reinterpret_cast<uint64_t *>(sOut + (NOUT < kHidden ? 32768 : 0));
     uint32_t *tslot = reinterpret_cast<uint32_t *>(mbar + 1);
-    const int t = threadIdx.x;
+    const int tid = threadIdx.x, t = tid & (kRows - 1), part = tid >> 7, lane = tid & 31;
     const bool want_dx = a.dx != nullptr;
+    const long ntiles = (a.rows + kRows - 1) / kRows;
+    auto stage = [&](long tile, int b) {
+        unsigned char *y = sIn + (size_t)b * (TY + TH);
+        if (NOUT == kHidden) stage_sw(y, a.dy, kRows, NOUT, tile * kRows, a.rows);
+        else stage_dense(y, a.dy, kRows, NOUT, tile * kRows, a.rows);
+        stage_sw(y + TY, a.h1, kRows, kHidden, tile * kRows, a.rows);
+    };
 
     stage_dense(sW2, a.w.w2, kHidden, NOUT, 0, kHidden);
     if (want_dx) stage_dense(sW1, a.w.w1, KIN, kHidden, 0, KIN);
-    cp_wait_all();
+    if (NB > 1 && blockIdx.x < ntiles) stage(blockIdx.x, 0);
+    cp_commit();
     const uint32_t tm = tc_setup(mbar, tslot, 512);
-    const uint32_t aW1 = tc::smem_u32(sW1), aW2 = tc::smem_u32(sW2), aY = tc::smem_u32(sY), aZ = tc::smem_u32(sZ);
+    const uint32_t aW1 = tc::smem_u32(sW1), aW2 = tc::smem_u32(sW2);
     constexpr uint32_t id1 = tc::idesc_bf16(kRows, kHidden, false, false);
     constexpr int NX = KIN < 128 ? KIN : 128;   // N of one input-gradient chunk
     constexpr uint32_t idx = tc::idesc_bf16(kRows, NX, false, false);
     uint32_t phase = 0;
     bool ok = true;
-    const long ntiles = (a.rows + kRows - 1) / kRows;
-    for (long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+    int b = 0;
+    for (long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, b = NB > 1 ? b ^ 1 : 0) {
         const long row0 = tile * kRows;
         const long grow = row0 + t;
-        stage_dense(sY, a.dy, kRows, NOUT, row0, a.rows);
-        stage_dense(sH, a.h1, kRows, kHidden, row0, a.rows);
-        stage_done();
-        if (t == 0) {
+        unsigned char *sY = sIn + (size_t)b * (TY + TH), *sZ = sY + TY;
+        const uint32_t aY = tc::smem_u32(sY), aZ = tc::smem_u32(sZ);
+        if (NB > 1) {
+            if (tile + gridDim.x < ntiles) stage(tile + gridDim.x, b ^ 1);
+            cp_commit();
+            cp_wait<1>();
+        } else {
+            stage(tile, 0);
+            cp_wait_all();
+        }
+        tc::fence_async_smem();
+        tc::fence_before_sync();
+        __syncthreads();
+        if (tid == 0) {
             tc::fence_after_sync();
             for (int ks = 0; ks < NOUT / 16; ++ks)
-                mma_issue(tm, tc::kmajor_desc(aY, kRows, ks), tc::kmajor_desc(aW2, kHidden, ks), id1, ks > 0);
+                mma_issue(tm, NOUT == kHidden ? tc::kmajor_sw(aY, kRows, ks) : tc::kmajor_desc(aY, kRows, ks), tc::kmajor_desc(aW2, kHidden, ks), id1, ks > 0);
             mma_commit_issue(mbar);
         }
         ok = mma_wait(mbar, phase);
         if (!ok) break;
-        for (int c = 0; c < kHidden / 16; ++c) {
-            float v[16], h[8];
-            acc16(tm, c * 16, v);
-            if (grow < a.rows) {
-                tc::unpack8(*reinterpret_cast<const uint4 *>(sH + tc::tile_off(kRows, t, 2 * c)), h);
-                for (int k = 0; k < 8; ++k) v[k] = h[k] > 0.f ? v[k] : 0.f;
-                tc::unpack8(*reinterpret_cast<const uint4 *>(sH + tc::tile_off(kRows, t, 2 * c + 1)), h);
-                for (int k = 0; k < 8; ++k) v[8 + k] = h[k] > 0.f ? v[8 + k] : 0.f;
-            } else {
-                for (int k = 0; k < 16; ++k) v[k] = 0.f;
-            }
-            const uint4 lo = tc::pack8(v), hi = tc::pack8(v + 8);
-            *reinterpret_cast<uint4 *>(sZ + tc::tile_off(kRows, t, 2 * c)) = lo;
-            *reinterpret_cast<uint4 *>(sZ + tc::tile_off(kRows, t, 2 * c + 1)) = hi;
-            if (grow < a.rows) {
-                uint4 *dst = reinterpret_cast<uint4 *>(a.dz1 + grow * kHidden + c * 16);
-                dst[0] = lo;
-                dst[1] = hi;
+        {
+            float w[32], h[8];
+            acc32(tm, part * 32, w);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                unsigned char *at = sZ + tc::sw_off(kRows, t, part * 4 + c);
+                float *v = w + 8 * c;
+                tc::unpack8(*reinterpret_cast<const uint4 *>(at), h);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) v[k] = grow < a.rows && h[k] > 0.f ? v[k] : 0.f;
+                *reinterpret_cast<uint4 *>(at) = tc::pack8(v);
             }
         }
+        tc::fence_async_smem();
+        tc::fence_before_sync();
+        __syncthreads();
+        if (want_dx && tid == 0) {
+            tc::fence_after_sync();
+            for (int j = 0; j < KIN / NX; ++j)   // N chunk j: input features [j*NX, j*NX + NX)
+                for (int ks = 0; ks < kHidden / 16; ++ks)
+                    mma_issue(tm + kHidden + j * NX, tc::kmajor_sw(aZ, kRows, ks),
+                                 tc::kmajor_desc(aW1 + (uint32_t)(j * NX * 16), KIN, ks), idx, ks > 0);
+            mma_commit_issue(mbar);
+        }
+        for (int q = tid; q < kRows * (kHidden / 8); q += kBwdThreads) {   // dZ rows, while the tensor core reads them too
+            const int row = q >> 4, c = q & 15;
+            if (row0 + row < a.rows)
+                *reinterpret_cast<uint4 *>(a.dz1 + (row0 + row) * kHidden + c * 8) =
+                    *reinterpret_cast<const uint4 *>(sZ + tc::sw_off(kRows, row, c));
+        }
         if (want_dx) {
-            tc::fence_async_smem();
-            tc::fence_before_sync();
-            __syncthreads();
-            if (t == 0) {
-                tc::fence_after_sync();
-                for (int j = 0; j < KIN / NX; ++j)   // N chunk j: input features [j*NX, j*NX + NX)
-                    for (int ks = 0; ks < kHidden / 16; ++ks)
-                        mma_issue(tm + kHidden + j * NX, tc::kmajor_desc(aZ, kRows, ks),
-                                     tc::kmajor_desc(aW1 + (uint32_t)(j * NX * 16), KIN, ks), idx, ks > 0);
-                mma_commit_issue(mbar);
-            }
             ok = mma_wait(mbar, phase);
             if (!ok) break;
-            for (int c = 0; c < KIN / 16; ++c) {
-                float v[16];
-                acc16(tm, kHidden + c * 16, v);
-                if (grow < a.rows) {
-                    float4 *dst = reinterpret_cast<float4 *>(a.dx + grow * KIN + c * 16);
-                    for (int k = 0; k < 4; ++k) dst[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+            if constexpr (KIN >= 64) {
+                // 32 columns of 16 rows at a time
+                float4 *buf = reinterpret_cast<float4 *>((NOUT < kHidden ? sOut : sY) + (tid >> 5) * 2048);
+                const long wrow0 = row0 + (t & ~31);
+                for (int c = part; c < KIN / 32; c += 4) {
+                    float v[32];
+                    acc32(tm, kHidden + c * 32, v);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        if ((lane >> 4) == h)
+#pragma unroll
+                            for (int k = 0; k < 8; ++k)
+                                buf[(lane & 15) * 8 + ((k ^ lane) & 7)] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+                        __syncwarp();
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const int r = 4 * k + (lane >> 3), f = lane & 7;
+                            const long grow_r = wrow0 + 16 * h + r;
+                            if (grow_r < a.rows)
+                                *reinterpret_cast<float4 *>(a.dx + grow_r * KIN + c * 32 + f * 4) = buf[r * 8 + ((f ^ r) & 7)];
+                        }
+                        __syncwarp();
+                    }
+                }
+            } else if (part == 0) {
+                for (int c = 0; c < KIN / 16; ++c) {
+                    float v[16];
+                    acc16(tm, kHidden + c * 16, v);
+                    if (grow < a.rows) {
+                        float4 *dst = reinterpret_cast<float4 *>(a.dx + grow * KIN + c * 16);
+                        for (int k = 0; k < 4; ++k) dst[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+                    }
                 }
             }
         }
         tc::fence_before_sync();
         __syncthreads();
     }
+    cp_wait_all();
     tc_teardown(tm, 512, ok, a.err, mbar, phase);
 }
 
@@ -489,85 +585,155 @@ template <int KIN, int NOUT>
 __host__ __device__ constexpr int wgrad_tmem_cols() {
     return (KIN + wgrad_w2_cols<NOUT>()) <= 256 ? 256 : 512;
 }
+// Rows of a stage and stages in flight: all the shared memory holds.
+constexpr int kWgRows = 64;
 template <int KIN, int NOUT>
-constexpr size_t wgrad_smem() {
-    return (size_t)kRows * kHidden * 2 * 2 + (size_t)kRows * KIN * 2 + (size_t)kRows * NOUT * 2 + 64;
-}
+__host__ __device__ constexpr size_t wgrad_stage() { return (size_t)kWgRows * (2 * kHidden + KIN + NOUT) * 2; }
+template <int KIN>
+__host__ __device__ constexpr int wgrad_stages() { return KIN >= 2 * kHidden ? 2 : 3; }
+template <int KIN, int NOUT>
+constexpr size_t wgrad_smem() { return wgrad_stages<KIN>() * wgrad_stage<KIN, NOUT>() + 1024 + 64; }
 
+// The rows pass through a ring of stages of 64, each a K = 64 step of both products: while the tensor
+// core and the bias sums take one, the copies of the next one or two are in flight.  A stage's buffer is
+// filled again once its own products are done, a stage later.  One tile of 128 rows at a time, loaded by
+// 128 threads and summed by one thread per column, 240,000 edges took 157 us (B200); the ring with 512
+// threads 107, in the swizzled layout 64.  HBM: 246 MB, 38 us at the copy rate.
 template <int KIN, int NOUT>
-__global__ void __launch_bounds__(kThreads, 1) k_mlp_wgrad(WgradArgs a) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    unsigned char *sZ = smem;                                   // dZ tile: 128 rows x 128
-    unsigned char *sH = sZ + (size_t)kRows * kHidden * 2;       // H tile: 128 x 128
-    unsigned char *sX = sH + (size_t)kRows * kHidden * 2;       // X tile: 128 x KIN
-    unsigned char *sY = sX + (size_t)kRows * KIN * 2;           // dY tile: 128 x NOUT
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(sY + (size_t)kRows * NOUT * 2);
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(mbar + 1);
-    __shared__ int s_idx[3 * kRows];
-    const int t = threadIdx.x;
+__global__ void __launch_bounds__(kBwdThreads, 1) k_mlp_wgrad(WgradArgs a) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    unsigned char *smem = align1024(smem_raw);
+    constexpr int NS = wgrad_stages<KIN>(), R = kWgRows;
+    constexpr uint32_t SB = (uint32_t)wgrad_stage<KIN, NOUT>();
+    constexpr uint32_t OH = R * kHidden * 2, OX = 2 * OH, OY = OX + R * KIN * 2;   // dZ at 0, H, X, dY
+    uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + (size_t)NS * SB);         // one per stage
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(mbar + NS);
+    const int tid = threadIdx.x;
     constexpr int TC = wgrad_tmem_cols<KIN, NOUT>();
+    if (tid > 0 && tid < NS) tc::mbar_init(mbar + tid, 1);
     const uint32_t tm = tc_setup(mbar, tslot, TC);
-    const uint32_t aZ = tc::smem_u32(sZ), aH = tc::smem_u32(sH), aX = tc::smem_u32(sX), aY = tc::smem_u32(sY);
     constexpr int NX = KIN < 128 ? KIN : 128;
+    constexpr bool SWX = KIN % 64 == 0, SWY = NOUT == kHidden;   // swizzled tiles (16 features: plain ones)
     constexpr uint32_t idx = tc::idesc_bf16(kRows, NX, true, true);
     constexpr uint32_t id2 = tc::idesc_bf16(kRows, NOUT == kHidden ? kHidden : NOUT, true, true);
-    uint32_t phase = 0;
-    bool ok = true;
-    float db1 = 0.f, db2 = 0.f;   // thread t: bias sums of hidden unit t and output t
-    bool first = true;
     const long ntiles = (a.rows + kRows - 1) / kRows;
-    for (long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-        const long row0 = tile * kRows;
-        load_row_index(s_idx, a.src, a.nsrc, row0, a.rows);
-        __syncthreads();
-        stage_dense(sZ, a.dz1, kRows, kHidden, row0, a.rows);
-        stage_dense(sH, a.h1, kRows, kHidden, row0, a.rows);
-        stage_gather(sX, a.src, a.nsrc, KIN / 8, row0, a.rows, s_idx);
-        stage_dense(sY, a.dy, kRows, NOUT, row0, a.rows);
-        stage_done();
-        if (t == 0) {
-            tc::fence_after_sync();
-            for (int j = 0; j < KIN / NX; ++j)   // dW1^T[:, j*NX .. ] += dZ^T X_j
-                for (int ks = 0; ks < kRows / 16; ++ks)
-                    mma_issue(tm + j * NX, tc::mnmajor_desc(aZ, kRows, ks),
-                                 tc::mnmajor_desc(aX + (uint32_t)(j * (NX / 8) * kRows * 16), kRows, ks), idx,
-                                 (!first || ks > 0) ? 1u : 0u);
-            for (int ks = 0; ks < kRows / 16; ++ks) {
-                if (NOUT == kHidden)   // dW2^T += dY^T H
-                    mma_issue(tm + KIN, tc::mnmajor_desc(aY, kRows, ks), tc::mnmajor_desc(aH, kRows, ks), id2,
-                                 (!first || ks > 0) ? 1u : 0u);
-                else                   // dW2 += H^T dY (M = 128 hidden, N = NOUT)
-                    mma_issue(tm + KIN, tc::mnmajor_desc(aH, kRows, ks), tc::mnmajor_desc(aY, kRows, ks), id2,
-                                 (!first || ks > 0) ? 1u : 0u);
+    const long units = 2 * ((ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x);   // the grid has no more CTAs than tiles
+    auto fill = [&](long u) {
+        unsigned char *s = smem + (size_t)(u % NS) * SB;
+        const long row0 = (blockIdx.x + (u >> 1) * gridDim.x) * kRows + (u & 1) * R;
+        stage_sw(s, a.dz1, R, kHidden, row0, a.rows);
+        stage_sw(s + OH, a.h1, R, kHidden, row0, a.rows);
+        for (int q = tid; q < R * (KIN / 8); q += kBwdThreads) {   // the concatenated input row
+            const int row = q / (KIN / 8), kc = q % (KIN / 8);
+            unsigned char *dst = s + OX + (SWX ? tc::sw_off(R, row, kc) : tc::tile_off(R, row, kc));
+            const long grow = row0 + row;
+            if (grow < a.rows) {
+                int f = kc * 8, k;
+                const RowSrc src = pick_source(a.src, a.nsrc, f, k);
+                cp16(dst, src.p + (src.idx ? (long)src.idx[grow] : grow) * src.width + f);
+            } else {
+                *reinterpret_cast<uint4 *>(dst) = make_uint4(0, 0, 0, 0);
             }
-            mma_commit_issue(mbar);
         }
-        // bias sums from the staged tiles while the tensor core runs (fixed row order)
-        for (int r = 0; r < kRows; ++r) {
-            db1 += __bfloat162float(*reinterpret_cast<const bf16 *>(sZ + tc::tile_off(kRows, r, t >> 3) + (t & 7) * 2));
-            if (t < NOUT)
-                db2 += __bfloat162float(*reinterpret_cast<const bf16 *>(sY + tc::tile_off(kRows, r, t >> 3) + (t & 7) * 2));
-        }
-        ok = mma_wait(mbar, phase);
-        first = false;
-        tc::fence_before_sync();
-        __syncthreads();
+        if (SWY) stage_sw(s + OY, a.dy, R, NOUT, row0, a.rows);
+        else stage_dense(s + OY, a.dy, R, NOUT, row0, a.rows);
+    };
+    // bias sums: features [8 kc, 8 kc + 8) of rows r0 and r0 + 32
+    const int kc = (tid >> 4) & 15, r0 = (tid & 15) + 16 * (tid >> 8);
+    float z[8], y[8];
+    for (int k = 0; k < 8; ++k) z[k] = y[k] = 0.f;
+    bool ok = true;
+    long u = 0;
+    for (; u < NS - 1; ++u) {
+        if (u < units) fill(u);
+        cp_commit();
     }
+    for (u = 0; u < units; ++u) {
+        cp_wait<NS - 2>();   // this thread's share of stage u has landed
+        tc::fence_async_smem();
+        tc::fence_before_sync();
+        ok = __syncthreads_and(ok) != 0;
+        if (!ok) break;
+        unsigned char *s = smem + (size_t)(u % NS) * SB;
+        if (tid == 0) {
+            tc::fence_after_sync();
+            const uint32_t aZ = tc::smem_u32(s), aH = aZ + OH, aX = aZ + OX, aY = aZ + OY;
+            for (int j = 0; j < KIN / NX; ++j)   // dW1^T[:, j*NX .. ] += dZ^T X_j
+                for (int ks = 0; ks < R / 16; ++ks)
+                    mma_issue(tm + j * NX, tc::mnmajor_sw(aZ, R, ks),
+                                 SWX ? tc::mnmajor_sw(aX + (uint32_t)(j * NX * R * 2), R, ks) : tc::mnmajor_desc(aX, R, ks), idx,
+                                 (u > 0 || ks > 0) ? 1u : 0u);
+            for (int ks = 0; ks < R / 16; ++ks) {
+                if (NOUT == kHidden)   // dW2^T += dY^T H
+                    mma_issue(tm + KIN, tc::mnmajor_sw(aY, R, ks), tc::mnmajor_sw(aH, R, ks), id2,
+                                 (u > 0 || ks > 0) ? 1u : 0u);
+                else                   // dW2 += H^T dY (M = 128 hidden, N = NOUT)
+                    mma_issue(tm + KIN, tc::mnmajor_sw(aH, R, ks), tc::mnmajor_desc(aY, R, ks), id2,
+                                 (u > 0 || ks > 0) ? 1u : 0u);
+            }
+            mma_commit_issue(mbar + u % NS);
+        }
+        // stage u - 1's products are done and its sums were taken before the barrier: fill its buffer again
+        if (u > 0) ok = tc::mbar_wait(mbar + (u - 1) % NS, (uint32_t)((u - 1) / NS) & 1u, g_tc_wait_limit);
+        if (u + NS - 1 < units) fill(u + NS - 1);
+        cp_commit();
+        // bias sums from the stage while the tensor core runs (fixed row order)
+#pragma unroll
+        for (int i = 0; i < R / 32; ++i) {
+            float v[8];
+            tc::unpack8(*reinterpret_cast<const uint4 *>(s + tc::sw_off(R, r0 + 32 * i, kc)), v);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) z[k] += v[k];
+            if (kc < NOUT / 8) {
+                tc::unpack8(*reinterpret_cast<const uint4 *>(s + OY + (SWY ? tc::sw_off(R, r0 + 32 * i, kc) : tc::tile_off(R, r0 + 32 * i, kc))), v);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) y[k] += v[k];
+            }
+        }
+    }
+    cp_wait_all();
+    // the last stage's products (after a wait that gave up: of the stages issued, again with a limit)
+    if (u > 0) ok = tc::mbar_wait(mbar + (u - 1) % NS, (uint32_t)((u - 1) / NS) & 1u, g_tc_wait_limit) && ok;
+    ok = __syncthreads_and(ok) != 0;
     constexpr int NC = wgrad_cols<KIN, NOUT>();
-    float *dst = a.part + ((long)blockIdx.x * kRows + t) * NC;
-    if (ok && !first) {
+    float *part = a.part + (long)blockIdx.x * kRows * NC;
+    const int t = tid & (kRows - 1);
+    __shared__ float s_db[2][2][kHidden];   // [rows 16 (tid / 256) ..][layer]
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        for (int o = 8; o > 0; o >>= 1) {
+            z[k] += __shfl_xor_sync(0xffffffffu, z[k], o);
+            y[k] += __shfl_xor_sync(0xffffffffu, y[k], o);
+        }
+    if ((tid & 15) == 0)
+        for (int k = 0; k < 8; ++k) {
+            s_db[tid >> 8][0][kc * 8 + k] = z[k];
+            s_db[tid >> 8][1][kc * 8 + k] = y[k];
+        }
+    __syncthreads();
+    if (ok) {
         tc::fence_after_sync();
-        for (int c = 0; c < (KIN + wgrad_w2_cols<NOUT>()) / 16; ++c) {
+        float *dst = part + (long)t * NC;
+        for (int c = tid >> 7; c < (KIN + wgrad_w2_cols<NOUT>()) / 16; c += 4) {
             float v[16];
             acc16(tm, c * 16, v);
-            for (int k = 0; k < 16; ++k) dst[c * 16 + k] = v[k];
+            for (int k = 0; k < 8; ++k) *reinterpret_cast<float2 *>(dst + c * 16 + 2 * k) = make_float2(v[2 * k], v[2 * k + 1]);
         }
     } else {
-        for (int c = 0; c < NC - 2; ++c) dst[c] = 0.f;
+        for (int c = tid; c < kRows * NC; c += kBwdThreads) part[c] = 0.f;
+        __syncthreads();
     }
-    dst[NC - 2] = db1;
-    dst[NC - 1] = t < NOUT ? db2 : 0.f;
-    tc_teardown(tm, TC, ok, a.err, mbar, phase);
+    if (tid < kRows) {
+        part[(long)tid * NC + NC - 2] = s_db[0][0][tid] + s_db[1][0][tid];
+        part[(long)tid * NC + NC - 1] = s_db[0][1][tid] + s_db[1][1][tid];
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    if (tid < 32) {
+        tc::fence_after_sync();
+        tc::tmem_dealloc(tm, TC);
+    }
+    if (!ok && tid == 0 && a.err) atomicOr(a.err, DEM_ERR_TIMEOUT);
 }
 
 // p[0] + p[stride] + ... over the blocks in order, eight loads in flight.
@@ -1217,8 +1383,9 @@ int nn_mlp_backward(const dem_nn_mlp &m, long rows, const dem_nn_rows *src, int 
     int st = DEM_ERR_UNSUPPORTED;
 #define X(KI, NO)                                                                             \
     if (m.kin == KI && m.nout == NO) {                                                        \
-        st = launch_tc(k_mlp_bwd<KI, NO>, bwd_smem<KI, NO>(), 512, rows, b, s);                    \
-        if (st == DEM_OK) st = launch_tc(k_mlp_wgrad<KI, NO>, wgrad_smem<KI, NO>(), wgrad_tmem_cols<KI, NO>(), rows, g, s); \
+        st = launch_tc(k_mlp_bwd<KI, NO>, bwd_smem<KI, NO>(), 512, rows, b, s, 148, kBwdThreads);  \
+        if (st == DEM_OK)                                                                     \
+            st = launch_tc(k_mlp_wgrad<KI, NO>, wgrad_smem<KI, NO>(), wgrad_tmem_cols<KI, NO>(), rows, g, s, 148, kBwdThreads); \
     }
     B200_NN_SHAPES(X)
 #undef X

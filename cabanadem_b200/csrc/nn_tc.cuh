@@ -69,6 +69,22 @@ __device__ __forceinline__ uint64_t sdesc_sw128(uint32_t addr) {
     return d;
 }
 
+// Row tiles in the 128-byte swizzle layout: blocks of 64 features, R rows of 128 bytes each (R a multiple
+// of 8, the tile on a 1,024-byte boundary), a row's eight 16-byte chunks XOR-ed with the row's number.
+// Eight threads write or read one row's 128 bytes, or one chunk of eight rows, without bank conflicts.
+__device__ __forceinline__ uint32_t sw_off(int R, int row, int c) {
+    return (uint32_t)((c >> 3) * R * 128 + row * 128 + (((c ^ row) & 7) << 4));
+}
+// K-major operand: 16 features (k-step ks) of the rows.
+__device__ __forceinline__ uint64_t kmajor_sw(uint32_t base, int R, int ks) {
+    return sdesc_sw128(base + (uint32_t)((ks >> 2) * R * 128 + (ks & 3) * 32));
+}
+// MN-major operand: 16 rows (k-step ks) of all features; the leading offset leads to the next 64
+// features, the stride offset to the next 8 rows.
+__device__ __forceinline__ uint64_t mnmajor_sw(uint32_t base, int R, int ks) {
+    return sdesc(base + (uint32_t)(ks * 2048), (uint32_t)(R * 128), 1024u) | (uint64_t)2 << 61;
+}
+
 // ---- TMEM allocation (one full warp; power-of-two column count >= 32) ----
 __device__ __forceinline__ void tmem_alloc(uint32_t *smem_dst, int ncols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_dst)),
