@@ -14,8 +14,8 @@
 //                partials are then summed in a fixed order (k_wgrad_reduce), so the
 //                gradients are deterministic.
 //
-// One CTA of 128 threads per SM (persistent over row tiles): thread t owns tile row t, which
-// is TMEM lane t of the M = 128 accumulators.  One elected thread issues tcgen05.mma and
+// Persistent CTAs over row tiles, one per SM for the wide shapes: threads t, t + 128, ... share tile row
+// t, which is TMEM lane t of the M = 128 accumulators.  One elected thread issues tcgen05.mma and
 // commits to an mbarrier; every wait is bounded and a timeout raises the context's error
 // word instead of hanging.
 #include <cuda.h>   // CUtensorMap (encoded on the host through the driver entry point)
@@ -32,9 +32,9 @@ namespace {
 using bf16 = __nv_bfloat16;
 constexpr int kRows = 128;      // rows per tile (= MMA M)
 constexpr int kHidden = 128;    // hidden width
-constexpr int kThreads = 128;
-constexpr int kFwdThreads = 256;   // forward kernels: warps w and w + 4 split a TMEM lane quarter's columns
-constexpr int kBwdThreads = 512;   // gradient kernels: warps w, w + 4, w + 8 and w + 12 do
+constexpr int kFwdThreads = 256;   // k_edge_fwd: warps w and w + 4 split a TMEM lane quarter's columns
+constexpr int kLinThreads = 512;   // the other kernels: warps w, w + 4, w + 8 and w + 12 do
+constexpr int kBwdThreads = 512;
 
 struct RowSrc {
     const bf16 *p;
@@ -81,35 +81,6 @@ __device__ __forceinline__ RowSrc pick_source(const RowSrc *src, int nsrc, int &
         }
     }
     return r;
-}
-
-// Row indices of the tile's rows for the gathered sources: s_idx[s][row] (one round trip).
-__device__ __forceinline__ void load_row_index(int *s_idx, const RowSrc *src, int nsrc, long row0, long rows) {
-    const int t = threadIdx.x;
-    if (t < kRows) {
-        const long grow = row0 + t;
-        for (int s = 0; s < nsrc; ++s)
-            s_idx[s * kRows + t] = src[s].idx ? (grow < rows ? src[s].idx[grow] : 0) : (int)(grow < rows ? grow : 0);
-    }
-}
-
-// Queue the copies of rows [row0, row0 + kRows) of the concatenated sources (C chunks of 8
-// features per row) into a row tile of 128 rows; rows past `rows` are zero-filled.
-// s_idx must hold the tile's row indices (load_row_index + barrier).
-__device__ __forceinline__ void stage_gather(unsigned char *tile, const RowSrc *src, int nsrc, int C, long row0,
-                                             long rows, const int *s_idx) {
-    for (int q = threadIdx.x; q < kRows * C; q += blockDim.x) {
-        int row, kc;
-        tile_element(q, kRows, C, row, kc);
-        unsigned char *dst = tile + tc::tile_off(kRows, row, kc);
-        if (row0 + row < rows) {
-            int f = kc * 8, s;
-            const RowSrc r = pick_source(src, nsrc, f, s);
-            cp16(dst, r.p + (long)s_idx[s * kRows + row] * r.width + f);
-        } else {
-            *reinterpret_cast<uint4 *>(dst) = make_uint4(0, 0, 0, 0);
-        }
-    }
 }
 
 // Queue the copies of a dense row-major block [R rows][F features] (row stride F) into a row
@@ -266,76 +237,111 @@ struct FwdArgs {
     int *err;
 };
 
+// Input tiles in flight (384 features leave room for one) and threads: an SM's shared memory holds one CTA
+// of the wide shapes, so its own warps have to hide the latencies; of the narrow ones several.
+template <int KIN>
+__host__ __device__ constexpr int fwd_bufs() { return KIN > 2 * kHidden ? 1 : 2; }
+template <int KIN>
+__host__ __device__ constexpr int fwd_threads() { return KIN >= kHidden ? 512 : 256; }
+// The hidden tile lies in the input tile when that is wide enough: behind source 0 when the input is two
+// sources wide, so that a residual taken from source 0 is still there for the second epilogue.
+template <int KIN>
+__host__ __device__ constexpr bool fwd_own_hidden() { return KIN < kHidden; }
 template <int KIN, int NOUT>
 constexpr size_t fwd_smem() {
-    return (size_t)kHidden * KIN * 2 + (size_t)NOUT * kHidden * 2 + (size_t)kRows * (KIN > kHidden ? KIN : kHidden) * 2 + 64;
+    return (size_t)kHidden * KIN * 2 + (size_t)NOUT * kHidden * 2 + fwd_bufs<KIN>() * (size_t)kRows * KIN * 2 +
+           (fwd_own_hidden<KIN>() ? (size_t)kRows * kHidden * 2 : 0) + 1024 + 64;
 }
 
+// The next tile's rows arrive while this one is worked on.  Tiles of 64 features and more, the hidden and
+// the output tile are in the swizzled layout (see stage_sw).  One tile at a time, chunk-major, 200,000
+// particles took 90 us with 256 inputs (B200), now 62; 1.2 M edges and 200,000 particles with 16 inputs 222,
+// now 156.
 template <int KIN, int NOUT>
-__global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_fwd(FwdArgs a) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    constexpr int KA = KIN > kHidden ? KIN : kHidden;
-    unsigned char *sW1 = smem;                                // W1^T: 128 rows x KIN
-    unsigned char *sW2 = sW1 + (size_t)kHidden * KIN * 2;     // W2^T: NOUT rows x 128
-    unsigned char *sA = sW2 + (size_t)NOUT * kHidden * 2;     // input tile, then hidden tile
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(sA + (size_t)kRows * KA * 2);
+__global__ void __launch_bounds__(fwd_threads<KIN>(), 1) k_mlp_fwd(FwdArgs a) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    constexpr int NB = fwd_bufs<KIN>(), NT = fwd_threads<KIN>(), NP = NT / kRows;   // NP threads per row
+    constexpr bool SW = KIN % 64 == 0;
+    constexpr uint32_t TA = (uint32_t)kRows * KIN * 2;
+    unsigned char *sIn = align1024(smem_raw);                          // NB input tiles
+    unsigned char *sHid = sIn + NB * TA;                               // hidden tile of its own
+    unsigned char *sW1 = sHid + (fwd_own_hidden<KIN>() ? kRows * kHidden * 2 : 0);   // W1^T: 128 rows x KIN
+    unsigned char *sW2 = sW1 + (size_t)kHidden * KIN * 2;              // W2^T: NOUT rows x 128
+    uint64_t *mbar = reinterpret_cast<uint64_t *>(sW2 + (size_t)NOUT * kHidden * 2);
     uint32_t *tslot = reinterpret_cast<uint32_t *>(mbar + 1);
-    __shared__ int s_idx[3 * kRows];
     __shared__ float s_b1[kHidden], s_b2[kHidden];
     const int tid = threadIdx.x;
     const int t = tid & (kRows - 1);   // tile row (TMEM lane) of this thread
-    const int half = tid >> 7;         // column half [64 half, 64 half + 64) of the epilogues
-    // the hidden tile goes behind source 0 when the input is wide enough, so that a residual
-    // taken from source 0 is still in shared memory for the second epilogue
-    constexpr int HC = KIN >= 2 * kHidden ? kHidden / 8 : 0;   // first chunk of the hidden tile
-    const uint32_t aH = tc::smem_u32(sA) + (uint32_t)(HC * kRows * 16);
-    unsigned char *sOut = sA + (size_t)HC * kRows * 16;        // output tile (hidden tile is spent)
-    if (half == 0) s_b1[t] = a.w.b1[t];
-    else if (t < NOUT) s_b2[t] = a.w.b2[t];
-
+    const int part = tid >> 7;         // columns [128 / NP part, + 128 / NP) of the epilogues
+    if (tid < kHidden) s_b1[t] = a.w.b1[t];
+    else if (tid < kHidden + NOUT) s_b2[t] = a.w.b2[t];
+    const long ntiles = (a.rows + kRows - 1) / kRows;
+    auto stage = [&](long tile, int b) {
+        const long row0 = tile * kRows;
+        for (int q = tid; q < kRows * (KIN / 8); q += NT) {
+            int row = q / (KIN / 8), kc = q % (KIN / 8);
+            if (!SW) tile_element(q, kRows, KIN / 8, row, kc);
+            unsigned char *dst = sIn + b * TA + (SW ? tc::sw_off(kRows, row, kc) : tc::tile_off(kRows, row, kc));
+            const long grow = row0 + row;
+            if (grow < a.rows) {
+                int f = kc * 8, k;
+                const RowSrc r = pick_source(a.src, a.nsrc, f, k);
+                cp16(dst, r.p + (r.idx ? (long)r.idx[grow] : grow) * r.width + f);
+            } else {
+                *reinterpret_cast<uint4 *>(dst) = make_uint4(0, 0, 0, 0);
+            }
+        }
+    };
     stage_dense(sW1, a.w.w1t, kHidden, KIN, 0, kHidden);
     stage_dense(sW2, a.w.w2t, NOUT, kHidden, 0, NOUT);
-    cp_wait_all();
+    if (NB > 1 && blockIdx.x < ntiles) stage(blockIdx.x, 0);
+    cp_commit();
     const uint32_t tm = tc_setup(mbar, tslot, 128);
-    const uint32_t aW1 = tc::smem_u32(sW1), aW2 = tc::smem_u32(sW2), aA = tc::smem_u32(sA);
+    const uint32_t aW1 = tc::smem_u32(sW1), aW2 = tc::smem_u32(sW2);
     constexpr uint32_t id1 = tc::idesc_bf16(kRows, kHidden, false, false);
     constexpr uint32_t id2 = tc::idesc_bf16(kRows, NOUT, false, false);
     uint32_t phase = 0;
     bool ok = true;
-    const long ntiles = (a.rows + kRows - 1) / kRows;
-    for (long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+    int b = 0;
+    for (long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, b = NB > 1 ? b ^ 1 : 0) {
         const long row0 = tile * kRows;
         const long grow = row0 + t;
-        load_row_index(s_idx, a.src, a.nsrc, row0, a.rows);
+        unsigned char *sA = sIn + b * TA;
+        unsigned char *sH = fwd_own_hidden<KIN>() ? sHid : sA + (KIN >= 2 * kHidden ? kRows * kHidden * 2 : 0);
+        const uint32_t aA = tc::smem_u32(sA), aH = tc::smem_u32(sH);
+        if (NB > 1) {
+            if (tile + gridDim.x < ntiles) stage(tile + gridDim.x, b ^ 1);
+            cp_commit();
+            cp_wait<1>();
+        } else {
+            stage(tile, 0);
+            cp_wait_all();
+        }
+        tc::fence_async_smem();
+        tc::fence_before_sync();
         __syncthreads();
-        stage_gather(sA, a.src, a.nsrc, KIN / 8, row0, a.rows, s_idx);
-        stage_done();
         if (tid == 0) {
             tc::fence_after_sync();
             for (int ks = 0; ks < KIN / 16; ++ks)
-                mma_issue(tm, tc::kmajor_desc(aA, kRows, ks), tc::kmajor_desc(aW1, kHidden, ks), id1, ks > 0);
+                mma_issue(tm, SW ? tc::kmajor_sw(aA, kRows, ks) : tc::kmajor_desc(aA, kRows, ks), tc::kmajor_desc(aW1, kHidden, ks),
+                          id1, ks > 0);
             mma_commit_issue(mbar);
         }
         ok = mma_wait(mbar, phase);
         if (!ok) break;
         // hidden = relu(acc + b1) -> bf16 tile (A operand of GEMM2), optionally saved
-        for (int c64 = half; c64 < kHidden / 64; c64 += 2) {
-          float w[64];
-          acc64(tm, c64 * 64, w);
 #pragma unroll
-          for (int cc = 0; cc < 4; ++cc) {
-            const int c = c64 * 4 + cc;
-            float *v = w + 16 * cc;
-            for (int k = 0; k < 16; ++k) v[k] = fmaxf(v[k] + s_b1[c * 16 + k], 0.f);
-            const uint4 lo = tc::pack8(v), hi = tc::pack8(v + 8);
-            *reinterpret_cast<uint4 *>(sA + tc::tile_off(kRows, t, HC + 2 * c)) = lo;
-            *reinterpret_cast<uint4 *>(sA + tc::tile_off(kRows, t, HC + 2 * c + 1)) = hi;
-            if (a.h1 && grow < a.rows) {
-                uint4 *dst = reinterpret_cast<uint4 *>(a.h1 + grow * kHidden + c * 16);
-                dst[0] = lo;
-                dst[1] = hi;
+        for (int c32 = 0; c32 < 4 / NP; ++c32) {
+            const int c0 = (part * (4 / NP) + c32) * 32;
+            float w[32];
+            acc32(tm, c0, w);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                float *v = w + 8 * c;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) v[k] = fmaxf(v[k] + s_b1[c0 + 8 * c + k], 0.f);
+                *reinterpret_cast<uint4 *>(sH + tc::sw_off(kRows, t, c0 / 8 + c)) = tc::pack8(v);
             }
-          }
         }
         tc::fence_async_smem();
         tc::fence_before_sync();
@@ -343,61 +349,62 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_fwd(FwdArgs a) {
         if (tid == 0) {
             tc::fence_after_sync();
             for (int ks = 0; ks < kHidden / 16; ++ks)
-                mma_issue(tm, tc::kmajor_desc(aH, kRows, ks), tc::kmajor_desc(aW2, NOUT, ks), id2, ks > 0);
+                mma_issue(tm, tc::kmajor_sw(aH, kRows, ks), tc::kmajor_desc(aW2, NOUT, ks), id2, ks > 0);
             mma_commit_issue(mbar);
         }
+        auto rows_out = [&](bf16 *g) {   // the hidden tile's rows, or the output's in its place
+            for (int q = tid; q < kRows * 16; q += NT) {
+                const int row = q >> 4, c = q & 15;
+                if (row0 + row < a.rows)
+                    *reinterpret_cast<uint4 *>(g + (row0 + row) * kHidden + c * 8) =
+                        *reinterpret_cast<const uint4 *>(sH + tc::sw_off(kRows, row, c));
+            }
+        };
+        if (a.h1) rows_out(a.h1);   // while the tensor core reads them too
         ok = mma_wait(mbar, phase);
         if (!ok) break;
         constexpr bool kStaged = NOUT == kHidden;   // bf16 rows written through the output tile
-        constexpr int CB = NOUT >= 64 ? 64 : NOUT;   // columns per TMEM wait
-        for (int c64 = half; c64 < NOUT / CB; c64 += 2) {
-          float w[64];
-          if (CB == 64) acc64(tm, c64 * 64, w);
-          else acc16(tm, 0, w);
+        constexpr int CB = kStaged ? 32 : NOUT;      // columns per TMEM wait
+        static_assert(kStaged || NOUT == 16, "a narrow output is one block of 16 columns");
 #pragma unroll
-          for (int cc = 0; cc < CB / 16; ++cc) {
-            const int c = c64 * (CB / 16) + cc;
-            float *v = w + 16 * cc;
-            if (grow < a.rows) {
-                for (int k = 0; k < 16; ++k) v[k] += s_b2[c * 16 + k];
+        for (int cb = 0; cb < (kStaged ? 4 / NP : 1); ++cb) {
+            if (!kStaged && part > 0) break;
+            const int c0 = kStaged ? (part * (4 / NP) + cb) * 32 : 0;
+            float w[32];
+            if (kStaged) acc32(tm, c0, w);
+            else acc16(tm, 0, w);
+            if (grow >= a.rows) continue;
+#pragma unroll
+            for (int c = 0; c < CB / 8; ++c) {
+                float *v = w + 8 * c;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) v[k] += s_b2[c0 + 8 * c + k];
                 if (a.resid) {
                     float r[8];
-                    uint4 r0, r1;
-                    if (HC > 0 && a.resid_src0) {   // source 0 is still staged in chunks [0, 16)
-                        r0 = *reinterpret_cast<const uint4 *>(sA + tc::tile_off(kRows, t, 2 * c));
-                        r1 = *reinterpret_cast<const uint4 *>(sA + tc::tile_off(kRows, t, 2 * c + 1));
-                    } else {
-                        const uint4 *src = reinterpret_cast<const uint4 *>(a.resid + grow * NOUT + c * 16);
-                        r0 = src[0];
-                        r1 = src[1];
-                    }
-                    tc::unpack8(r0, r);
+                    if (KIN >= 2 * kHidden && a.resid_src0)   // source 0 is still staged in chunks [0, 16)
+                        tc::unpack8(*reinterpret_cast<const uint4 *>(sA + tc::sw_off(kRows, t, c0 / 8 + c)), r);
+                    else
+                        tc::unpack8(*reinterpret_cast<const uint4 *>(a.resid + grow * NOUT + c0 + 8 * c), r);
+#pragma unroll
                     for (int k = 0; k < 8; ++k) v[k] += r[k];
-                    tc::unpack8(r1, r);
-                    for (int k = 0; k < 8; ++k) v[8 + k] += r[k];
                 }
-                if (a.out && kStaged) {
-                    out_put(sOut, t, 2 * c, tc::pack8(v));
-                    out_put(sOut, t, 2 * c + 1, tc::pack8(v + 8));
-                } else if (a.out) {
-                    uint4 *dst = reinterpret_cast<uint4 *>(a.out + grow * NOUT + c * 16);
-                    dst[0] = tc::pack8(v);
-                    dst[1] = tc::pack8(v + 8);
-                }
+                if (a.out && kStaged) *reinterpret_cast<uint4 *>(sH + tc::sw_off(kRows, t, c0 / 8 + c)) = tc::pack8(v);
+                else if (a.out) *reinterpret_cast<uint4 *>(a.out + grow * NOUT + c0 + 8 * c) = tc::pack8(v);
                 if (a.out_f32) {
-                    float4 *dst = reinterpret_cast<float4 *>(a.out_f32 + grow * NOUT + c * 16);
-                    for (int k = 0; k < 4; ++k) dst[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+                    float4 *dst = reinterpret_cast<float4 *>(a.out_f32 + grow * NOUT + c0 + 8 * c);
+                    dst[0] = make_float4(v[0], v[1], v[2], v[3]);
+                    dst[1] = make_float4(v[4], v[5], v[6], v[7]);
                 }
             }
-          }
         }
         tc::fence_before_sync();
-        __syncthreads();   // TMEM and the A tile are reused by the next tile
+        __syncthreads();   // TMEM and the tiles are reused by the next tile
         if (a.out && kStaged) {
-            copy_out(sOut, a.out, row0, a.rows);
+            rows_out(a.out);
             __syncthreads();
         }
     }
+    cp_wait_all();
     tc_teardown(tm, 128, ok, a.err, mbar, phase);
 }
 
@@ -786,63 +793,114 @@ struct LinArgs {
     int *err;
 };
 
-// out = x W^T (no bias), M = 128 rows per tile, N = NOUT (<= 256), K = KIN.
+// out = x W^T (no bias), M = 128 rows per tile, N = NOUT (<= 256), K = KIN.  The next tile's rows arrive
+// while this one is worked on (swizzled layout, see stage_sw); the output leaves through a buffer per warp
+// in whole lines.  One tile at a time, chunk-major and rows written by the thread that owned them, 200,000
+// rows took 65 us with 128 in and 256 out (B200), now 35, and the 40,000 rows of the backward product,
+// added to FP32, 39, now 17.
 template <int KIN, int NOUT>
-constexpr size_t lin_smem() { return (size_t)NOUT * KIN * 2 + (size_t)kRows * KIN * 2 + 64; }
+constexpr size_t lin_smem() {
+    return (size_t)NOUT * KIN * 2 + 2 * (size_t)kRows * KIN * 2 + (kLinThreads / 32) * 2048 + 1024 + 64;
+}
 
 template <int KIN, int NOUT>
-__global__ void __launch_bounds__(kThreads, 1) k_linear(LinArgs a) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    unsigned char *sW = smem;                                  // NOUT rows x KIN
-    unsigned char *sA = sW + (size_t)NOUT * KIN * 2;           // 128 rows x KIN
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(sA + (size_t)kRows * KIN * 2);
+__global__ void __launch_bounds__(kLinThreads, 1) k_linear(LinArgs a) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    unsigned char *sA = align1024(smem_raw);                   // two tiles of 128 rows x KIN
+    constexpr uint32_t TA = (uint32_t)kRows * KIN * 2;
+    unsigned char *sW = sA + 2 * TA;                           // NOUT rows x KIN
+    unsigned char *sBuf = sW + (size_t)NOUT * KIN * 2;         // 2 KB per warp
+    uint64_t *mbar = reinterpret_cast<uint64_t *>(sBuf + (kLinThreads / 32) * 2048);
     uint32_t *tslot = reinterpret_cast<uint32_t *>(mbar + 1);
-    const int t = threadIdx.x;
-    constexpr int TC = NOUT <= 128 ? 128 : 256;
-    stage_dense(sW, a.wt, NOUT, KIN, 0, NOUT);
-    cp_wait_all();
+    const int tid = threadIdx.x, t = tid & (kRows - 1), part = tid >> 7, lane = tid & 31;
+    constexpr int TC = NOUT <= 128 ? 128 : 256, NP = kLinThreads / kRows;
+    const long ntiles = (a.rows + kRows - 1) / kRows;
+    stage_sw(sW, a.wt, NOUT, KIN, 0, NOUT);
+    if (blockIdx.x < ntiles) stage_sw(sA, a.x, kRows, KIN, (long)blockIdx.x * kRows, a.rows);
+    cp_commit();
     const uint32_t tm = tc_setup(mbar, tslot, TC);
-    const uint32_t aW = tc::smem_u32(sW), aA = tc::smem_u32(sA);
+    const uint32_t aW = tc::smem_u32(sW);
     constexpr uint32_t id = tc::idesc_bf16(kRows, NOUT, false, false);
     uint32_t phase = 0;
     bool ok = true;
-    const long ntiles = (a.rows + kRows - 1) / kRows;
-    for (long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-        const long row0 = tile * kRows, grow = row0 + t;
-        stage_dense(sA, a.x, kRows, KIN, row0, a.rows);
-        stage_done();
-        if (t == 0) {
+    int b = 0;
+    for (long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, b ^= 1) {
+        const uint32_t aA = tc::smem_u32(sA) + (uint32_t)b * TA;
+        if (tile + gridDim.x < ntiles) stage_sw(sA + (b ^ 1) * TA, a.x, kRows, KIN, (tile + gridDim.x) * kRows, a.rows);
+        cp_commit();
+        cp_wait<1>();
+        tc::fence_async_smem();
+        tc::fence_before_sync();
+        __syncthreads();
+        if (tid == 0) {
             tc::fence_after_sync();
             for (int ks = 0; ks < KIN / 16; ++ks)
-                mma_issue(tm, tc::kmajor_desc(aA, kRows, ks), tc::kmajor_desc(aW, NOUT, ks), id, ks > 0);
+                mma_issue(tm, tc::kmajor_sw(aA, kRows, ks), tc::kmajor_sw(aW, NOUT, ks), id, ks > 0);
             mma_commit_issue(mbar);
         }
         ok = mma_wait(mbar, phase);
         if (!ok) break;
-        for (int c = 0; c < NOUT / 16; ++c) {
-            float v[16];
-            acc16(tm, c * 16, v);
-            if (grow < a.rows) {
-                if (a.acc_out) {
-                    float4 *d = reinterpret_cast<float4 *>(a.acc_out + grow * NOUT + c * 16);
+        const long wrow0 = tile * kRows + (t & ~31);
+        uint4 *buf = reinterpret_cast<uint4 *>(sBuf + (tid >> 5) * 2048);
+        if (a.acc_out) {   // 32 columns of 16 rows at a time
+            for (int c = part; c < NOUT / 32; c += NP) {
+                float v[32];
+                acc32(tm, c * 32, v);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    if ((lane >> 4) == h)
+#pragma unroll
+                        for (int k = 0; k < 8; ++k)
+                            reinterpret_cast<float4 *>(buf)[(lane & 15) * 8 + ((k ^ lane) & 7)] =
+                                make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+                    __syncwarp();
+                    float4 o[4];
+#pragma unroll
                     for (int k = 0; k < 4; ++k) {
-                        float4 o = d[k];
-                        o.x += v[4 * k];
-                        o.y += v[4 * k + 1];
-                        o.z += v[4 * k + 2];
-                        o.w += v[4 * k + 3];
-                        d[k] = o;
+                        const long grow = wrow0 + 16 * h + 4 * k + (lane >> 3);
+                        if (grow < a.rows) o[k] = *reinterpret_cast<const float4 *>(a.acc_out + grow * NOUT + c * 32 + (lane & 7) * 4);
                     }
-                } else {
-                    uint4 *d = reinterpret_cast<uint4 *>(a.out + grow * NOUT + c * 16);
-                    d[0] = tc::pack8(v);
-                    d[1] = tc::pack8(v + 8);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const int r = 4 * k + (lane >> 3), f = lane & 7;
+                        const long grow = wrow0 + 16 * h + r;
+                        const float4 s = reinterpret_cast<const float4 *>(buf)[r * 8 + ((f ^ r) & 7)];
+                        if (grow < a.rows) {
+                            o[k].x += s.x;
+                            o[k].y += s.y;
+                            o[k].z += s.z;
+                            o[k].w += s.w;
+                            *reinterpret_cast<float4 *>(a.acc_out + grow * NOUT + c * 32 + f * 4) = o[k];
+                        }
+                    }
+                    __syncwarp();
+                }
+            }
+        } else {           // 64 columns of 16 rows at a time
+            for (int c = part; c < NOUT / 64; c += NP) {
+                float v[64];
+                acc64(tm, c * 64, v);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    if ((lane >> 4) == h)
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) buf[(lane & 15) * 8 + ((k ^ lane) & 7)] = tc::pack8(v + 8 * k);
+                    __syncwarp();
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const int r = 4 * k + (lane >> 3), f = lane & 7;
+                        const long grow = wrow0 + 16 * h + r;
+                        if (grow < a.rows)
+                            *reinterpret_cast<uint4 *>(a.out + grow * NOUT + c * 64 + f * 8) = buf[r * 8 + ((f ^ r) & 7)];
+                    }
+                    __syncwarp();
                 }
             }
         }
         tc::fence_before_sync();
         __syncthreads();
     }
+    cp_wait_all();
     tc_teardown(tm, TC, ok, a.err, mbar, phase);
 }
 
@@ -1245,51 +1303,78 @@ struct LinWgradArgs {
     float *part;       // [gridDim.x][128][256]
     int *err;
 };
-constexpr size_t linw_smem() { return (size_t)kRows * 256 * 2 + (size_t)kRows * kHidden * 2 + 64; }
+constexpr uint32_t kLinwStage = kWgRows * (256 + kHidden) * 2;
+constexpr int kLinwStages = 4;
+constexpr size_t linw_smem() { return kLinwStages * (size_t)kLinwStage + 1024 + 64; }
 
-__global__ void __launch_bounds__(kThreads, 1) k_linear_wgrad(LinWgradArgs a) {
-    extern __shared__ __align__(128) unsigned char smem[];
-    unsigned char *sA = smem;                              // 128 rows x 256
-    unsigned char *sB = sA + (size_t)kRows * 256 * 2;      // 128 rows x 128
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(sB + (size_t)kRows * kHidden * 2);
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(mbar + 1);
-    const int t = threadIdx.x;
+// The row pipeline of k_mlp_wgrad.  One tile of 128 rows at a time, 40,000 rows took 42 us (B200),
+// now 15.
+__global__ void __launch_bounds__(kBwdThreads, 1) k_linear_wgrad(LinWgradArgs a) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    unsigned char *smem = align1024(smem_raw);
+    constexpr int NS = kLinwStages, R = kWgRows;
+    constexpr uint32_t SB = kLinwStage, OB = R * 256 * 2;    // A rows, then B rows
+    uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + (size_t)NS * SB);
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(mbar + NS);
+    const int tid = threadIdx.x;
+    if (tid > 0 && tid < NS) tc::mbar_init(mbar + tid, 1);
     const uint32_t tm = tc_setup(mbar, tslot, 256);
-    const uint32_t aA = tc::smem_u32(sA), aB = tc::smem_u32(sB);
     constexpr uint32_t id = tc::idesc_bf16(kRows, kHidden, true, true);
-    uint32_t phase = 0;
-    bool ok = true, first = true;
     const long ntiles = (a.rows + kRows - 1) / kRows;
-    for (long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-        const long row0 = tile * kRows;
-        stage_dense(sA, a.a, kRows, 256, row0, a.rows);
-        stage_dense(sB, a.b, kRows, kHidden, row0, a.rows);
-        stage_done();
-        if (t == 0) {
-            tc::fence_after_sync();
-            for (int h = 0; h < 2; ++h)
-                for (int ks = 0; ks < kRows / 16; ++ks)
-                    mma_issue(tm + h * kHidden, tc::mnmajor_desc(aA + (uint32_t)(h * 16 * kRows * 16), kRows, ks),
-                                 tc::mnmajor_desc(aB, kRows, ks), id, (!first || ks > 0) ? 1u : 0u);
-            mma_commit_issue(mbar);
-        }
-        ok = mma_wait(mbar, phase);
-        first = false;
-        tc::fence_before_sync();
-        __syncthreads();
+    const long units = 2 * ((ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x);   // the grid has no more CTAs than tiles
+    auto fill = [&](long u) {
+        unsigned char *s = smem + (size_t)(u % NS) * SB;
+        const long row0 = (blockIdx.x + (u >> 1) * gridDim.x) * kRows + (u & 1) * R;
+        stage_sw(s, a.a, R, 256, row0, a.rows);
+        stage_sw(s + OB, a.b, R, kHidden, row0, a.rows);
+    };
+    bool ok = true;
+    long u = 0;
+    for (; u < NS - 1; ++u) {
+        if (u < units) fill(u);
+        cp_commit();
     }
-    float *dst = a.part + ((long)blockIdx.x * kRows + t) * 256;
-    if (ok && !first) {
+    for (u = 0; u < units; ++u) {
+        cp_wait<NS - 2>();
+        tc::fence_async_smem();
+        tc::fence_before_sync();
+        ok = __syncthreads_and(ok) != 0;
+        if (!ok) break;
+        if (tid == 0) {
+            tc::fence_after_sync();
+            const uint32_t aA = tc::smem_u32(smem + (size_t)(u % NS) * SB), aB = aA + OB;
+            for (int h = 0; h < 2; ++h)
+                for (int ks = 0; ks < R / 16; ++ks)
+                    mma_issue(tm + h * kHidden, tc::mnmajor_sw(aA + (uint32_t)(h * kHidden * R * 2), R, ks),
+                                 tc::mnmajor_sw(aB, R, ks), id, (u > 0 || ks > 0) ? 1u : 0u);
+            mma_commit_issue(mbar + u % NS);
+        }
+        if (u > 0) ok = tc::mbar_wait(mbar + (u - 1) % NS, (uint32_t)((u - 1) / NS) & 1u, g_tc_wait_limit);
+        if (u + NS - 1 < units) fill(u + NS - 1);
+        cp_commit();
+    }
+    cp_wait_all();
+    if (u > 0) ok = tc::mbar_wait(mbar + (u - 1) % NS, (uint32_t)((u - 1) / NS) & 1u, g_tc_wait_limit) && ok;
+    ok = __syncthreads_and(ok) != 0;
+    float *dst = a.part + ((long)blockIdx.x * kRows + (tid & (kRows - 1))) * 256;
+    if (ok) {
         tc::fence_after_sync();
-        for (int c = 0; c < 256 / 16; ++c) {
+        for (int c = tid >> 7; c < 256 / 16; c += 4) {
             float v[16];
             acc16(tm, c * 16, v);
-            for (int k = 0; k < 16; ++k) dst[c * 16 + k] = v[k];
+            for (int k = 0; k < 4; ++k)
+                *reinterpret_cast<float4 *>(dst + c * 16 + 4 * k) = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
         }
     } else {
-        for (int c = 0; c < 256; ++c) dst[c] = 0.f;
+        for (int c = tid >> 7; c < 256; c += 4) dst[c] = 0.f;
     }
-    tc_teardown(tm, 256, ok, a.err, mbar, phase);
+    tc::fence_before_sync();
+    __syncthreads();
+    if (tid < 32) {
+        tc::fence_after_sync();
+        tc::tmem_dealloc(tm, 256);
+    }
+    if (!ok && tid == 0 && a.err) atomicOr(a.err, DEM_ERR_TIMEOUT);
 }
 
 // g[o * ld + col0 + c] += sum over blocks of part[b][o][c]   (o < 128, c < 256)
@@ -1301,8 +1386,7 @@ __global__ void k_linw_reduce(const float *part, int nblocks, float *g, int ld, 
 }
 
 template <typename K, typename A>
-int launch_tc(K kernel, size_t smem, int tmem_cols, long rows, A args, cudaStream_t s, int max_blocks = 148,
-              int threads = kThreads) {
+int launch_tc(K kernel, size_t smem, int tmem_cols, long rows, A args, cudaStream_t s, int max_blocks, int threads) {
     if (rows <= 0) return DEM_OK;
     const size_t floor_bytes = tmem_cols >= 512 ? 116 * 1024 : (tmem_cols >= 256 ? 80 * 1024 : 0);
     if (smem < floor_bytes) smem = floor_bytes;
@@ -1347,7 +1431,7 @@ int nn_mlp_forward(const dem_nn_mlp &m, long rows, const dem_nn_rows *src, int n
     a.err = err;
 #define X(KI, NO) \
     if (m.kin == KI && m.nout == NO)                                                                        \
-        return launch_tc(k_mlp_fwd<KI, NO>, fwd_smem<KI, NO>(), 128, rows, a, s, 0, kFwdThreads);
+        return launch_tc(k_mlp_fwd<KI, NO>, fwd_smem<KI, NO>(), 128, rows, a, s, 0, fwd_threads<KI>());
     B200_NN_SHAPES(X)
 #undef X
     return DEM_ERR_UNSUPPORTED;
@@ -1399,13 +1483,13 @@ int nn_mlp_backward(const dem_nn_mlp &m, long rows, const dem_nn_rows *src, int 
 // PQ[rows][256] = h W1ij^T (W1ij^T: [256][128]).
 int nn_linear_pq(long rows, const void *h, const void *w1ij_t, void *pq, int *err, cudaStream_t s) {
     LinArgs a{rows, (const bf16 *)h, (const bf16 *)w1ij_t, (bf16 *)pq, nullptr, err};
-    return launch_tc(k_linear<128, 256>, lin_smem<128, 256>(), 256, rows, a, s, 0);
+    return launch_tc(k_linear<128, 256>, lin_smem<128, 256>(), 256, rows, a, s, 0, kLinThreads);
 }
 
 // dh[rows][128] += dPQ W1ij (dPQ: [rows][256] bf16, W1ij: [128][256]).
 int nn_linear_pq_backward(long rows, const void *dpq, const void *w1ij, float *dh, int *err, cudaStream_t s) {
     LinArgs a{rows, (const bf16 *)dpq, (const bf16 *)w1ij, nullptr, dh, err};
-    return launch_tc(k_linear<256, 128>, lin_smem<256, 128>(), 128, rows, a, s, 0);
+    return launch_tc(k_linear<256, 128>, lin_smem<256, 128>(), 128, rows, a, s, 0, kLinThreads);
 }
 
 // g_w1t[o][col0 + c] += sum_rows dPQ[row][c'] h[row][k] arranged as dW1ij^T (ld = row stride).
@@ -1413,7 +1497,7 @@ int nn_linear_pq_wgrad(long rows, const void *dpq, const void *h, float *g_w1t, 
                        int *err, cudaStream_t s) {
     if (rows <= 0) return DEM_OK;
     LinWgradArgs a{rows, (const bf16 *)dpq, (const bf16 *)h, part, err};
-    const int st = launch_tc(k_linear_wgrad, linw_smem(), 256, rows, a, s);
+    const int st = launch_tc(k_linear_wgrad, linw_smem(), 256, rows, a, s, 148, kBwdThreads);
     if (st) return st;
     const long ntiles = (rows + kRows - 1) / kRows;
     k_linw_reduce<<<kRows * 256 / 128, 128, 0, s>>>(part, (int)(ntiles < 148 ? ntiles : 148), g_w1t, ld, col0);
