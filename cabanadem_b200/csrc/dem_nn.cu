@@ -135,6 +135,13 @@ __device__ __forceinline__ void copy_out(const unsigned char *tile, bf16 *g, lon
     }
 }
 
+// Eight floats of shared memory in two loads (p on a 16-byte boundary).
+__device__ __forceinline__ void load8(const float *p, float v[8]) {
+    const float4 a = reinterpret_cast<const float4 *>(p)[0], b = reinterpret_cast<const float4 *>(p)[1];
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+    v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+}
+
 // Thread t reads 16 accumulator columns [col, col + 16) of its TMEM lane.
 __device__ __forceinline__ void acc16(uint32_t tm, int col, float v[16]) {
     tc::tmem_ld16(tc::tmem_warp_addr(tm, col), v);
@@ -1040,22 +1047,26 @@ __global__ void __launch_bounds__(kFwdThreads, 2) k_edge_fwd(EdgeArgs a) {
 
 // The same layer with its row tiles brought in by the tensor copy engine and the hidden tile
 // kept in tensor memory.  One CTA of 512 threads per SM: two groups of 256, each with a tile of its
-// own in flight (its e tile, accumulator, barriers), share the weights.  Per tile the e rows arrive as
+// own in flight (its e tiles, accumulator, barriers), share the weights.  Per tile the e rows arrive as
 // two 64-feature boxes of a tiled tensor copy in the 128-byte swizzle layout (one elected thread
-// issues them on an mbarrier, one tile ahead: as soon as the first product of the current tile
-// has read the buffer); the first product reads it from shared memory; the epilogue writes the
+// issues them on an mbarrier, one tile ahead, into the other of the group's two buffers); the first
+// product reads them from shared memory while the group gathers P and Q; the epilogue writes the
 // hidden activations as BF16 pairs into tensor memory (tcgen05.st), which is the A operand of
-// the second product.  Same arithmetic, in the same order, as k_edge_fwd.
+// the second product; the output rows take the place of the residual's in the e tile and leave by a
+// tensor copy, which leaves out rows past the end.  Same arithmetic, in the same order, as k_edge_fwd.
 //
-// Rows reach and leave the threads through a 4 KB buffer per warp: eight lanes read or write one
+// P, Q and the saved hidden rows pass through a 2 KB buffer per warp: eight lanes read or write one
 // row's 128 bytes in global memory, and a thread takes its own row's eight chunks from the buffer
 // (chunks XOR-swizzled by the row, no bank conflicts).  A thread reading its own row directly touched
-// 32 lines per instruction: P, Q, residual and output rows then cost 1,024 L1 wavefronts per warp and
-// tile, and two CTAs per SM spent three quarters of their time on them; now 384.  Measured (B200, 1.2 M edges):
-// 358 -> 277 us.
+// 32 lines per instruction: 1,024 L1 wavefronts per warp and tile.  What bounds it now: latency, with
+// no unit above 40 %: the gathers, two products and two epilogues of a tile follow one another, and
+// two groups are all that shared memory holds.  Measured (B200, 1.2 M edges): rows read directly 358 us,
+// through the buffers 277, with the gather behind the first product and the residual from the e tile
+// 268.  Not kept: 1,024 threads, 32 features each (64-byte gathers) 325; prefetches of the next rows
+// 269; the weights in the chunk-major layout 268.
 constexpr int kEdgeThreads = 512, kEdgeGroup = 256;
 constexpr size_t edge_tma_smem() {
-    return 1024 + 4 * (size_t)kRows * kHidden * 2 + (size_t)(kEdgeThreads / 32) * 4096 + 128;
+    return 1024 + 6 * (size_t)kRows * kHidden * 2 + (size_t)(kEdgeThreads / 32) * 2048 + 128;
 }
 
 // Barrier of one group of 256 threads (ids 1 and 2), and the same with a vote.
@@ -1092,52 +1103,65 @@ __device__ __forceinline__ void warp_rows_issue(const bf16 *base, long stride, i
 __device__ __forceinline__ void warp_rows_take(unsigned char *buf, const uint4 v[8], uint4 own[8]) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) *reinterpret_cast<uint4 *>(warp_chunk(buf, 4 * k + (lane >> 3), lane & 7)) = v[k];
-    __syncwarp();
+    for (int h = 0; h < 2; ++h) {   // 16 rows at a time
 #pragma unroll
-    for (int c = 0; c < 8; ++c) own[c] = *reinterpret_cast<const uint4 *>(warp_chunk(buf, lane, c));
-    __syncwarp();
+        for (int k = 0; k < 4; ++k)
+            *reinterpret_cast<uint4 *>(warp_chunk(buf, 4 * k + (lane >> 3), lane & 7)) = v[4 * h + k];
+        __syncwarp();
+        if ((lane >> 4) == h)
+#pragma unroll
+            for (int c = 0; c < 8; ++c) own[c] = *reinterpret_cast<const uint4 *>(warp_chunk(buf, lane & 15, c));
+        __syncwarp();
+    }
 }
 __device__ __forceinline__ void warp_rows_store(unsigned char *buf, const uint4 own[8], bf16 *g, long row0, long rows) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4 *>(warp_chunk(buf, lane, c)) = own[c];
-    __syncwarp();
+    for (int h = 0; h < 2; ++h) {
+        if ((lane >> 4) == h)
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const int row = 4 * k + (lane >> 3);
-        if (row0 + row < rows)
-            *reinterpret_cast<uint4 *>(g + (row0 + row) * kHidden + (lane & 7) * 8) =
-                *reinterpret_cast<const uint4 *>(warp_chunk(buf, row, lane & 7));
+            for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4 *>(warp_chunk(buf, lane & 15, c)) = own[c];
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int row = 4 * k + (lane >> 3);
+            const long grow = row0 + 16 * h + row;
+            if (grow < rows)
+                *reinterpret_cast<uint4 *>(g + grow * kHidden + (lane & 7) * 8) =
+                    *reinterpret_cast<const uint4 *>(warp_chunk(buf, row, lane & 7));
+        }
+        __syncwarp();
     }
-    __syncwarp();
 }
 
-__global__ void __launch_bounds__(kEdgeThreads, 1) k_edge_fwd_tma(const __grid_constant__ CUtensorMap tm_e, EdgeArgs a) {
+template <bool SAVE_H1>
+__global__ void __launch_bounds__(kEdgeThreads, 1) k_edge_fwd_tma(const __grid_constant__ CUtensorMap tm_e, const __grid_constant__ CUtensorMap tm_out,
+                                                                    EdgeArgs a) {
     // 1,024-byte alignment by hand: an extern array declared with it would raise the alignment of
     // every kernel's dynamic shared memory in this file (and their static padding with it)
     extern __shared__ __align__(128) unsigned char smem_raw[];
     constexpr uint32_t T = (uint32_t)kRows * kHidden * 2;   // one 128 x 128 BF16 tile
-    unsigned char *sE0 = smem_raw + ((1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u);   // 1,024-byte aligned
-    unsigned char *sW1 = sE0 + 2 * T;   // W1e^T 128 x 128 (row tile), after the groups' e tiles
+    unsigned char *sE0 = align1024(smem_raw);
+    unsigned char *sW1 = sE0 + 4 * T;   // W1e^T 128 x 128 (row tile), after the groups' two e tiles each
     unsigned char *sW2 = sW1 + T;       // W2^T 128 x 128 (row tile)
-    unsigned char *sBuf = sW2 + T;      // 4 KB per warp
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sBuf + (kEdgeThreads / 32) * 4096);
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(bars + 4);
-    __shared__ float s_b1[kHidden], s_b2[kHidden];
+    unsigned char *sBuf = sW2 + T;      // 2 KB per warp
+    uint64_t *bars = reinterpret_cast<uint64_t *>(sBuf + (kEdgeThreads / 32) * 2048);
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(bars + 6);
+    __shared__ __align__(16) float s_b1[kHidden], s_b2[kHidden];
     const int group = threadIdx.x / kEdgeGroup, tid = threadIdx.x % kEdgeGroup, bid = 1 + group;
     const int t = tid & (kRows - 1);   // tile row (TMEM lane)
     const int half = tid >> 7;         // features [64 half, 64 half + 64)
-    unsigned char *sE = sE0 + group * T, *buf = sBuf + (threadIdx.x >> 5) * 4096;
-    uint64_t *bar_mma = bars + 2 * group, *bar_e = bar_mma + 1;
+    unsigned char *sEg = sE0 + group * 2 * T, *buf = sBuf + (threadIdx.x >> 5) * 2048;
+    uint64_t *bar_mma = bars + 3 * group, *bar_e = bar_mma + 1;   // bar_e: one per e tile
     if (threadIdx.x < kHidden) s_b1[threadIdx.x] = a.b1[threadIdx.x];
     else if (threadIdx.x < 2 * kHidden) s_b2[threadIdx.x - kHidden] = a.b2[threadIdx.x - kHidden];
-    stage_dense(sW1, a.w1e_t, kHidden, kHidden, 0, kHidden);
-    stage_dense(sW2, a.w2t, kHidden, kHidden, 0, kHidden);
+    stage_sw(sW1, a.w1e_t, kHidden, kHidden, 0, kHidden);
+    stage_sw(sW2, a.w2t, kHidden, kHidden, 0, kHidden);
     cp_wait_all();
     if (tid == 0) {
         tc::mbar_init(bar_mma, 1);
         tc::mbar_init(bar_e, 1);
+        tc::mbar_init(bar_e + 1, 1);
         tc::mbar_init_fence();
     }
     if (threadIdx.x < 32) {
@@ -1151,20 +1175,27 @@ __global__ void __launch_bounds__(kEdgeThreads, 1) k_edge_fwd_tma(const __grid_c
     const uint32_t tm = *tslot;
     const uint32_t tacc = tm + 256u * group;   // accumulator, 128 columns (both products)
     const uint32_t ta = tacc + 128;            // hidden tile as the second product's A operand, 64 columns
-    const uint32_t aE = tc::smem_u32(sE), aW1 = tc::smem_u32(sW1), aW2 = tc::smem_u32(sW2);
+    const uint32_t aW1 = tc::smem_u32(sW1), aW2 = tc::smem_u32(sW2);
     constexpr uint32_t id = tc::idesc_bf16(kRows, kHidden, false, false);
     const long ntiles = (a.rows + kRows - 1) / kRows, step = 2L * gridDim.x;
-    auto issue_e = [&](long tile) {   // the group's thread 0: the tile's two feature boxes
-        tc::mbar_arrive_expect(bar_e, T);
-        tc::tma_load_2d(sE, &tm_e, 0, (int)(tile * kRows), bar_e);
-        tc::tma_load_2d(sE + T / 2, &tm_e, 64, (int)(tile * kRows), bar_e);
+    auto issue_e = [&](long tile, int b) {   // the group's thread 0: the tile's two feature boxes
+        unsigned char *sE = sEg + b * T;
+        tc::mbar_arrive_expect(bar_e + b, T);
+        tc::tma_load_2d(sE, &tm_e, 0, (int)(tile * kRows), bar_e + b);
+        tc::tma_load_2d(sE + T / 2, &tm_e, 64, (int)(tile * kRows), bar_e + b);
     };
     uint32_t ph_mma = 0, ph_e = 0;
     bool ok = true, e_pending = false, mma_pending = false;   // of thread 0: not yet waited for
     const long tile0 = 2L * blockIdx.x + group;
     if (tid == 0 && tile0 < ntiles) {
-        issue_e(tile0);
+        issue_e(tile0, 0);
         e_pending = true;
+    }
+    int b = 0, e_buf = 0;   // the e tile in work (ph_e: bit b its barrier's phase), and the one pending
+    int ir = 0, ic = 0;
+    if (tile0 * kRows + t < a.rows) {
+        ir = a.recv[tile0 * kRows + t];
+        ic = a.send[tile0 * kRows + t];
     }
     auto wait_mma = [&]() {
         const bool w = tc::mbar_wait(bar_mma, ph_mma, g_tc_wait_limit);
@@ -1176,59 +1207,66 @@ __global__ void __launch_bounds__(kEdgeThreads, 1) k_edge_fwd_tma(const __grid_c
         tc::fence_after_sync();
         return all;
     };
-    for (long tile = tile0; tile < ntiles; tile += step) {
+    for (long tile = tile0; tile < ntiles; tile += step, b ^= 1) {
         const long row0 = tile * kRows, grow = row0 + t, wrow0 = row0 + (t & ~31);   // the warp's first row
-        const bool live = grow < a.rows;
-        uint4 p[8], q[8];
-        {
-            const int r = live ? a.recv[grow] : 0, c = live ? a.send[grow] : 0;
-            uint4 vp[8], vq[8];
-            warp_rows_issue(a.pq + half * 64, 2 * kHidden, r, vp);
-            warp_rows_issue(a.pq + kHidden + half * 64, 2 * kHidden, c, vq);
-            warp_rows_take(buf, vp, p);
-            warp_rows_take(buf, vq, q);
-        }
+        unsigned char *sE = sEg + b * T;
+        const uint32_t aE = tc::smem_u32(sE);
         // the e tile; the group's barrier also orders every thread's reads of the previous tile's
         // accumulator before this tile's first product
-        const bool e_ok = tc::mbar_wait(bar_e, ph_e, g_tc_wait_limit);
+        const bool e_ok = tc::mbar_wait(bar_e + b, (ph_e >> b) & 1u, g_tc_wait_limit);
         if (!group_and(bid, e_ok)) {
             ok = false;
             break;
         }
-        ph_e ^= 1u;
+        ph_e ^= 1u << b;
         if (tid == 0) {
             e_pending = false;
             tc::fence_after_sync();
             for (int ks = 0; ks < kHidden / 16; ++ks)
                 mma_issue(tacc, tc::sdesc_sw128(aE + (uint32_t)(ks >> 2) * (T / 2) + (uint32_t)(ks & 3) * 32u),
-                          tc::kmajor_desc(aW1, kHidden, ks), id, ks > 0);
+                          tc::kmajor_sw(aW1, kHidden, ks), id, ks > 0);
             mma_commit_issue(bar_mma);
             mma_pending = true;
+            // the next tile's copy, once the previous tile's output has left that buffer
+            if (tile + step < ntiles) {
+                tc::bulk_wait_read();
+                issue_e(tile + step, b ^ 1);
+                e_pending = true;
+                e_buf = b ^ 1;
+            }
+        }
+        uint4 p[8], q[8];   // P and Q of the row while the first product runs; the next tile's indices
+        {
+            uint4 vp[8], vq[8];
+            warp_rows_issue(a.pq + half * 64, 2 * kHidden, ir, vp);
+            warp_rows_issue(a.pq + kHidden + half * 64, 2 * kHidden, ic, vq);
+            const long gnext = grow + step * kRows;
+            ir = gnext < a.rows ? a.recv[gnext] : 0;
+            ic = gnext < a.rows ? a.send[gnext] : 0;
+            warp_rows_take(buf, vp, p);
+            warp_rows_take(buf, vq, q);
         }
         ok = wait_mma();
         if (!ok) break;
-        // the first product has read the e tile: the next tile's copy goes into its buffer
-        if (tid == 0 && tile + step < ntiles) {
-            issue_e(tile + step);
-            e_pending = true;
-        }
         uint4 hv[8];   // the thread's hidden half row
 #pragma unroll
-        for (int b = 0; b < 2; ++b) {   // two batches of 32 columns keep the P/Q registers live
+        for (int g = 0; g < 2; ++g) {   // two batches of 32 columns keep the P/Q registers live
             float w[32];
-            acc32(tacc, half * 64 + b * 32, w);
+            acc32(tacc, half * 64 + g * 32, w);
             uint32_t hw[16];
 #pragma unroll
             for (int c2 = 0; c2 < 2; ++c2) {
-                const int cc = 2 * b + c2;
+                const int cc = 2 * g + c2;
                 const int c = half * 4 + cc;   // 16-feature group
                 float *v = w + 16 * c2, pf[8], qf[8];
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     tc::unpack8(p[2 * cc + h], pf);
                     tc::unpack8(q[2 * cc + h], qf);
-                    for (int k = 0; k < 8; ++k)
-                        v[8 * h + k] = fmaxf(v[8 * h + k] + s_b1[c * 16 + 8 * h + k] + pf[k] + qf[k], 0.f);
+                    float bias[8];
+                    load8(s_b1 + c * 16 + 8 * h, bias);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) v[8 * h + k] = fmaxf(v[8 * h + k] + bias[k] + pf[k] + qf[k], 0.f);
                 }
                 const uint4 lo = tc::pack8(v), hi = tc::pack8(v + 8);
                 hw[8 * c2 + 0] = lo.x;
@@ -1242,8 +1280,8 @@ __global__ void __launch_bounds__(kEdgeThreads, 1) k_edge_fwd_tma(const __grid_c
                 hv[2 * cc] = lo;
                 hv[2 * cc + 1] = hi;
             }
-            // features [64 half + 32 b, + 32) as 16 columns of BF16 pairs
-            tc::tmem_st16(tc::tmem_warp_addr(ta, half * 32 + b * 16), hw);
+            // features [64 half + 32 g, + 32) as 16 columns of BF16 pairs
+            tc::tmem_st16(tc::tmem_warp_addr(ta, half * 32 + g * 16), hw);
         }
         tc::tmem_wait_st();
         tc::fence_before_sync();
@@ -1251,40 +1289,44 @@ __global__ void __launch_bounds__(kEdgeThreads, 1) k_edge_fwd_tma(const __grid_c
         if (tid == 0) {
             tc::fence_after_sync();
             for (int ks = 0; ks < kHidden / 16; ++ks)
-                mma_issue_tmem_a(tacc, ta + (uint32_t)ks * 8u, tc::kmajor_desc(aW2, kHidden, ks), id, ks > 0);
+                mma_issue_tmem_a(tacc, ta + (uint32_t)ks * 8u, tc::kmajor_sw(aW2, kHidden, ks), id, ks > 0);
             mma_commit_issue(bar_mma);
             mma_pending = true;
         }
-        {   // hidden rows out (training) and the residual half row in, while the second product runs
-            uint4 v[8];
-            warp_rows_issue(a.e + half * 64, kHidden, live ? (int)grow : 0, v);
-            if (a.h1) warp_rows_store(buf, hv, a.h1 + half * 64, wrow0, a.rows);
-            warp_rows_take(buf, v, p);
-        }
+        // hidden rows out (training), while the second product runs
+        if constexpr (SAVE_H1) warp_rows_store(buf, hv, a.h1 + half * 64, wrow0, a.rows);
         ok = wait_mma();
         if (!ok) break;
-        {
-            float w[64];
-            acc64(tacc, half * 64, w);
-            uint4 o[8];
+        {   // the output half row takes the place of the residual's in the e tile
 #pragma unroll
-            for (int cc = 0; cc < 4; ++cc) {
-                const int c = half * 4 + cc;
-                float *v = w + 16 * cc, r[8];
+            for (int g = 0; g < 2; ++g) {
+                float w[32];
+                acc32(tacc, half * 64 + g * 32, w);
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    tc::unpack8(p[2 * cc + h], r);
-                    for (int k = 0; k < 8; ++k) v[8 * h + k] += s_b2[c * 16 + 8 * h + k] + r[k];
+                for (int c = 0; c < 4; ++c) {
+                    uint4 *at = reinterpret_cast<uint4 *>(sE + tc::sw_off(kRows, t, half * 8 + g * 4 + c));
+                    float *v = w + 8 * c, r[8];
+                    tc::unpack8(*at, r);
+                    float bias[8];
+                    load8(s_b2 + half * 64 + g * 32 + 8 * c, bias);
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) v[k] += bias[k] + r[k];
+                    *at = tc::pack8(v);
                 }
-                o[2 * cc] = tc::pack8(v);
-                o[2 * cc + 1] = tc::pack8(v + 8);
             }
-            warp_rows_store(buf, o, a.out + half * 64, wrow0, a.rows);
         }
+        tc::fence_async_smem();
         tc::fence_before_sync();
+        group_sync(bid);
+        if (tid == 0) {
+            tc::tma_store_2d(&tm_out, 0, (int)row0, sE);
+            tc::tma_store_2d(&tm_out, 64, (int)row0, sE + T / 2);
+            tc::bulk_commit();
+        }
     }
+    if (tid == 0) tc::bulk_wait();
     // a wait gave up: let the group's copy and product in flight land before the block's memory goes
-    if (tid == 0 && e_pending) (void)tc::mbar_wait(bar_e, ph_e, g_tc_wait_limit);
+    if (tid == 0 && e_pending) (void)tc::mbar_wait(bar_e + e_buf, (ph_e >> e_buf) & 1u, g_tc_wait_limit);
     if (tid == 0 && mma_pending) (void)tc::mbar_wait(bar_mma, ph_mma, g_tc_wait_limit);
     tc::fence_before_sync();
     __syncthreads();
@@ -1549,16 +1591,17 @@ int nn_edge_forward(long rows, const void *e, const void *pq, const int *recv, c
                (bf16 *)out, (bf16 *)h1, err};
     if (rows <= 0) return DEM_OK;
     if (form < 0) form = EDGE_FORM_DEFAULT;
-    CUtensorMap m;
-    if (form == 0 && edge_map(&m, e, rows)) {
+    CUtensorMap m, mo;
+    if (form == 0 && edge_map(&m, e, rows) && edge_map(&mo, out, rows)) {
         const size_t smem = edge_tma_smem();
-        if (cudaFuncSetAttribute(k_edge_fwd_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        const auto kernel = h1 ? k_edge_fwd_tma<true> : k_edge_fwd_tma<false>;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
             return DEM_ERR_CUDA;
         int sms = 148, dev = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         const long pairs = ((rows + kRows - 1) / kRows + 1) / 2, cap = sms > 0 ? sms : 148;   // a CTA steps two tiles
-        k_edge_fwd_tma<<<(int)(pairs < cap ? pairs : cap), kEdgeThreads, smem, s>>>(m, a);
+        kernel<<<(int)(pairs < cap ? pairs : cap), kEdgeThreads, smem, s>>>(m, mo, a);
         return cudaGetLastError() == cudaSuccess ? DEM_OK : DEM_ERR_CUDA;
     }
     return launch_tc(k_edge_fwd, edge_smem(), 128, rows, a, s, 0, kFwdThreads);

@@ -219,6 +219,18 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const void *tmap, int x, 
         : "memory");
 }
 
+// Tensor copy of a box from shared to global memory (rows past the tensor are not written), its group's
+// commit, and the wait until the group's reads of shared memory (all its writes) are done.
+__device__ __forceinline__ void tma_store_2d(const void *tmap, int x, int y, const void *src) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];" ::"l"(
+                     reinterpret_cast<uint64_t>(tmap)),
+                 "r"(x), "r"(y), "r"(smem_u32(src))
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 // TMEM address of (lane = 32 * (warp % 4), column col) for this warp's quarter.
 __device__ __forceinline__ uint32_t tmem_warp_addr(uint32_t base, int col) {
     const uint32_t q = (threadIdx.x >> 5) & 3u;
