@@ -389,9 +389,18 @@ cudaError_t launch_steps_ref_mixed(const Particles &P, const NbrList &L, Ctl *ct
 // dense layers of the surrogate (dem_nn.cu)
 int nn_mlp_forward(const dem_nn_mlp &m, long rows, const dem_nn_rows *src, int nsrc, const void *resid, void *out,
                    float *out_f32, void *h1, int *err, cudaStream_t s);
+// What the input gradient dX of a 128-in, 128-out layer is added to before it is stored: run (null: 0) +
+// row idx[row] of add (stride ld, from column col on); stored as FP32 in dx, or as BF16 in out_bf when that
+// is set.  dx may be run.
+struct DxSum {
+    const float *run, *add;
+    const int *idx;
+    int ld, col;
+    void *out_bf;
+};
 int nn_mlp_backward(const dem_nn_mlp &m, long rows, const dem_nn_rows *src, int nsrc, const void *dy, const void *h1,
                     void *dz1, float *dx, float *g_w1t, int ld_w1, float *g_b1, float *g_w2t, float *g_b2,
-                    float *part, int *err, cudaStream_t s);
+                    float *part, int *err, cudaStream_t s, const DxSum *sum = nullptr);
 long nn_wgrad_scratch(int kin, int nout);
 int nn_debug_waits(int poll_limit, int drop_mma, cudaStream_t s);
 // factorised edge layer of the surrogate (dem_nn.cu)

@@ -425,6 +425,7 @@ struct BwdArgs {
     const bf16 *h1;   // [rows][128]
     bf16 *dz1;        // [rows][128]
     float *dx;        // [rows][KIN] or null
+    DxSum sum;        // what dX is added to (the SUM form)
     int *err;
 };
 
@@ -443,8 +444,10 @@ constexpr size_t bwd_smem() {
 // whole sectors.  One CTA fills an SM's shared memory, so the epilogues' warps are all there is to hide
 // latency: four per scheduler.  With 128 threads, one tile at a time and rows written by the thread that
 // owned them, 240,000 edges took 129 us (B200); with 512 threads and this order 120, in the swizzled layout
-// 74.  HBM: 306 MB, 47 us at the copy rate.
-template <int KIN, int NOUT>
+// 74.  HBM: 306 MB, 47 us at the copy rate.  SUM: dX is added to a running sum here instead of in a pass of
+// its own (k_edge_grad 57 -> 36 us, one pass of four less) for 74 -> 105 us; the sum's loads are issued behind
+// the first product (after the second one 145).
+template <int KIN, int NOUT, bool SUM>
 __global__ void __launch_bounds__(kBwdThreads, 1) k_mlp_bwd(BwdArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char *smem = align1024(smem_raw);
@@ -500,6 +503,27 @@ __global__ void __launch_bounds__(kBwdThreads, 1) k_mlp_bwd(BwdArgs a) {
                 mma_issue(tm, NOUT == kHidden ? tc::kmajor_sw(aY, kRows, ks) : tc::kmajor_desc(aY, kRows, ks), tc::kmajor_desc(aW2, kHidden, ks), id1, ks > 0);
             mma_commit_issue(mbar);
         }
+        // what dX is added to, of the rows and columns this lane stores, while the products run
+        [[maybe_unused]] float4 base[8];
+        [[maybe_unused]] const DxSum &S = a.sum;
+        if constexpr (SUM) {
+            static_assert(KIN == kHidden, "one block of 32 columns per thread");
+            const int col = part * 32 + (lane & 7) * 4;
+            float4 d[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const long r = row0 + (t & ~31) + 4 * k + (lane >> 3), rr = r < a.rows ? r : 0;
+                base[k] = S.run ? *reinterpret_cast<const float4 *>(S.run + rr * KIN + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+                d[k] = *reinterpret_cast<const float4 *>(S.add + (long)S.idx[rr] * S.ld + S.col + col);
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                base[k].x += d[k].x;
+                base[k].y += d[k].y;
+                base[k].z += d[k].z;
+                base[k].w += d[k].w;
+            }
+        }
         ok = mma_wait(mbar, phase);
         if (!ok) break;
         {
@@ -553,8 +577,20 @@ __global__ void __launch_bounds__(kBwdThreads, 1) k_mlp_bwd(BwdArgs a) {
                         for (int k = 0; k < 4; ++k) {
                             const int r = 4 * k + (lane >> 3), f = lane & 7;
                             const long grow_r = wrow0 + 16 * h + r;
-                            if (grow_r < a.rows)
-                                *reinterpret_cast<float4 *>(a.dx + grow_r * KIN + c * 32 + f * 4) = buf[r * 8 + ((f ^ r) & 7)];
+                            float4 o = buf[r * 8 + ((f ^ r) & 7)];
+                            if constexpr (SUM) {
+                                const float4 &s = base[4 * h + k];
+                                o = make_float4(s.x + o.x, s.y + o.y, s.z + o.z, s.w + o.w);
+                            }
+                            if (grow_r < a.rows) {
+                                if (SUM && S.out_bf) {
+                                    const __nv_bfloat162 lo = __floats2bfloat162_rn(o.x, o.y), hi = __floats2bfloat162_rn(o.z, o.w);
+                                    *reinterpret_cast<uint2 *>((bf16 *)S.out_bf + grow_r * KIN + c * 32 + f * 4) =
+                                        make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
+                                } else {
+                                    *reinterpret_cast<float4 *>(a.dx + grow_r * KIN + c * 32 + f * 4) = o;
+                                }
+                            }
                         }
                         __syncwarp();
                     }
@@ -587,7 +623,7 @@ struct WgradArgs {
     const bf16 *dz1;   // [rows][128]
     const bf16 *h1;    // [rows][128]
     const bf16 *dy;    // [rows][NOUT]
-    float *part;       // [gridDim.x][128][KIN + NW2 + 2]: dW1^T | dW2 block | db1 | db2
+    float *part;       // per CTA: [128][KIN + NW2]: dW1^T | dW2 block, then db1 [128], db2 [128]
     int *err;
 };
 
@@ -612,7 +648,8 @@ constexpr size_t wgrad_smem() { return wgrad_stages<KIN>() * wgrad_stage<KIN, NO
 // core and the bias sums take one, the copies of the next one or two are in flight.  A stage's buffer is
 // filled again once its own products are done, a stage later.  One tile of 128 rows at a time, loaded by
 // 128 threads and summed by one thread per column, 240,000 edges took 157 us (B200); the ring with 512
-// threads 107, in the swizzled layout 64.  HBM: 246 MB, 38 us at the copy rate.
+// threads 107, in the swizzled layout 64, with the accumulators' rows written in whole sectors 55 (256 inputs,
+// 40,000 rows: 73 -> 24).  HBM: 246 MB, 38 us at the copy rate.
 template <int KIN, int NOUT>
 __global__ void __launch_bounds__(kBwdThreads, 1) k_mlp_wgrad(WgradArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -709,9 +746,9 @@ __global__ void __launch_bounds__(kBwdThreads, 1) k_mlp_wgrad(WgradArgs a) {
     // the last stage's products (after a wait that gave up: of the stages issued, again with a limit)
     if (u > 0) ok = tc::mbar_wait(mbar + (u - 1) % NS, (uint32_t)((u - 1) / NS) & 1u, g_tc_wait_limit) && ok;
     ok = __syncthreads_and(ok) != 0;
-    constexpr int NC = wgrad_cols<KIN, NOUT>();
+    constexpr int NM = KIN + wgrad_w2_cols<NOUT>(), NC = NM + 2;
     float *part = a.part + (long)blockIdx.x * kRows * NC;
-    const int t = tid & (kRows - 1);
+    const int t = tid & (kRows - 1), lane = tid & 31;
     __shared__ float s_db[2][2][kHidden];   // [rows 16 (tid / 256) ..][layer]
 #pragma unroll
     for (int k = 0; k < 8; ++k)
@@ -727,19 +764,29 @@ __global__ void __launch_bounds__(kBwdThreads, 1) k_mlp_wgrad(WgradArgs a) {
     __syncthreads();
     if (ok) {
         tc::fence_after_sync();
-        float *dst = part + (long)t * NC;
-        for (int c = tid >> 7; c < (KIN + wgrad_w2_cols<NOUT>()) / 16; c += 4) {
+        // the accumulators' rows through a buffer per warp in the spent stages, 16 columns at a time
+        float4 *buf = reinterpret_cast<float4 *>(smem + (tid >> 5) * 2048);
+        for (int c = tid >> 7; c < NM / 16; c += 4) {
             float v[16];
             acc16(tm, c * 16, v);
-            for (int k = 0; k < 8; ++k) *reinterpret_cast<float2 *>(dst + c * 16 + 2 * k) = make_float2(v[2 * k], v[2 * k + 1]);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                buf[lane * 4 + ((k + (lane >> 1)) & 3)] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int r = 8 * k + (lane >> 2), f = lane & 3;
+                *reinterpret_cast<float4 *>(part + (long)((t & ~31) + r) * NM + c * 16 + f * 4) = buf[r * 4 + ((f + (r >> 1)) & 3)];
+            }
+            __syncwarp();
         }
     } else {
         for (int c = tid; c < kRows * NC; c += kBwdThreads) part[c] = 0.f;
         __syncthreads();
     }
     if (tid < kRows) {
-        part[(long)tid * NC + NC - 2] = s_db[0][0][tid] + s_db[1][0][tid];
-        part[(long)tid * NC + NC - 1] = s_db[0][1][tid] + s_db[1][1][tid];
+        part[(long)kRows * NM + tid] = s_db[0][0][tid] + s_db[1][0][tid];
+        part[(long)kRows * NM + kRows + tid] = s_db[0][1][tid] + s_db[1][1][tid];
     }
     tc::fence_before_sync();
     __syncthreads();
@@ -770,10 +817,11 @@ __device__ __forceinline__ float sum_blocks(const float *p, long stride, int nbl
 __global__ void k_wgrad_reduce(const float *part, int nblocks, int kin, int nout, float *g_w1t, int ld_w1, float *g_b1,
                                float *g_w2t, float *g_b2) {
     const int nw2 = nout == kHidden ? kHidden : nout;
-    const int nc = kin + nw2 + 2;
+    const int nm = kin + nw2, nc = nm + 2;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < kRows * nc; e += gridDim.x * blockDim.x) {
-        const int r = e / nc, c = e % nc;
-        const float s = sum_blocks(part + (long)r * nc + c, (long)kRows * nc, nblocks);
+        const int bias = e - kRows * nm;   // from 0 on: db1, then db2
+        const int r = bias < 0 ? e / nm : bias % kRows, c = bias < 0 ? e % nm : nm + bias / kRows;
+        const float s = sum_blocks(part + e, (long)kRows * nc, nblocks);
         if (c < kin) g_w1t[(long)r * ld_w1 + c] += s;
         else if (c < kin + nw2) {
             const int cc = c - kin;
@@ -1398,17 +1446,27 @@ __global__ void __launch_bounds__(kBwdThreads, 1) k_linear_wgrad(LinWgradArgs a)
     cp_wait_all();
     if (u > 0) ok = tc::mbar_wait(mbar + (u - 1) % NS, (uint32_t)((u - 1) / NS) & 1u, g_tc_wait_limit) && ok;
     ok = __syncthreads_and(ok) != 0;
-    float *dst = a.part + ((long)blockIdx.x * kRows + (tid & (kRows - 1))) * 256;
+    float *part = a.part + (long)blockIdx.x * kRows * 256;
+    const int t = tid & (kRows - 1), lane = tid & 31;
     if (ok) {
         tc::fence_after_sync();
+        float4 *buf = reinterpret_cast<float4 *>(smem + (tid >> 5) * 2048);   // as in k_mlp_wgrad
         for (int c = tid >> 7; c < 256 / 16; c += 4) {
             float v[16];
             acc16(tm, c * 16, v);
+#pragma unroll
             for (int k = 0; k < 4; ++k)
-                *reinterpret_cast<float4 *>(dst + c * 16 + 4 * k) = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+                buf[lane * 4 + ((k + (lane >> 1)) & 3)] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int r = 8 * k + (lane >> 2), f = lane & 3;
+                *reinterpret_cast<float4 *>(part + (long)((t & ~31) + r) * 256 + c * 16 + f * 4) = buf[r * 4 + ((f + (r >> 1)) & 3)];
+            }
+            __syncwarp();
         }
     } else {
-        for (int c = tid >> 7; c < 256; c += 4) dst[c] = 0.f;
+        for (int c = tid; c < kRows * 256; c += kBwdThreads) part[c] = 0.f;
     }
     tc::fence_before_sync();
     __syncthreads();
@@ -1481,8 +1539,9 @@ int nn_mlp_forward(const dem_nn_mlp &m, long rows, const dem_nn_rows *src, int n
 
 int nn_mlp_backward(const dem_nn_mlp &m, long rows, const dem_nn_rows *src, int nsrc, const void *dy, const void *h1,
                     void *dz1, float *dx, float *g_w1t, int ld_w1, float *g_b1, float *g_w2t, float *g_b2,
-                    float *part, int *err, cudaStream_t s) {
+                    float *part, int *err, cudaStream_t s, const DxSum *sum) {
     BwdArgs b{};
+    if (sum) b.sum = *sum;
     b.rows = rows;
     b.w = MlpW{(const bf16 *)m.w1t, (const bf16 *)m.w1, (const bf16 *)m.w2t, (const bf16 *)m.w2, m.b1, m.b2};
     b.dy = (const bf16 *)dy;
@@ -1509,7 +1568,10 @@ int nn_mlp_backward(const dem_nn_mlp &m, long rows, const dem_nn_rows *src, int 
     int st = DEM_ERR_UNSUPPORTED;
 #define X(KI, NO)                                                                             \
     if (m.kin == KI && m.nout == NO) {                                                        \
-        st = launch_tc(k_mlp_bwd<KI, NO>, bwd_smem<KI, NO>(), 512, rows, b, s, 148, kBwdThreads);  \
+        if (KI == kHidden && NO == kHidden && sum)                                            \
+            st = launch_tc(k_mlp_bwd<kHidden, kHidden, true>, bwd_smem<KI, NO>(), 512, rows, b, s, 148, kBwdThreads); \
+        else if (!sum)                                                                        \
+            st = launch_tc(k_mlp_bwd<KI, NO, false>, bwd_smem<KI, NO>(), 512, rows, b, s, 148, kBwdThreads);  \
         if (st == DEM_OK)                                                                     \
             st = launch_tc(k_mlp_wgrad<KI, NO>, wgrad_smem<KI, NO>(), wgrad_tmem_cols<KI, NO>(), rows, g, s, 148, kBwdThreads); \
     }

@@ -239,31 +239,21 @@ __global__ void k_segsum(int n, const int *offs, const bf16 *ev, bf16 *agg) {
     }
 }
 
-// One pass over the edges' gradient between two layers of the backward pass: de (0 when `first`) +
-// dxe, the input gradient of the message layer above (null: none), + the receiver's aggregate gradient
-// dn[recv[e]][128:256] (null: none), in that order; stored in FP32 (unless it is the last pass) and as
-// the BF16 upstream gradient of the next layer.
-__global__ void k_edge_grad(int ne, const int *recv, const float *dn, const float *dxe, float *de, bf16 *dyb, int first) {
+// The upstream gradient of a message layer, in BF16: de (null: 0; the running FP32 sum, which the input
+// gradient of the layer above was added to, DxSum) + the receiver's aggregate gradient dn[recv[e]][128:256].
+// The layer's own input gradient kernel takes the same sum again and adds to it, so it is not stored in
+// FP32 here: 738 MB less per training step on 240,000 edges than a pass of its own over de, dX and dn.
+__global__ void k_edge_grad(int ne, const int *recv, const float *dn, const float *de, bf16 *dyb) {
     for (long q = blockIdx.x * (long)blockDim.x + threadIdx.x; q < (long)ne * (kH / 4); q += (long)gridDim.x * blockDim.x) {
         const long e = q / (kH / 4);
         const int c = (int)(q % (kH / 4)) * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (!first) v = *reinterpret_cast<const float4 *>(de + e * kH + c);
-        if (dxe) {
-            const float4 a = *reinterpret_cast<const float4 *>(dxe + e * kH + c);
-            v.x += a.x;
-            v.y += a.y;
-            v.z += a.z;
-            v.w += a.w;
-        }
-        if (dn) {
-            const float4 a = *reinterpret_cast<const float4 *>(dn + (long)recv[e] * 2 * kH + kH + c);
-            v.x += a.x;
-            v.y += a.y;
-            v.z += a.z;
-            v.w += a.w;
-            *reinterpret_cast<float4 *>(de + e * kH + c) = v;
-        }
+        if (de) v = *reinterpret_cast<const float4 *>(de + e * kH + c);
+        const float4 a = *reinterpret_cast<const float4 *>(dn + (long)recv[e] * 2 * kH + kH + c);
+        v.x += a.x;
+        v.y += a.y;
+        v.z += a.z;
+        v.w += a.w;
         const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
         uint2 o;
         o.x = *reinterpret_cast<const uint32_t *>(&lo);
@@ -598,7 +588,8 @@ struct dem_surrogate {
     float *out = nullptr;
     bf16 *dout = nullptr, *dz1 = nullptr, *dyb = nullptr;
     bf16 *pq = nullptr, *dpq = nullptr;   // [nodes][256] P | Q of a message layer and its gradient
-    float *dxe = nullptr, *dxn = nullptr, *dh = nullptr, *de = nullptr;
+    float *dxn = nullptr, *dh = nullptr, *de = nullptr;
+    bf16 *dye = nullptr;   // upstream gradient of the edge encoder
     double *part = nullptr, *d_loss = nullptr;
     // rollout scratch (caller order)
     double *x_prev = nullptr, *x_cur = nullptr, *x_next = nullptr, *x_tmp = nullptr, *rad = nullptr,
@@ -733,14 +724,14 @@ int ensure_edges(dem_surrogate *sg, long ne, bool training) {
     if (training && (cap > sg->ecap || !sg->train_ready)) {
         const long rows = std::max<long>(cap, sg->cap);
         for (int l = 0; l < kNL; ++l) cudaFree(sg->h1[l]);
-        cudaFree(sg->dz1); cudaFree(sg->dyb); cudaFree(sg->dxe); cudaFree(sg->de);
+        cudaFree(sg->dz1); cudaFree(sg->dyb); cudaFree(sg->dye); cudaFree(sg->de);
         for (int l = 0; l < kNL; ++l) {
             const bool edge = (l == L_ENC_E) || (l == L_MSG(0)) || (l == L_MSG(1)) || (l == L_MSG(2));
             SCK(dmalloc(&sg->h1[l], (size_t)(edge ? cap : sg->cap) * kH));
         }
         SCK(dmalloc(&sg->dz1, (size_t)rows * kH));
         SCK(dmalloc(&sg->dyb, (size_t)rows * kH));
-        SCK(dmalloc(&sg->dxe, (size_t)cap * kH));
+        SCK(dmalloc(&sg->dye, (size_t)cap * kH));
         SCK(dmalloc(&sg->de, (size_t)cap * kH));
         if (!sg->dxn) {
             SCK(dmalloc(&sg->dxn, (size_t)sg->cap * 256));
@@ -842,9 +833,10 @@ int msg_fwd(dem_surrogate *sg, int l, int n, long ne, const bf16 *h, const bf16 
     return st ? sg_fail(sg, st, "surrogate: message layer forward") : DEM_OK;
 }
 
-// Backward of msg_fwd: dy (BF16 [ne][128]) -> dE_in (sg->dxe, FP32 [ne][128]), dh += dMsg/dh,
+// Backward of msg_fwd: dy (BF16 [ne][128]) -> `sum` + dE_in (sg->de, or BF16 where sum says), dh += dMsg/dh,
 // weight gradients added.
-int msg_bwd(dem_surrogate *sg, int l, int n, long ne, const bf16 *h, const bf16 *ein, const bf16 *dy, float *dh) {
+int msg_bwd(dem_surrogate *sg, int l, int n, long ne, const bf16 *h, const bf16 *ein, const bf16 *dy, float *dh,
+            const DxSum &sum) {
     int *err;
     float *part;
     const long need = std::max(nn_wgrad_scratch(128, 128), nn_linear_wgrad_scratch());
@@ -860,7 +852,7 @@ int msg_bwd(dem_surrogate *sg, int l, int n, long ne, const bf16 *h, const bf16 
     grad_ptrs(sg, l, &gw1t, &gb1, &gw2t, &gb2);
     cudaStream_t s = ctx_stream(sg->ctx);
     dem_nn_rows src{ein, nullptr, kH};
-    int st = nn_mlp_backward(d, ne, &src, 1, dy, sg->h1[l], sg->dz1, sg->dxe, gw1t, 384, gb1, gw2t, gb2, part, err, s);
+    int st = nn_mlp_backward(d, ne, &src, 1, dy, sg->h1[l], sg->dz1, sg->de, gw1t, 384, gb1, gw2t, gb2, part, err, s, &sum);
     if (st) return sg_fail(sg, st, "surrogate: message layer backward");
     k_dpq<<<kGS, kTB, 0, s>>>(n, sg->offs, sg->rev, sg->dz1, sg->dpq);
     st = nn_linear_pq_backward(n, sg->dpq, ij, dh, err, s);
@@ -918,14 +910,14 @@ int backward(dem_surrogate *sg, int n, long ne) {
         if (ne > 0) {
             // agg_l = sum over edges of e_{l+1}: de_{l+1} += dagg[recv], after the layer above's
             // de_{l+1} += dMsg/de_{l+1}; then e_{l+1} = e_l + Msg[e_l, h_l[recv], h_l[send]]
-            k_edge_grad<<<kGS, kTB, 0, s>>>((int)ne, sg->recv, sg->dxn, l < 2 ? sg->dxe : nullptr, sg->de, sg->dyb, l == 2);
-            SG(msg_bwd(sg, L_MSG(l), n, ne, sg->h[l], sg->e[l], sg->dyb, sg->dh));   // dh += dMsg/dh_l
+            const DxSum sum{l < 2 ? sg->de : nullptr, sg->dxn, sg->recv, 2 * kH, kH, l == 0 ? sg->dye : nullptr};
+            k_edge_grad<<<kGS, kTB, 0, s>>>((int)ne, sg->recv, sg->dxn, sum.run, sg->dyb);
+            SG(msg_bwd(sg, L_MSG(l), n, ne, sg->h[l], sg->e[l], sg->dyb, sg->dh, sum));   // dh += dMsg/dh_l
         }
     }
     if (ne > 0) {
-        k_edge_grad<<<kGS, kTB, 0, s>>>((int)ne, sg->recv, nullptr, sg->dxe, sg->de, sg->dyb, 0);
         dem_nn_rows xe{sg->xe, nullptr, kF};
-        SG(mlp_bwd(sg, L_ENC_E, ne, &xe, 1, sg->dyb, nullptr));
+        SG(mlp_bwd(sg, L_ENC_E, ne, &xe, 1, sg->dye, nullptr));
     }
     k_f2bf<<<kGS, kTB, 0, s>>>((long)n * kH, sg->dh, sg->dyb);
     dem_nn_rows xn{sg->xn, nullptr, kF};
@@ -1102,7 +1094,7 @@ extern "C" int dem_surrogate_destroy(dem_surrogate *sg) {
     cudaStreamSynchronize(ctx_stream(sg->ctx));
     void *ptrs[] = {sg->w, sg->g, sg->m, sg->v, sg->wb, sg->ctl, sg->perm, sg->scene, sg->packed, sg->disp, sg->offs,
                     sg->bsum, sg->d_total, sg->recv, sg->send, sg->rev, sg->xn, sg->xe, sg->out, sg->dout, sg->dz1,
-                    sg->dyb, sg->dxe, sg->dxn, sg->dh, sg->de, sg->pq, sg->dpq, sg->part, sg->d_loss, sg->x_prev, sg->x_cur,
+                    sg->dyb, sg->dye, sg->dxn, sg->dh, sg->de, sg->pq, sg->dpq, sg->part, sg->d_loss, sg->x_prev, sg->x_cur,
                     sg->x_next, sg->x_tmp, sg->rad, sg->mass, sg->L.nn, sg->L.idx, sg->B.grid, sg->B.total, sg->B.key,
                     sg->B.cell_start, sg->B.cell_fill, sg->B.cell_items, sg->B.block_sums, sg->B.bbox};
     for (void *p : ptrs) cudaFree(p);
