@@ -46,6 +46,13 @@ struct GroupList {
     __device__ __forceinline__ int at(int, int k) const { return list[k]; }
 };
 
+// A particle's own state where the caller has it already (every lane of the group): a round trip less.
+struct CoopOwn {
+    D4 p;
+    double u[3], w[3], m, I;
+    int cs;
+};
+
 // Warp-collective: all 32 lanes call it; the groups of lanes [g NL, g NL + NL) each take one
 // particle i (i < 0: no particle, the group still takes part in the warp's shuffles).  t is
 // the particle's deferred slot.  s_tidx / s_h are the group's shared slots.
@@ -57,7 +64,7 @@ __device__ __forceinline__ void particle_coop(const Particles &P, const LIST &li
                                               const WallGeom *__restrict__ walls, const int cur, const int nxt,
                                               const int vcur, const int last, const int i, const int t,
                                               int *s_tidx, double *s_h, double *vn, double *wn, double &vmax2,
-                                              int &status, D4 *pn_out = nullptr) {
+                                              int &status, D4 *pn_out = nullptr, const CoopOwn *own = nullptr) {
     constexpr bool ONE = LIST::kOneStep;
     constexpr unsigned FULL = 0xffffffffu;
     constexpr unsigned GLOW = NL == 32 ? 0xffffffffu : ((1u << NL) - 1u);
@@ -80,7 +87,19 @@ __device__ __forceinline__ void particle_coop(const Particles &P, const LIST &li
     double ui0 = 0., ui1 = 0., ui2 = 0., wi0 = 0., wi1 = 0., wi2 = 0.;
     double2 mIi = make_double2(0., 0.);
     int mi = 0, cs0 = 0, nn = 0;
-    if (act) {
+    if (act && own) {
+        pi = own->p;
+        ui0 = own->u[0];
+        ui1 = own->u[1];
+        ui2 = own->u[2];
+        wi0 = own->w[0];
+        wi1 = own->w[1];
+        wi2 = own->w[2];
+        mIi = make_double2(own->m, own->I);
+        cs0 = own->cs;
+        nn = list.count(i);
+        mi = fc.nmat > 1 ? (int)P.mat[i] : 0;
+    } else if (act) {
         pi = ONE ? ld4_early(pc, i) : ld4(pc, i);
         ui0 = ONE ? ld_early(vc + i) : vc[i];
         ui1 = ONE ? ld_early(vc + cap + i) : vc[cap + i];

@@ -234,6 +234,8 @@ cudaError_t launch_steps_ref_mixed(const Particles &P, const NbrList &L, Ctl *ct
                              int max_steps, unsigned long long *arrive, cudaStream_t s) {
     return P.n <= kRefWideMax
                ? steps_ref_t<32, true>(P, L, ctl, fc, pp, pw, walls, R, delta, skin, max_steps, arrive, s)
+           : P.n <= kRefMidMax
+               ? steps_ref_t<16, true>(P, L, ctl, fc, pp, pw, walls, R, delta, skin, max_steps, arrive, s)
                : steps_ref_t<8, true>(P, L, ctl, fc, pp, pw, walls, R, delta, skin, max_steps, arrive, s);
 }
 

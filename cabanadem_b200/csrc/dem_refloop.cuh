@@ -3,8 +3,8 @@
 //
 // As a graph, such a step is 13 build kernels and the step kernel: 36 us for 2 spheres, 109 us for
 // 3,000, nearly all of it launches and dependent round trips of nearly empty grids.  Here a step is
-// one search-and-force pass of a resident grid and one grid barrier.  A group of NL lanes (32 or
-// 8) takes a particle: its lanes read the 27 cells around it and test their particles, the
+// one search-and-force pass of a resident grid and one grid barrier.  A group of NL lanes (32, 16
+// or 8) takes a particle: its lanes read the 27 cells around it and test their particles, the
 // candidates that can overlap go to the group's list in shared memory in ascending caller index
 // (the order of every sum), and particle_coop does the step with that list.  The group then enters
 // the new position into the next step's cell table, so the barrier at the end of a step separates
@@ -19,8 +19,8 @@
 // which grows the lists or reports the error.  The run's last step writes the lists (all
 // candidates within the cutoff) where the build kernels leave them.
 //
-// Measured (B200, FP64, us per step over 1,000 steps, graph / this loop): 2 spheres 37 / 4.4, a dense
-// cloud of 200 94 / 8.9, of 3,000 113 / 12.9, of 12,000 115 / 23, of 65,000 134 / 78; a gas of 65,000
+// Measured (B200, FP64, us per step over 1,000 steps, graph / this loop): 2 spheres 37 / 4.2, a dense
+// cloud of 200 94 / 8.5, of 3,000 113 / 11.0, of 12,000 115 / 22.9, of 65,000 134 / 78; a gas of 65,000
 // 69 / 50: faster at every size the mode's one-kernel step takes.  What bounds it: the grid barrier
 // (1.2 us: two L2 round trips and a fence) and, below some 10,000 particles, the instructions of the
 // slowest warp (a search and a contact, about 1,800 instructions at 6-8 cycles each); above, those of
@@ -33,14 +33,13 @@
 namespace b200dem {
 namespace {
 
-// Lanes per particle and the block's shape: a warp each (8 warps per SM, no register cap) while
-// every particle's warp is resident at once, else 8 lanes (12 warps per SM).  A warp each at 3,000
-// and 12,000 spheres took 15.2 and 37 us against 12.8 and 22.7 with 8 lanes; 8 lanes at 2 and 200
-// spheres 11.9 and 12.9 against 7.9 and 8.4.
-#ifndef REF_WIDE_MAX
-#define REF_WIDE_MAX 1184
-#endif
-constexpr int kRefWideMax = REF_WIDE_MAX;   // 148 SMs x 8 warps
+// Lanes per particle and the block's shape: a warp each (8 warps per SM, no register cap), then 16 lanes
+// (12 warps per SM), while every particle's lanes are resident at once, else 8 lanes.
+// A warp each at 3,000 and 12,000 spheres took 15.2 and 37 us against 12.8 and 22.7 with 8 lanes; 8 lanes at 2
+// and 200 spheres 11.9 and 12.9 against 7.9 and 8.4.  16 lanes, two cells each, against 8: 1,185 spheres 10.0,
+// 12.2; 3,000 11.0, 13.0; 3,552 11.3, 13.2.
+constexpr int kRefWideMax = 148 * 8;        // a warp each: 8 warps per SM
+constexpr int kRefMidMax = 148 * 12 * 2;    // 16 lanes each: 12 warps per SM
 template <int NL>
 struct RefShape {
     static constexpr int block = NL == 32 ? 256 : 128, min_blocks = NL == 32 ? 1 : 3;
@@ -149,16 +148,18 @@ __global__ void __launch_bounds__(RefShape<NL>::block, RefShape<NL>::min_blocks)
             if (gl == 0) S.n = S.all = 0;
             __syncwarp();
             bool busy = false;   // tracked contacts, a wall within reach (or candidates, below)
-            D4 pi = {0., 0., 0., 0.};
-            double u[3] = {0., 0., 0.}, w[3] = {0., 0., 0.}, m_i = 1.;
+            CoopOwn o = {{0., 0., 0., 0.}, {0., 0., 0.}, {0., 0., 0.}, 1., 1., 0};
+            D4 &pi = o.p;
             if (i >= 0) {
                 pi = ld4(pc, i);
-                busy = P.cstate[i] != 0;
-                m_i = P.mI[i];
+                o.cs = P.cstate[i];
+                o.m = P.mI[i];
+                o.I = P.mI[(long)cap + i];
                 for (int d = 0; d < 3; ++d) {
-                    u[d] = P.vel[vcur][d * cap + i];
-                    w[d] = P.omg[vcur][d * cap + i];
+                    o.u[d] = P.vel[vcur][d * cap + i];
+                    o.w[d] = P.omg[vcur][d * cap + i];
                 }
+                busy = o.cs != 0;
                 for (int q = gl; q < fc.nwall; q += NL) {   // a margin above the law's own test
                     const WallGeom &g = walls[q];
                     const double at = (pi.x - g.x[0]) * g.n[0] + (pi.y - g.x[1]) * g.n[1] + (pi.z - g.x[2]) * g.n[2];
@@ -242,14 +243,14 @@ __global__ void __launch_bounds__(RefShape<NL>::block, RefShape<NL>::min_blocks)
                 double v2 = 0.0;
                 particle_coop<NL, MIXED, false>(P, GroupList{S.list, i >= 0 ? nc : 0}, fc, pp, pw, walls, cur, cur ^ 1,
                                                 vcur, last, i, i, S.tidx, S.h, P.vel[vcur ^ 1], P.omg[vcur ^ 1], v2,
-                                                status, &pn);
+                                                status, &pn, &o);
             } else if (i >= 0 && gl == 0) {
                 // nothing touches this particle: the step of particle_coop without contacts
-                free_step(P, fc, i, last, m_i, u, pn);
+                free_step(P, fc, i, last, o.m, o.u, pn);
                 st4(P.pos[cur ^ 1], i, pn);
                 for (int d = 0; d < 3; ++d) {
-                    P.vel[vcur ^ 1][d * cap + i] = u[d];
-                    P.omg[vcur ^ 1][d * cap + i] = w[d];
+                    P.vel[vcur ^ 1][d * cap + i] = o.u[d];
+                    P.omg[vcur ^ 1][d * cap + i] = o.w[d];
                 }
             }
             if (i >= 0 && gl == 0) {

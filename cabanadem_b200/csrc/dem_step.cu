@@ -930,6 +930,8 @@ cudaError_t launch_steps_ref(const Particles &P, const NbrList &L, Ctl *ctl, con
         return launch_steps_ref_mixed(P, L, ctl, fc, pp, pw, walls, R, delta, skin, max_steps, arrive, s);
     return P.n <= kRefWideMax
                ? steps_ref_t<32, false>(P, L, ctl, fc, pp, pw, walls, R, delta, skin, max_steps, arrive, s)
+           : P.n <= kRefMidMax
+               ? steps_ref_t<16, false>(P, L, ctl, fc, pp, pw, walls, R, delta, skin, max_steps, arrive, s)
                : steps_ref_t<8, false>(P, L, ctl, fc, pp, pw, walls, R, delta, skin, max_steps, arrive, s);
 }
 

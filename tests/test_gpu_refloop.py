@@ -41,7 +41,7 @@ def _pair(sc, steps, grown=0, **kw):
 
 
 @pytest.mark.parametrize("precision", [_lib.DEM_FP64, _lib.DEM_MIXED], ids=["fp64", "mixed"])
-@pytest.mark.parametrize("n", [1, 2, 7, 33, 1184, 1185, 5001])
+@pytest.mark.parametrize("n", [1, 2, 7, 33, 1184, 1185, 3552, 3553, 5001])
 def test_loop_equals_graph(n, precision):
     sc = _box(n)
     sc.delta = 3.6e-3
