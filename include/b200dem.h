@@ -143,11 +143,13 @@ typedef struct dem_solver_params {
                             * overlaps that kernel's tail (it waits for that kernel's completion
                             * before it touches any state); 2 off: plain stream order.  Same
                             * results.                                                         */
-    int cooperative_loop;  /* 0 = automatic (on), 1 on: while the step is one kernel over every
-                            * particle (at most 65,536 particles, Verlet-skin mode, the graph
-                            * while-loop, steps_per_launch 0), a run's steps between neighbour
-                            * builds are one cooperative launch with a grid barrier between
-                            * steps instead of a graph replay of per-step kernels; 2 off.  Same
+    int cooperative_loop;  /* 0 = automatic (on), 1 on: steps run in cooperative launches with a grid
+                            * barrier between them instead of a graph replay of per-step kernels,
+                            * where the solver has a form for it: up to 65,536 particles (a few
+                            * forms more while few are in contact; not a dense system above the
+                            * particles resident at once), rebuild_every_step without scenes, and
+                            * systems nearly all of whose particles can reach nothing (advanced
+                            * many steps per pass).  With steps_per_launch 0.  2 off.  Same
                             * results.                                                         */
 } dem_solver_params;
 
