@@ -10,7 +10,7 @@
 //
 // k_steps_coop_lean (dem_persist.cuh) reloads each particle's state and runs the full body in every
 // thread.  Measured (B200, device us per step, that form / this one): 4,096 spheres, no pair in
-// contact 6.6 / 4.8, some 9.0 / 6.0; 30,011 spheres 11.0 / 6.9, FP32 forces 9.8 / 6.1; 200 spheres
+// contact 6.6 / 4.8, some 9.0 / 5.6; 30,011 spheres 11.0 / 6.9, FP32 forces 9.8 / 5.8; 200 spheres
 // 7.5 / 5.4; a column of disks with most in contact, 5,000 29.5 / 20.6, 56,000 36.0 / 26.2
 // (some of it the pair law's).  Contacts
 // by eight lanes each (particle_coop) instead took 11.2 us on the 4,096: some 1,400 dependent
@@ -55,6 +55,14 @@ __device__ __forceinline__ void live_contact(const Particles &P, const NbrList &
     unsigned wmask = (unsigned)cs >> 8;
     int *tidx = P.tidx + i;
     double *thx = P.th + i, *thy = P.th + (long)P.mc * cap + i, *thz = P.th + 2L * P.mc * cap + i;
+    // One tracked partner, and it is the first marked entry (most steps of a contact): the list's test
+    // decides whether its slot stays, so the partner's position is not read for the compaction first (4,096
+    // spheres 5.94 -> 5.64 us per step; columns, with several contacts each, 1 % slower).
+    const int kf = pairs ? __ffs(pairs) - 1 : nn;
+    const int t0 = cnt == 1 ? tidx[0] : -1;
+    const bool early = !MIXED && cnt == 1;   // its history with it (FP32 forces: 5.88 us with, 5.81 without)
+    const double g0 = early ? thx[0] : 0., g1 = early ? thy[0] : 0., g2 = early ? thz[0] : 0.;
+    const bool lone = t0 >= 0 && kf < nn && t0 == (kf == 0 ? j0 : kf == 1 ? j1 : L.idx[(long)kf * cap + i]);
     double F0 = 0., F1 = 0., F2 = 0., T0 = 0., T1 = 0., T2 = 0.;
     if (fc.has_ext) {
         F0 += P.ext[i];
@@ -62,7 +70,7 @@ __device__ __forceinline__ void live_contact(const Particles &P, const NbrList &
         F2 += P.ext[2 * cap + i];
     }
     // ---- update_tangential_contacts (Force.hpp:364-441)
-    if (cnt > 0) {
+    if (cnt > 0 && !lone) {
         int count = 0, k = 0;
         const int total = cnt;
         int back = cnt - 1;
@@ -101,7 +109,7 @@ __device__ __forceinline__ void live_contact(const Particles &P, const NbrList &
     }
     // ---- particle-particle (Force.hpp:73-329), list in ascending caller index
     unsigned todo = pairs;
-    for (int kk = todo ? __ffs(todo) - 1 : nn; kk < nn;) {
+    for (int kk = kf; kk < nn;) {
         const int j = kk == 0 ? j0 : kk == 1 ? j1 : L.idx[(long)kk * cap + i];
         const D4 pj = ld4(pc, j);
         const Mate b = load_mate(P.mI, vc, wc, cap, j);   // most marked entries are in contact
@@ -112,9 +120,10 @@ __device__ __forceinline__ void live_contact(const Particles &P, const NbrList &
         const double overlap = sr - rij;
         if (!(r2ij >= sr * sr * 1.0000000001) && overlap > 0.) {
             // slot lookup / insert (Force.hpp:166-192)
-            int found_at = -1;
-            for (int s = 0; s < cnt; ++s)
-                if (tidx[(long)s * cap] == j) found_at = s;
+            int found_at = lone && kk == kf ? 0 : -1;
+            if (found_at < 0)
+                for (int s = 0; s < cnt; ++s)
+                    if (tidx[(long)s * cap] == j) found_at = s;
             double h0 = 0., h1 = 0., h2 = 0.;
             if (found_at < 0) {
                 if (cnt < P.mc) {
@@ -124,6 +133,10 @@ __device__ __forceinline__ void live_contact(const Particles &P, const NbrList &
                 } else {
                     status |= DEM_ERR_CONTACT_OVERFLOW;
                 }
+            } else if (!MIXED && lone && kk == kf) {
+                h0 = g0;
+                h1 = g1;
+                h2 = g2;
             } else {
                 const long a = (long)found_at * cap;
                 h0 = thx[a];
@@ -150,6 +163,12 @@ __device__ __forceinline__ void live_contact(const Particles &P, const NbrList &
                 T1 += cf[4];
                 T2 += cf[5];
             }
+        } else if (lone && kk == kf && x.w + pj.w - rij <= 0.) {   // the compaction of the lone slot
+            tidx[0] = -1;
+            thx[0] = 0.;
+            thy[0] = 0.;
+            thz[0] = 0.;
+            cnt = 0;
         }
         if (kk < 31) {   // the next marked entry; from 31 on every entry
             todo &= todo - 1u;
