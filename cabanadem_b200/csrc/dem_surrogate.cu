@@ -755,12 +755,19 @@ int build_graph(dem_surrogate *sg, int n, const int *frame, int nframes, bool tr
     if (P.scene) SCK(cudaMemcpyAsync(sg->scene, frame, sizeof(int) * n, cudaMemcpyDeviceToDevice, s));
     BuildBuffers B = sg->B;
     B.nscenes = P.scene ? nframes : 1;
+    const int nb = (n + kScanB - 1) / kScanB;
+    int total = 0;
     for (int attempt = 0; attempt < 4; ++attempt) {
         SCK(cudaMemsetAsync(sg->ctl, 0, sizeof(Ctl), s));
         launch_build(P, sg->GA, sg->L, B, sg->ctl, sg->prm.radius_graph, 0.0, false, false, s);
+        // the edge offsets before the host has looked at the build, so that it waits once for both
+        k_scan_block<<<nb, kScanB, 0, s>>>(n, sg->L.nn, sg->offs, sg->bsum);
+        k_scan_sums<<<1, kScanB, 0, s>>>(nb, sg->bsum, sg->d_total);
+        k_scan_add<<<nb, kScanB, 0, s>>>(n, sg->offs, sg->bsum, sg->d_total);
         SCK(cudaGetLastError());
         Ctl c{};
         SCK(cudaMemcpyAsync(&c, sg->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s));
+        SCK(cudaMemcpyAsync(&total, sg->d_total, sizeof(int), cudaMemcpyDeviceToHost, s));
         SCK(cudaStreamSynchronize(s));
         if (c.status & DEM_ERR_NAN) return sg_fail(sg, DEM_ERR_NAN, "surrogate: non-finite positions");
         if (!(c.status & DEM_ERR_NEIGHBOR_OVERFLOW)) break;
@@ -770,13 +777,6 @@ int build_graph(dem_surrogate *sg, int n, const int *frame, int nframes, bool tr
         sg->L.maxnb = want;
         SCK(dmalloc(&sg->L.idx, (size_t)want * sg->cap));
     }
-    const int nb = (n + kScanB - 1) / kScanB;
-    k_scan_block<<<nb, kScanB, 0, s>>>(n, sg->L.nn, sg->offs, sg->bsum);
-    k_scan_sums<<<1, kScanB, 0, s>>>(nb, sg->bsum, sg->d_total);
-    k_scan_add<<<nb, kScanB, 0, s>>>(n, sg->offs, sg->bsum, sg->d_total);
-    int total = 0;
-    SCK(cudaMemcpyAsync(&total, sg->d_total, sizeof(int), cudaMemcpyDeviceToHost, s));
-    SCK(cudaStreamSynchronize(s));
     int st = ensure_edges(sg, total, training);
     if (st) return st;
     k_csr_fill<<<kGS, kTB, 0, s>>>(n, sg->cap, sg->L.nn, sg->L.idx, sg->offs, sg->recv, sg->send);
@@ -946,13 +946,13 @@ int loss_grad(dem_surrogate *sg, int n, const double *prev, const double *cur, c
     k_loss<<<kLossBlocks, kTB, 0, s>>>(n, sg->out, sg->packed, sg->disp, next, 1.0 / sg->prm.sigma_a, sg->dout, sg->part);
     k_sum_parts<<<1, kTB, 0, s>>>(kLossBlocks, sg->part, sg->d_loss);
     SG(backward(sg, n, ne));
-    SCK(cudaMemcpyAsync(loss, sg->d_loss, sizeof(double), cudaMemcpyDeviceToHost, s));
-    SCK(cudaStreamSynchronize(s));
     int *err;
     float *part;
     SG(ctx_nn_scratch(sg->ctx, 0, &err, &part));
     int e = 0;
-    SCK(cudaMemcpy(&e, err, sizeof(int), cudaMemcpyDeviceToHost));
+    SCK(cudaMemcpyAsync(loss, sg->d_loss, sizeof(double), cudaMemcpyDeviceToHost, s));
+    SCK(cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, s));
+    SCK(cudaStreamSynchronize(s));
     if (e) return sg_fail(sg, e, "surrogate: tensor-core kernel gave up waiting");
     return DEM_OK;
 }
