@@ -21,7 +21,7 @@
 //
 // Bounds: 120 bytes per particle and flight (HBM), and four FP64 operations per particle, step and
 // axis along a force, one along the others; at kFlightSteps = 64 about as long.  Measured (B200, device us per
-// step, three-kernel step / this one): 2,000,000 spheres 57 / 8.0; 300,007, FP32 forces 19 / 5.4; 70,001
+// step, three-kernel step / this one): 2,000,000 spheres 57 / 7.4; 300,007, FP32 forces 19 / 5.4; 70,001
 // 14.3 / 4.6.
 #pragma once
 #include "dem_particle.cuh"
