@@ -36,15 +36,15 @@ __device__ __forceinline__ void ld_acquire_b128(const void *p, unsigned long lon
 }
 
 // Largest of the warp's non-negative doubles, exactly: the high words, then the low words of those
-// that share the largest high word.
+// that share the largest high word.  A NaN counts as 0, as in finish_step (its bits would be the largest
+// of all and end the displacement bound): the next list build reports it.
 __device__ __forceinline__ unsigned long long warp_max_bits(double v) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    const unsigned long long b = (unsigned long long)__double_as_longlong(fmax(v, 0.0));
     const unsigned hi = (unsigned)(b >> 32);
     const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
     const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)b : 0u);
     return ((unsigned long long)mh << 32) | ml;
 }
-
 
 // Step k (0, 1, ... of the launch) ends: v2 >= 0 of the thread, count of the warp (the same in its
 // lanes).  Returns false when the wait gave up (DEM_ERR_TIMEOUT is set); else `big` holds the bits of
