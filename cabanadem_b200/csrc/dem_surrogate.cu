@@ -580,6 +580,7 @@ struct dem_surrogate {
     double2 *disp = nullptr;
     int *offs = nullptr, *bsum = nullptr, *d_total = nullptr;
     long ecap = 0;               // edge capacity
+    long tcap = 0;               // edge capacity of the training buffers
     int *recv = nullptr, *send = nullptr, *rev = nullptr;
     // activations
     bf16 *xn = nullptr, *xe = nullptr;
@@ -705,11 +706,12 @@ int alloc_nodes(dem_surrogate *sg) {
     return DEM_OK;
 }
 
-// Edge-capacity buffers (grown on demand).
+// Edge-capacity buffers (grown on demand): the graph's and the edge latents', and for training, which
+// may lag behind them, the gradients' (tcap edges).
 int ensure_edges(dem_surrogate *sg, long ne, bool training) {
-    const bool need_train = training && !sg->train_ready;
+    const bool need_train = training && (!sg->train_ready || ne > sg->tcap);
     if (ne <= sg->ecap && !need_train) return DEM_OK;
-    const long cap = std::max<long>(ne + ne / 4, sg->ecap);
+    const long cap = ne > sg->ecap ? ne + ne / 4 : sg->ecap;
     cudaStream_t s = ctx_stream(sg->ctx);
     SCK(cudaStreamSynchronize(s));
     if (cap > sg->ecap) {
@@ -721,7 +723,7 @@ int ensure_edges(dem_surrogate *sg, long ne, bool training) {
         SCK(dmalloc(&sg->xe, (size_t)cap * kF));
         for (int k = 0; k < 4; ++k) SCK(dmalloc(&sg->e[k], (size_t)cap * kH));
     }
-    if (training && (cap > sg->ecap || !sg->train_ready)) {
+    if (need_train) {
         const long rows = std::max<long>(cap, sg->cap);
         for (int l = 0; l < kNL; ++l) cudaFree(sg->h1[l]);
         cudaFree(sg->dz1); cudaFree(sg->dyb); cudaFree(sg->dye); cudaFree(sg->de);
@@ -740,6 +742,7 @@ int ensure_edges(dem_surrogate *sg, long ne, bool training) {
             SCK(dmalloc(&sg->dpq, (size_t)sg->cap * 2 * kH));
         }
         sg->train_ready = true;
+        sg->tcap = cap;
     }
     sg->ecap = cap;
     return DEM_OK;
