@@ -145,6 +145,7 @@ _PROTOS = {
     "dem_nn_status": ([_VP, C.POINTER(C.c_int)], C.c_int),
     "dem_nn_debug_waits": ([_VP, C.c_int, C.c_int], C.c_int),
     "dem_solver_debug_stream_waits": ([_VP, C.c_int, C.c_int], C.c_int),
+    "dem_ctx_debug_fail_alloc": ([_VP, C.c_int], C.c_int),
     "dem_particles_get_device": ([_VP, C.c_int, _VP, C.c_long], C.c_int),
     "dem_particles_clear_contacts": ([_VP], C.c_int),
     "dem_particles_clear_forces": ([_VP], C.c_int),

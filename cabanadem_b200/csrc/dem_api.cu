@@ -29,6 +29,7 @@ struct dem_ctx {
     int *d_err = nullptr;           // error word of the tensor-core kernels
     float *nn_part = nullptr;       // per-CTA weight-gradient partials
     long nn_part_floats = 0;
+    int fail_alloc = 0;             // dem_ctx_debug_fail_alloc: > 0 the allocation to fail, counted down
 };
 
 struct dem_particles {
@@ -2552,6 +2553,12 @@ extern "C" int dem_solver_debug_stream_waits(dem_solver *s, int poll_limit, int 
     return DEM_OK;
 }
 
+extern "C" int dem_ctx_debug_fail_alloc(dem_ctx *ctx, int nth) {
+    if (!ctx || nth < 0) return DEM_ERR_INVALID;
+    ctx->fail_alloc = nth;
+    return DEM_OK;
+}
+
 extern "C" int dem_nn_debug_waits(dem_ctx *ctx, int poll_limit, int drop_mma) {
     if (!ctx || poll_limit < 0) return DEM_ERR_INVALID;
     const int st = nn_debug_waits(poll_limit, drop_mma, ctx->stream);
@@ -2587,6 +2594,16 @@ void solver_particles_changed(dem_solver *s) {
 cudaStream_t ctx_stream(dem_ctx *ctx) { return ctx->stream; }
 int ctx_fail(dem_ctx *ctx, int code, const char *msg) { return fail(ctx, code, msg); }
 int ctx_cuda(dem_ctx *ctx, cudaError_t e, const char *what) { return cuda_check(ctx, e, what); }
+cudaError_t ctx_malloc(dem_ctx *ctx, void **p, size_t bytes) {
+    *p = nullptr;
+    if (ctx->fail_alloc > 0 && --ctx->fail_alloc == 0) return cudaErrorMemoryAllocation;
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) {
+        *p = nullptr;
+        (void)cudaGetLastError();   // reported here: the next call's checks start clean
+    }
+    return e;
+}
 int ctx_nn_scratch(dem_ctx *ctx, long part_floats, int **err, float **part) {
     const int st = nn_prepare(ctx, part_floats);
     *err = ctx->d_err;

@@ -427,5 +427,8 @@ cudaStream_t ctx_stream(dem_ctx *ctx);
 int ctx_fail(dem_ctx *ctx, int code, const char *msg);
 int ctx_cuda(dem_ctx *ctx, cudaError_t e, const char *what);
 int ctx_nn_scratch(dem_ctx *ctx, long part_floats, int **err, float **part);
+// cudaMalloc of a buffer that grows between calls (dem_ctx_debug_fail_alloc counts these): null and no
+// error left pending when it fails.
+cudaError_t ctx_malloc(dem_ctx *ctx, void **p, size_t bytes);
 
 }  // namespace b200dem

@@ -706,6 +706,18 @@ int alloc_nodes(dem_surrogate *sg) {
     return DEM_OK;
 }
 
+// A buffer that is made larger: given back first, then allocated; whatever fails, no pointer is left to
+// freed memory and the capacity says what is there.
+template <typename T>
+void release(T *&p) {
+    cudaFree(p);
+    p = nullptr;
+}
+template <typename T>
+cudaError_t grow(dem_surrogate *sg, T **p, size_t count) {
+    return ctx_malloc(sg->ctx, reinterpret_cast<void **>(p), std::max<size_t>(count, 1) * sizeof(T));
+}
+
 // Edge-capacity buffers (grown on demand): the graph's and the edge latents', and for training, which
 // may lag behind them, the gradients' (tcap edges).
 int ensure_edges(dem_surrogate *sg, long ne, bool training) {
@@ -715,36 +727,37 @@ int ensure_edges(dem_surrogate *sg, long ne, bool training) {
     cudaStream_t s = ctx_stream(sg->ctx);
     SCK(cudaStreamSynchronize(s));
     if (cap > sg->ecap) {
-        cudaFree(sg->recv); cudaFree(sg->send); cudaFree(sg->rev); cudaFree(sg->xe);
-        for (int k = 0; k < 4; ++k) cudaFree(sg->e[k]);
-        SCK(dmalloc(&sg->recv, cap));
-        SCK(dmalloc(&sg->send, cap));
-        SCK(dmalloc(&sg->rev, cap));
-        SCK(dmalloc(&sg->xe, (size_t)cap * kF));
-        for (int k = 0; k < 4; ++k) SCK(dmalloc(&sg->e[k], (size_t)cap * kH));
+        release(sg->recv), release(sg->send), release(sg->rev), release(sg->xe);
+        for (int k = 0; k < 4; ++k) release(sg->e[k]);
+        sg->ecap = 0;
+        SCK(grow(sg, &sg->recv, cap));
+        SCK(grow(sg, &sg->send, cap));
+        SCK(grow(sg, &sg->rev, cap));
+        SCK(grow(sg, &sg->xe, (size_t)cap * kF));
+        for (int k = 0; k < 4; ++k) SCK(grow(sg, &sg->e[k], (size_t)cap * kH));
+        sg->ecap = cap;
     }
     if (need_train) {
         const long rows = std::max<long>(cap, sg->cap);
-        for (int l = 0; l < kNL; ++l) cudaFree(sg->h1[l]);
-        cudaFree(sg->dz1); cudaFree(sg->dyb); cudaFree(sg->dye); cudaFree(sg->de);
+        for (int l = 0; l < kNL; ++l) release(sg->h1[l]);
+        release(sg->dz1), release(sg->dyb), release(sg->dye), release(sg->de);
+        release(sg->dxn), release(sg->dh), release(sg->dout), release(sg->dpq);
+        sg->train_ready = false;
         for (int l = 0; l < kNL; ++l) {
             const bool edge = (l == L_ENC_E) || (l == L_MSG(0)) || (l == L_MSG(1)) || (l == L_MSG(2));
-            SCK(dmalloc(&sg->h1[l], (size_t)(edge ? cap : sg->cap) * kH));
+            SCK(grow(sg, &sg->h1[l], (size_t)(edge ? cap : sg->cap) * kH));
         }
-        SCK(dmalloc(&sg->dz1, (size_t)rows * kH));
-        SCK(dmalloc(&sg->dyb, (size_t)rows * kH));
-        SCK(dmalloc(&sg->dye, (size_t)cap * kH));
-        SCK(dmalloc(&sg->de, (size_t)cap * kH));
-        if (!sg->dxn) {
-            SCK(dmalloc(&sg->dxn, (size_t)sg->cap * 256));
-            SCK(dmalloc(&sg->dh, (size_t)sg->cap * kH));
-            SCK(dmalloc(&sg->dout, (size_t)sg->cap * kF));
-            SCK(dmalloc(&sg->dpq, (size_t)sg->cap * 2 * kH));
-        }
+        SCK(grow(sg, &sg->dz1, (size_t)rows * kH));
+        SCK(grow(sg, &sg->dyb, (size_t)rows * kH));
+        SCK(grow(sg, &sg->dye, (size_t)cap * kH));
+        SCK(grow(sg, &sg->de, (size_t)cap * kH));
+        SCK(grow(sg, &sg->dxn, (size_t)sg->cap * 256));
+        SCK(grow(sg, &sg->dh, (size_t)sg->cap * kH));
+        SCK(grow(sg, &sg->dout, (size_t)sg->cap * kF));
+        SCK(grow(sg, &sg->dpq, (size_t)sg->cap * 2 * kH));
         sg->train_ready = true;
         sg->tcap = cap;
     }
-    sg->ecap = cap;
     return DEM_OK;
 }
 
@@ -776,9 +789,10 @@ int build_graph(dem_surrogate *sg, int n, const int *frame, int nframes, bool tr
         if (!(c.status & DEM_ERR_NEIGHBOR_OVERFLOW)) break;
         if (c.max_nbr > 128 || attempt == 3) return sg_fail(sg, DEM_ERR_NEIGHBOR_OVERFLOW, "surrogate: > 128 graph neighbours");
         const int want = std::min(std::max(2 * sg->L.maxnb, c.max_nbr + 8), 128);
-        cudaFree(sg->L.idx);
+        release(sg->L.idx);
+        sg->L.maxnb = 0;
+        SCK(grow(sg, &sg->L.idx, (size_t)want * sg->cap));
         sg->L.maxnb = want;
-        SCK(dmalloc(&sg->L.idx, (size_t)want * sg->cap));
     }
     int st = ensure_edges(sg, total, training);
     if (st) return st;
@@ -963,14 +977,16 @@ int loss_grad(dem_surrogate *sg, int n, const double *prev, const double *cur, c
 // Caller-order scratch of the rollout (and, of it, predict's projection), kept between calls.
 int ensure_rollout(dem_surrogate *sg, int n) {
     if (sg->roll_n < n) {
-        cudaFree(sg->x_prev); cudaFree(sg->x_cur); cudaFree(sg->x_next); cudaFree(sg->x_tmp); cudaFree(sg->rad);
-        cudaFree(sg->mass);
-        SCK(dmalloc(&sg->x_prev, 3 * (size_t)n));
-        SCK(dmalloc(&sg->x_tmp, 3 * (size_t)n));
-        SCK(dmalloc(&sg->x_cur, 3 * (size_t)n));
-        SCK(dmalloc(&sg->x_next, 3 * (size_t)n));
-        SCK(dmalloc(&sg->rad, n));
-        SCK(dmalloc(&sg->mass, n));
+        SCK(cudaStreamSynchronize(ctx_stream(sg->ctx)));
+        release(sg->x_prev), release(sg->x_cur), release(sg->x_next), release(sg->x_tmp), release(sg->rad);
+        release(sg->mass);
+        sg->roll_n = 0;
+        SCK(grow(sg, &sg->x_prev, 3 * (size_t)n));
+        SCK(grow(sg, &sg->x_tmp, 3 * (size_t)n));
+        SCK(grow(sg, &sg->x_cur, 3 * (size_t)n));
+        SCK(grow(sg, &sg->x_next, 3 * (size_t)n));
+        SCK(grow(sg, &sg->rad, n));
+        SCK(grow(sg, &sg->mass, n));
         sg->roll_n = n;
     }
     return DEM_OK;

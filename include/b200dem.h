@@ -448,6 +448,11 @@ int dem_nn_debug_waits(dem_ctx *ctx, int poll_limit, int drop_mma);
  * unfinished (the particle state must be set again).  Calling with drop_copies = 0 also clears
  * the DEM_ERR_TIMEOUT bit of the solver's control word. */
 int dem_solver_debug_stream_waits(dem_solver *s, int poll_limit, int drop_copies);
+/* The nth allocation from now on of a buffer that grows between calls (a surrogate's edge, training
+ * and rollout buffers, a solver's cell tables) of this context's objects reports out of memory, for
+ * testing that the call which meets it fails or falls back cleanly and the object stays usable
+ * (no reference counterpart).  nth 0: none. */
+int dem_ctx_debug_fail_alloc(dem_ctx *ctx, int nth);
 
 /* ---- Learned surrogate: message-passing network over the contact graph -------------------
  * Quasi-2D (x, y) particles.  One network stride replaces `steps_per_stride` DEM steps:

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from cabanadem_b200 import api, scenarios as S, surrogate as SG
+from cabanadem_b200 import _lib, api, scenarios as S, surrogate as SG
 
 pytestmark = pytest.mark.gpu
 
@@ -38,6 +38,50 @@ def test_training_buffers_follow_a_prediction_on_more_edges():
     fresh = _surrogate(ctx)
     want = fresh.loss_grad(*large)
     assert loss == want[0] and np.array_equal(grad, want[1])
+    sg.close()
+    fresh.close()
+    ctx.close()
+
+
+@pytest.mark.parametrize("nth", [1, 4, 8, 9, 11, 14])
+def test_prediction_after_one_that_ran_out_of_memory(nth):
+    """The edges' buffers (eight) and the projection's (six) grow for a larger frame; where one of them
+    cannot be had, the call reports it and the object still predicts."""
+    ctx = api.Context(0)
+    sg = _surrogate(ctx)
+    with torch.cuda.stream(sg.stream):
+        small, large = _frame(300, "cuda"), _frame(4000, "cuda")
+
+    def predict(s, t):
+        return s.predict(t[0], t[1], t[3]).cpu().numpy()
+
+    before = predict(sg, small)
+    assert _lib.lib().dem_ctx_debug_fail_alloc(ctx.h, nth) == 0
+    with pytest.raises(_lib.DemError, match="out of memory"):
+        predict(sg, large)
+    assert np.array_equal(predict(sg, small), before)
+    fresh = _surrogate(ctx)
+    assert np.array_equal(predict(sg, large), predict(fresh, large))
+    sg.close()
+    fresh.close()
+    ctx.close()
+
+
+@pytest.mark.parametrize("nth", [1, 8, 9, 20, 25])
+def test_training_after_a_call_that_ran_out_of_memory(nth):
+    ctx = api.Context(0)
+    sg = _surrogate(ctx)
+    with torch.cuda.stream(sg.stream):
+        small, large = _frame(300, "cuda"), _frame(4000, "cuda")
+    before = sg.loss_grad(*small)
+    assert _lib.lib().dem_ctx_debug_fail_alloc(ctx.h, nth) == 0
+    with pytest.raises(_lib.DemError, match="out of memory"):
+        sg.loss_grad(*large)
+    after = sg.loss_grad(*small)
+    assert after[0] == before[0] and np.array_equal(after[1], before[1])
+    fresh = _surrogate(ctx)
+    got, want = sg.loss_grad(*large), fresh.loss_grad(*large)
+    assert got[0] == want[0] and np.array_equal(got[1], want[1])
     sg.close()
     fresh.close()
     ctx.close()
