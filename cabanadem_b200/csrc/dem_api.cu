@@ -110,6 +110,7 @@ struct dem_solver {
     int quiet_wait = 0;                         // builds until quiet classes are tried again
     bool live_off = false;                      // the last step was too dense for several particles per thread
     RefTables ref{};                            // cell tables of the rebuild-every-step loop
+    bool ref_refused = false;                   // they could not be allocated
 };
 
 struct dem_bonds {
@@ -1653,22 +1654,30 @@ bool coop_loop(const dem_solver *s) {
 // The rebuild-every-step mode's run in one cooperative launch (dem_refloop.cuh): the one-kernel
 // step of a small system without batched scenes, static walls, no mesh.
 bool ref_loop(const dem_solver *s) {
-    return ref_mode(s) && s->sp.cooperative_loop != 2 && !s->coop_refused && s->fc.all == 1 &&
+    return ref_mode(s) && s->sp.cooperative_loop != 2 && !s->coop_refused && !s->ref_refused && s->fc.all == 1 &&
            s->p->P.n <= kCoopMaxN && s->loop && !s->fc.mwalls && s->mesh_nt == 0 && !s->p->P.scene && s->nscenes == 0 &&
            s->p->P.mc <= kCoopSlots;
 }
 
-int ensure_ref_tables(dem_solver *s) {
-    if (s->ref.count) return DEM_OK;
-    dem_ctx *ctx = s->ctx;
+// The loop's tables (204 bytes per cell key: 107 MB at 65,536 particles); false when they cannot be had.
+bool ensure_ref_tables(dem_solver *s) {
     RefTables &R = s->ref;
+    if (R.count) return true;
     R.grid = s->B.grid;
     R.total = s->B.total;
     R.codes = s->B.cell_cap;
-    CK(dalloc(&R.item, 3 * (size_t)R.codes * kRefCell));
-    CK(dalloc(&R.key, 3 * (size_t)s->p->P.cap));
-    CK(dalloc(&R.count, 3 * (size_t)R.codes));
-    return DEM_OK;
+    void *item = nullptr, *key = nullptr, *count = nullptr;
+    if (ctx_malloc(s->ctx, &item, 3 * (size_t)R.codes * kRefCell * sizeof(int)) != cudaSuccess ||
+        ctx_malloc(s->ctx, &key, 3 * (size_t)s->p->P.cap * sizeof(int)) != cudaSuccess ||
+        ctx_malloc(s->ctx, &count, 3 * (size_t)R.codes * sizeof(int)) != cudaSuccess) {
+        cudaFree(item);
+        cudaFree(key);
+        return false;
+    }
+    R.item = static_cast<int *>(item);
+    R.key = static_cast<int *>(key);
+    R.count = static_cast<int *>(count);
+    return true;
 }
 
 // Steps of a run in the rebuild-every-step mode, as many as the cooperative launch takes.
@@ -1677,8 +1686,11 @@ int run_ref_loop(dem_solver *s, int nsteps, bool *left) {
     dem_ctx *ctx = s->ctx;
     cudaStream_t st = ctx->stream;
     *left = true;
-    int e = ensure_ref_tables(s);
-    if (e) return e;
+    if (!ensure_ref_tables(s)) {   // the graph needs none
+        s->ref_refused = true;
+        return DEM_OK;
+    }
+    int e = DEM_OK;
     if (!s->d_coop) CK(dalloc(&s->d_coop, (size_t)kCoopScratch));
     s->ref.grid = s->B.grid;
     for (int done = 0;;) {
