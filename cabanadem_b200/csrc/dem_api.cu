@@ -1681,8 +1681,8 @@ bool ensure_ref_tables(dem_solver *s) {
 }
 
 // Steps of a run in the rebuild-every-step mode, as many as the cooperative launch takes.
-// *left: steps the graph of build and step kernels has to do.
-int run_ref_loop(dem_solver *s, int nsteps, bool *left) {
+// *left: steps the graph of build and step kernels has to do; *taken: the loop's.
+int run_ref_loop(dem_solver *s, int nsteps, bool *left, int *taken) {
     dem_ctx *ctx = s->ctx;
     cudaStream_t st = ctx->stream;
     *left = true;
@@ -1707,6 +1707,7 @@ int run_ref_loop(dem_solver *s, int nsteps, bool *left) {
         CK(cudaGetLastError());
         if (c.status & DEM_ERR_TIMEOUT) return fail(ctx, DEM_ERR_TIMEOUT, "a bounded device wait gave up");
         if (c.steps_done > done) s->coop_ran = true;
+        *taken = c.steps_done;
         if (c.status & DEM_ERR_NEIGHBOR_OVERFLOW) {   // the step was done, its list did not fit
             if (c.max_nbr > 128) return fail(ctx, DEM_ERR_NEIGHBOR_OVERFLOW, "more than 128 neighbours");
             e = alloc_lists(s, std::min(std::max(2 * s->L.maxnb, c.max_nbr + 8), 128));
@@ -1779,7 +1780,7 @@ extern "C" int dem_solver_run(dem_solver *s, int nsteps) {
     bool graph_steps = ref_mode(s);
     if (graph_steps) s->coop_ran = false;
     if (ref_loop(s)) {
-        const int e = run_ref_loop(s, nsteps, &graph_steps);
+        const int e = run_ref_loop(s, nsteps, &graph_steps, &steps_before);   // the graph's launches count from there
         if (e) return e;
     }
     if (ref_mode(s)) {

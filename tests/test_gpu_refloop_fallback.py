@@ -1,5 +1,5 @@
 """The rebuild-every-step loop (dem_refloop.cuh) where it cannot go on: tables that cannot be had, cells
-that fill up in the middle of a run or in every step.  The graph of build and step kernels
+that fill up in the middle of a run.  The graph of build and step kernels
 (cooperative_loop 2) takes the steps left, with the same results."""
 import numpy as np
 import pytest
@@ -37,3 +37,30 @@ def test_no_memory_for_the_tables(nth):
         assert np.array_equal(x, y)
     s.close()
     ctx.close()
+
+
+def test_a_cell_that_fills_up_in_the_middle_of_a_run():
+    """Spheres with a thin cutoff that fly together: the loop takes the first steps, a cell becomes full,
+    the loop starts again on a fresh grid and the graph takes what it cannot do."""
+    n, r = 216, 1e-3
+    sc = S.hcp_box(n=n, seed=4, vmax=0.0)
+    k = np.arange(n)
+    sc.state.rad[:] = 0.05 * r                         # small spheres ...
+    sc.state.rad[0] = r                                # ... and a large one, which makes the cells wide
+    sc.state.x[:] = np.stack([k % 6, (k // 6) % 6, k // 36], axis=1) * 2.0 * r + 3e-3
+    sc.state.x[0] = sc.state.x.max(axis=0) + 8e-3
+    sc.state.u[:] = -(sc.state.x - sc.state.x[1:].mean(axis=0)) * 2000.0
+    sc.state.u[0] = 0.0
+    sc.walls.x[:] -= 1.0 * sc.walls.normal
+    sc.delta, sc.gravity = 3e-3, (0.0, 0.0, 0.0)
+    out = []
+    for coop in (0, 2):
+        s = api.from_scenario(sc, rebuild_every_step=True, cooperative_loop=coop, max_neighbors=128)
+        s.run_steps(4000)
+        out.append((_state(s), s.stats()))
+    (a, sa), (b, sb) = out
+    for x, y in zip(a, b):
+        assert np.array_equal(x, y)
+    assert sa["cooperative_loop"] == 1 and sb["cooperative_loop"] == 0
+    # both forms took steps: more launches than the loop alone, far fewer than the graph (14 per step)
+    assert 4000 < sa["launches"] < sb["launches"] - 14 * 1000
