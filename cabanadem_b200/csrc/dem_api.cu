@@ -111,6 +111,7 @@ struct dem_solver {
     bool live_off = false;                      // the last step was too dense for several particles per thread
     RefTables ref{};                            // cell tables of the rebuild-every-step loop
     bool ref_refused = false;                   // they could not be allocated
+    int ref_wait = 0;                           // runs until the loop is tried again (kRefRetry)
 };
 
 struct dem_bonds {
@@ -1680,12 +1681,21 @@ bool ensure_ref_tables(dem_solver *s) {
     return true;
 }
 
+// Runs that go straight to the graph after one of whose steps the loop could take none (cells that are full
+// in every step: spheres much smaller than the cutoff).  A failed attempt costs 40 us, 8 % of a run of one
+// step (900 spheres, B200: 0.494 ms the graph alone, 0.533 with an attempt in each run).
+constexpr int kRefRetry = 16;
+
 // Steps of a run in the rebuild-every-step mode, as many as the cooperative launch takes.
 // *left: steps the graph of build and step kernels has to do; *taken: the loop's.
 int run_ref_loop(dem_solver *s, int nsteps, bool *left, int *taken) {
     dem_ctx *ctx = s->ctx;
     cudaStream_t st = ctx->stream;
     *left = true;
+    if (s->ref_wait > 0) {
+        --s->ref_wait;
+        return DEM_OK;
+    }
     if (!ensure_ref_tables(s)) {   // the graph needs none
         s->ref_refused = true;
         return DEM_OK;
@@ -1723,7 +1733,10 @@ int run_ref_loop(dem_solver *s, int nsteps, bool *left, int *taken) {
             *left = false;
             return DEM_OK;
         }
-        if (c.steps_done == done) return DEM_OK;   // no progress on a fresh grid: the graph
+        if (c.steps_done == done) {   // no progress on a fresh grid: the graph
+            if (done == 0) s->ref_wait = kRefRetry;
+            return DEM_OK;
+        }
         done = c.steps_done;
     }
 }

@@ -1,5 +1,5 @@
 """The rebuild-every-step loop (dem_refloop.cuh) where it cannot go on: tables that cannot be had, cells
-that fill up in the middle of a run.  The graph of build and step kernels
+that fill up in the middle of a run or in every step.  The graph of build and step kernels
 (cooperative_loop 2) takes the steps left, with the same results."""
 import numpy as np
 import pytest
@@ -37,6 +37,25 @@ def test_no_memory_for_the_tables(nth):
         assert np.array_equal(x, y)
     s.close()
     ctx.close()
+
+
+def test_full_cells_are_not_tried_in_every_run():
+    """Some 20 spheres in a cell: the loop takes no step, and runs of one step go straight to the graph
+    after one that found that out."""
+    sc = _box(900, 6e-3)
+    out = []
+    for coop in (0, 2):
+        s = api.from_scenario(sc, rebuild_every_step=True, cooperative_loop=coop, max_neighbors=128)
+        s.run_steps(1)
+        before = s.stats()["launches"]
+        for _ in range(33):
+            s.run_steps(1)
+        assert s.stats()["cooperative_loop"] == 0
+        out.append((s.stats()["launches"] - before, _state(s)))
+    (la, a), (lb, b) = out
+    assert lb < la <= lb + 2 * 6   # an attempt is six launches; one in every 17 runs
+    for x, y in zip(a, b):
+        assert np.array_equal(x, y)
 
 
 def test_a_cell_that_fills_up_in_the_middle_of_a_run():
