@@ -108,6 +108,8 @@ struct dem_solver {
     bool quiet = false;                         // the current list's build found a quiet system
     int rest = 0;                               // its particles that are not quiet
     int quiet_wait = 0;                         // builds until quiet classes are tried again
+    long quiet_from = 0;                        // total steps at the build that found it
+    double quiet_left = 0.0;                    // steps the classes are expected to last from here
     bool live_off = false;                      // the last step was too dense for several particles per thread
     RefTables ref{};                            // cell tables of the rebuild-every-step loop
     bool ref_refused = false;                   // they could not be allocated
@@ -1154,10 +1156,12 @@ int check_walls(dem_solver *s) {
 // the classes valid longer (a build is needed when the displacement bound reaches half of it), a
 // smaller one leaves fewer particles to step one by one.
 constexpr double kQuietGap = 0.25;
-constexpr int kQuietMinSteps = 64;   // steps a build has to last to be worth its classes
+constexpr int kQuietMinSteps = 64;   // steps a build has to last to be worth its classes: looked at with the
+                                     // largest speed of all particles at the build, and when it is stale
 constexpr int kQuietRetry = 16;      // builds until a system found not quiet is looked at again
 constexpr int kFlightSteps = 64;     // steps of the others per flight of the quiet ones
-constexpr int kFlightBatch = 16;     // flights queued before the host reads the control word
+constexpr int kFlightBatch = 16;     // most flights queued before the host reads the control word; fewer when
+                                     // the classes are expected to be stale before
 
 // kernels issued by one launch_build (see dem_nbr.cu)
 long build_kernel_count(bool resort) { return 13 + (resort ? 7 : 0); }
@@ -1231,11 +1235,14 @@ int build_with(dem_solver *s, bool resort, double delta, double skin) {
             s->built = true;
             s->p->dirty = false;
             if (quiet) {
-                double vq2;
-                std::memcpy(&vq2, &c.vq2, sizeof vq2);
+                // a few fast particles among the others end the classes as soon as fast quiet ones do
+                const unsigned long long b2 = std::max(c.vq2, c.vr2);
+                double v2;
+                std::memcpy(&v2, &b2, sizeof v2);
                 const int rest = s->p->P.n - c.nlone - c.nclear;
-                s->quiet = rest <= live_capacity(s->fc.mixed != 0) &&
-                           kQuietMinSteps * s->sp.dt * std::sqrt(vq2) < 0.5 * cc.gap;
+                s->quiet_left = 0.5 * cc.gap / (s->sp.dt * std::sqrt(v2));
+                s->quiet = rest <= live_capacity(s->fc.mixed != 0) && s->quiet_left > kQuietMinSteps;
+                s->quiet_from = c.total_steps;
                 s->rest = rest;
                 if (!s->quiet) s->quiet_wait = kQuietRetry;
             }
@@ -1844,7 +1851,9 @@ extern "C" int dem_solver_run(dem_solver *s, int nsteps) {
                 if (!s->d_coop) CK(dalloc(&s->d_coop, (size_t)kCoopScratch));
                 const int done_before = s->graph_done_mark, left = nsteps - done_before;
                 CK(cudaEventRecord(s->ev0, st));
-                for (int b = 0; b < kFlightBatch && b * kFlightSteps < left; ++b) {
+                const double want = std::min((double)left, s->quiet_left) / kFlightSteps;
+                const int flights = std::min(kFlightBatch, 1 + (int)std::min(want, (double)kFlightBatch));
+                for (int b = 0; b < flights && b * kFlightSteps < left; ++b) {
                     const cudaError_t le = launch_steps_live(s->p->P, s->L, s->p->ctl, s->fc, s->d_pp, s->d_pw,
                                                              s->d_walls, s->rest, kFlightSteps, s->d_coop, 1,
                                                              s->p->P.n, st);
@@ -1870,8 +1879,12 @@ extern "C" int dem_solver_run(dem_solver *s, int nsteps) {
                     s->graph_done_mark = c.steps_done;
                     steps_before = c.steps_done;
                 }
+                const double until = std::min(c.half_skin, c.clear_until);
+                const long lasted = c.total_steps - s->quiet_from;
+                s->quiet_left = lasted > 0 ? (until - c.disp) * lasted / c.disp : s->quiet_left;
                 if (c.steps_done >= c.target) break;
-                if (s->quiet && !(c.disp < std::min(c.half_skin, c.clear_until))) {
+                if (s->quiet && !(c.disp < until)) {
+                    if (lasted < kQuietMinSteps) s->quiet_wait = kQuietRetry;
                     int e = build_now(s, true);
                     if (e) return e;
                 }

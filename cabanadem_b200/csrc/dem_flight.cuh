@@ -29,21 +29,27 @@
 namespace b200dem {
 namespace {
 
-__device__ __forceinline__ void fold_vq2(Ctl *ctl, double v2) {
+__device__ __forceinline__ void fold_v2(unsigned long long *word, double v2) {
     for (int o = 16; o > 0; o >>= 1) v2 = fmax(v2, __shfl_xor_sync(0xffffffffu, v2, o));
     const unsigned long long b = (unsigned long long)__double_as_longlong(v2);
-    if ((threadIdx.x & 31) == 0 && b > *reinterpret_cast<volatile unsigned long long *>(&ctl->vq2)) atomicMax(&ctl->vq2, b);
+    if ((threadIdx.x & 31) == 0 && b > *reinterpret_cast<volatile unsigned long long *>(word)) atomicMax(word, b);
 }
 
 __global__ void __launch_bounds__(kBlock) k_quiet_begin(Particles P, Ctl *ctl) {
     const int cur = ctl->cur, vcur = ctl->vcur, nq = ctl->nlone + ctl->nclear, cap = P.cap;
-    double v2 = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nq; i += gridDim.x * blockDim.x) {
-        st4(P.pos[cur ^ 1], i, ld4(P.pos[cur], i));
+    double vq = 0.0, vr = 0.0;   // of the quiet ones, of the others
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P.n; i += gridDim.x * blockDim.x) {
         const double a = P.vel[vcur][i], b = P.vel[vcur][cap + i], c = P.vel[vcur][2 * cap + i];
-        v2 = fmax(v2, a * a + b * b + c * c);
+        const double v2 = a * a + b * b + c * c;
+        if (i < nq) {
+            st4(P.pos[cur ^ 1], i, ld4(P.pos[cur], i));
+            vq = fmax(vq, v2);
+        } else {
+            vr = fmax(vr, v2);
+        }
     }
-    fold_vq2(ctl, v2);
+    fold_v2(&ctl->vq2, vq);
+    fold_v2(&ctl->vr2, vr);
 }
 
 __global__ void __launch_bounds__(256) k_flight(Particles P, Ctl *ctl, ForceConsts fc) {
@@ -90,7 +96,7 @@ __global__ void __launch_bounds__(256) k_flight(Particles P, Ctl *ctl, ForceCons
         for (int d = 0; d < 3; ++d) vel[d * cap + i] = u[d];
         v2 = fmax(v2, u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
     }
-    fold_vq2(ctl, v2);
+    fold_v2(&ctl->vq2, v2);
 }
 
 }  // namespace

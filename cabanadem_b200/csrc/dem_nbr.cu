@@ -665,6 +665,7 @@ __global__ void __launch_bounds__(kPartBlock) k_part_place(int n, const int *cls
 __global__ void k_build_begin(Ctl *ctl) {
     if (threadIdx.x == 0) {
         ctl->vq2 = 0ull;
+        ctl->vr2 = 0ull;
         ctl->max_nbr = 0;
         ctl->nlone = 0;
         ctl->nclear = 0;

@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(kBlock) k_prologue(Particles P, Ctl *ctl, Forc
         if (i < nq) vq2 = fmax(vq2, v2);
         st4(P.pos[nxt], i, p);
     }
-    fold_vq2(ctl, vq2);
+    fold_v2(&ctl->vq2, vq2);
     finish_step(ctl, P.vslots, vmax2, fc.dt, 0, false, false, &fc);
 }
 
