@@ -1156,8 +1156,11 @@ int check_walls(dem_solver *s) {
 // the classes valid longer (a build is needed when the displacement bound reaches half of it), a
 // smaller one leaves fewer particles to step one by one.
 constexpr double kQuietGap = 0.25;
-constexpr int kQuietMinSteps = 64;   // steps a build has to last to be worth its classes: looked at with the
-                                     // largest speed of all particles at the build, and when it is stale
+constexpr int kQuietMinSteps = 64;   // steps the quiet particles' speed at a build has to leave its classes
+// Steps the classes have to last to be worth three more builds in the time of one without them: looked at
+// with the largest speed of all particles at the build, and again when they are stale.  A build is 0.2 ms +
+// 0.45 ns per particle, the steps' gain 15 to 45 us (B200): some 10 to 20 steps.
+constexpr int kQuietLast = 24;
 constexpr int kQuietRetry = 16;      // builds until a system found not quiet is looked at again
 constexpr int kFlightSteps = 64;     // steps of the others per flight of the quiet ones
 constexpr int kFlightBatch = 16;     // most flights queued before the host reads the control word; fewer when
@@ -1235,13 +1238,14 @@ int build_with(dem_solver *s, bool resort, double delta, double skin) {
             s->built = true;
             s->p->dirty = false;
             if (quiet) {
-                // a few fast particles among the others end the classes as soon as fast quiet ones do
-                const unsigned long long b2 = std::max(c.vq2, c.vr2);
-                double v2;
-                std::memcpy(&v2, &b2, sizeof v2);
+                // fast particles among the others end the classes as fast quiet ones do
+                double vq2, vr2;
+                std::memcpy(&vq2, &c.vq2, sizeof vq2);
+                std::memcpy(&vr2, &c.vr2, sizeof vr2);
                 const int rest = s->p->P.n - c.nlone - c.nclear;
-                s->quiet_left = 0.5 * cc.gap / (s->sp.dt * std::sqrt(v2));
-                s->quiet = rest <= live_capacity(s->fc.mixed != 0) && s->quiet_left > kQuietMinSteps;
+                s->quiet_left = 0.5 * cc.gap / (s->sp.dt * std::sqrt(std::max(vq2, vr2)));
+                s->quiet = rest <= live_capacity(s->fc.mixed != 0) && s->quiet_left > kQuietLast &&
+                           kQuietMinSteps * s->sp.dt * std::sqrt(vq2) < 0.5 * cc.gap;
                 s->quiet_from = c.total_steps;
                 s->rest = rest;
                 if (!s->quiet) s->quiet_wait = kQuietRetry;
@@ -1884,7 +1888,7 @@ extern "C" int dem_solver_run(dem_solver *s, int nsteps) {
                 s->quiet_left = lasted > 0 ? (until - c.disp) * lasted / c.disp : s->quiet_left;
                 if (c.steps_done >= c.target) break;
                 if (s->quiet && !(c.disp < until)) {
-                    if (lasted < kQuietMinSteps) s->quiet_wait = kQuietRetry;
+                    if (lasted < kQuietLast) s->quiet_wait = kQuietRetry;
                     int e = build_now(s, true);
                     if (e) return e;
                 }
