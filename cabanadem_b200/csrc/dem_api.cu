@@ -1094,7 +1094,18 @@ __global__ void k_clear_status(Ctl *ctl, int bits) {
 
 bool ref_mode(const dem_solver *s) { return s->sp.rebuild_every_step != 0; }
 
-// Kernels of the next graph.  Up to kOneKernelMaxN particles: always the one-kernel step (the
+// Largest system whose step is always one kernel: with static walls and no mesh the particles resident at
+// once (dem_live.cuh), since one more block of the kernel waits for a free place and doubles the step
+// (B200, 57,001 particles, FP64, device us per step, one kernel / three: packings with 24 % in contact 58.7 /
+// 43.6, with 59 % 74.7 / 44.5, a column of disks 48.4 / 30.2; FP32 forces 43.6 / 37.5, 56.4 / 43.7, 30.8 / 29.4).
+// A mesh, moving walls and the rebuild-every-step mode have cooperative loops of their own up to
+// kOneKernelMaxN.
+int one_kernel_max(const dem_solver *s) {
+    const bool resident = !ref_mode(s) && !s->fc.mwalls && s->mesh_nt == 0 && s->sp.dense_form == 0 && s->sp.stream_split == 0;
+    return resident ? std::min(live_capacity(s->fc.mixed != 0), kOneKernelMaxN) : kOneKernelMaxN;
+}
+
+// Kernels of the next graph.  Up to one_kernel_max particles: always the one-kernel step (the
 // three-kernel step is launch-bound there; B200, 4,096 spheres in a walled box: 16.8 -> 10.6 us
 // per step).  Larger, few particles in contact (a sparse step): streaming kernel,
 // cooperative contact kernel, apply kernel; the cooperative kernel's short dependent chains
@@ -1114,20 +1125,21 @@ void pick_contact_kernel(dem_solver *s) {
         s->fc.coop = fits ? req : 0;
     } else {
         // small systems are launch-bound: one kernel per step whatever the density
-        const bool one = s->fc.dense || s->p->P.n <= kOneKernelMaxN;
+        const int most = one_kernel_max(s);
+        const bool one = s->fc.dense || s->p->P.n <= most;
         s->fc.all = one ? 1 : 0;
         s->fc.coop = (!one && fits) ? 8 : 0;
         // a dense step of a larger system: the pair-parallel form, unless the caller asked for
         // the one-kernel form (dense_form 1); dense_form 2 uses it at every size and density
         const int df = s->sp.dense_form;
-        if ((one && df == 0 && s->p->P.n > kOneKernelMaxN) || df == 2) s->fc.all = 2;
+        if ((one && df == 0 && s->p->P.n > most) || df == 2) s->fc.all = 2;
     }
 }
 
 // Whether the kernel forms depend on the density: not for small systems (one kernel per step
 // at any density) nor for a pair-parallel step the caller forced (dense_form 2).
 bool density_matters(const dem_solver *s) {
-    return s->fc.all == 0 || (s->p->P.n > kOneKernelMaxN && s->sp.dense_form != 2);
+    return s->fc.all == 0 || (s->p->P.n > one_kernel_max(s) && s->sp.dense_form != 2);
 }
 
 // Pick the contact-kernel build for the next graph from the last step's deferred count: the
@@ -1645,8 +1657,7 @@ bool live_form(const dem_solver *s) {
 }
 // Particles in contact above which a step is not taken from memory by several per thread: their contacts
 // would follow one another in a thread.  Below it the loop is the faster one at every size it takes (device
-// us per step, three kernels / this loop, 176,000 spheres in scenes 25 / 14.4); a column with nearly all of
-// 65,000 disks in contact takes 54 us in one kernel per step and 66 with several per thread.
+// us per step, three kernels / this loop, 176,000 spheres in scenes 25 / 14.4).
 int live_dense(const dem_solver *s) { return s->p->P.n / 16; }
 
 // The run's steps in cooperative launches (dem_persist.cuh) rather than graph replays: the
@@ -1655,8 +1666,6 @@ int live_dense(const dem_solver *s) { return s->p->P.n / 16; }
 bool coop_loop(const dem_solver *s) {
     if (s->sp.cooperative_loop == 2 || s->coop_refused || !s->loop || ref_mode(s)) return false;
     if (s->fc.all == 1 && s->p->P.n <= kCoopMaxN) {
-        // dense and larger than one particle per resident thread: one kernel per step in a graph (a
-        // column of 65,000 disks, FP64 / FP32 forces: 54 / 32 us per step, 66 / 51 in one cooperative launch)
         return s->fc.mwalls || s->mesh_nt > 0 || live_form(s);
     }
     // larger sparse systems, several particles per thread (dem_live.cuh)
