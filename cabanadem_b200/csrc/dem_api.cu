@@ -111,6 +111,7 @@ struct dem_solver {
     long quiet_from = 0;                        // total steps at the build that found it
     double quiet_left = 0.0;                    // steps the classes are expected to last from here
     bool live_off = false;                      // the last step was too dense for several particles per thread
+    double listed = 0.0;                        // list entries of the last re-sorting build
     RefTables ref{};                            // cell tables of the rebuild-every-step loop
     bool ref_refused = false;                   // they could not be allocated
     int ref_wait = 0;                           // runs until the loop is tried again (kRefRetry)
@@ -1249,6 +1250,7 @@ int build_with(dem_solver *s, bool resort, double delta, double skin) {
             }
             s->built = true;
             s->p->dirty = false;
+            s->listed = (double)c.listed;
             if (quiet) {
                 // fast particles among the others end the classes as fast quiet ones do
                 double vq2, vr2;
@@ -1656,9 +1658,17 @@ bool live_form(const dem_solver *s) {
            (s->p->P.n <= one || (s->p->P.n <= kLiveMany * one && !s->live_off));
 }
 // Particles in contact above which a step is not taken from memory by several per thread: their contacts
-// would follow one another in a thread.  Below it the loop is the faster one at every size it takes (device
-// us per step, three kernels / this loop, 176,000 spheres in scenes 25 / 14.4).
-int live_dense(const dem_solver *s) { return s->p->P.n / 16; }
+// follow one another in a thread, and the more particles a thread has and the longer their lists, the longer
+// its gathers take.  Runs of 150 steps on lattices squeezed by 2 %, us per step with their builds, at most
+// 1/16 of the particles in contact / 1/32 / three kernels throughout (B200, FP64; listed partners each):
+//   two per thread: 113,000 with 2.2 30.9 / 35.5 / 35.6, with 7 34.0 / 36.1 / 36.3;
+//   three: 150,001 with 2.2 31.3 / 36.7 / 36.7, with 4.6 38.5 / 35.9 / 36.1, with 7 42.7 / 37.8 / 37.7;
+//   four: 227,000 with 0.8 38.6 / - / 43.0, with 2.2 47.1 / 44.1 / 43.6, with 7 48.9 / 46.6 / 46.7.
+int live_dense(const dem_solver *s) {
+    const int n = s->p->P.n, one = live_capacity(s->fc.mixed != 0);
+    const bool thick = n > 3 * one ? s->listed > 1.5 * n : n > 2 * one && s->listed > 4.0 * n;
+    return n / (thick ? 32 : 16);
+}
 
 // The run's steps in cooperative launches (dem_persist.cuh) rather than graph replays: the
 // one-kernel step of a small system in the Verlet-skin mode, with the step loop in while-loop

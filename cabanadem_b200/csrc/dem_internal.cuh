@@ -53,6 +53,7 @@ struct Ctl {
     double clear_until;       // displacement bound up to which the particles [0, nlone + nclear) are clear
     unsigned long long vq2;   // bound on |u|^2 of the quiet particles (double bits)
     unsigned long long vr2;   // largest |u|^2 of the others at the build
+    unsigned long long listed;   // list entries of all particles (a build that re-sorts)
     int flight_cur;           // position buffer the quiet particles are in
     int flight_steps;         // steps the others were advanced from there
     int flight_last;          // 1: the last of them was the run's last

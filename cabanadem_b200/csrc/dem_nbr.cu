@@ -567,22 +567,25 @@ __global__ void __launch_bounds__(kPartBlock) k_part_list(Particles P, NbrList L
         c_s = !cc.on ? 2 : (cc.walls && near) ? 2 : count == 0 ? 0 : (near ? 2 : 1);
     }
     if (s < n) cls[s] = c_s;
-    __shared__ int cnt[2];
+    __shared__ int cnt[3];   // classes 0 and 1, list entries
     __shared__ int smax;
-    if (threadIdx.x < 2) cnt[threadIdx.x] = 0;
+    if (threadIdx.x < 3) cnt[threadIdx.x] = 0;
     if (threadIdx.x == 0) smax = 0;
     __syncthreads();
     const int w0 = __popc(__ballot_sync(0xffffffffu, s < n && c_s == 0));
     const int w1 = __popc(__ballot_sync(0xffffffffu, s < n && c_s == 1));
+    const int w2 = (int)__reduce_add_sync(0xffffffffu, (unsigned)count);
     if ((threadIdx.x & 31) == 0) {
         if (w0) atomicAdd(&cnt[0], w0);
         if (w1) atomicAdd(&cnt[1], w1);
+        if (w2) atomicAdd(&cnt[2], w2);
     }
     atomicMax(&smax, count);
     __syncthreads();
     if (threadIdx.x < 2) sums[threadIdx.x * (nb + 1) + blockIdx.x] = cnt[threadIdx.x];
     if (threadIdx.x == 0) {
         atomicMax(&ctl->max_nbr, smax);
+        if (cnt[2]) atomicAdd(&ctl->listed, (unsigned long long)cnt[2]);
         if (smax > L.maxnb || smax > kMaxCand) atomicOr(&ctl->status, DEM_ERR_NEIGHBOR_OVERFLOW);
     }
 }
@@ -666,6 +669,7 @@ __global__ void k_build_begin(Ctl *ctl) {
     if (threadIdx.x == 0) {
         ctl->vq2 = 0ull;
         ctl->vr2 = 0ull;
+        ctl->listed = 0ull;
         ctl->max_nbr = 0;
         ctl->nlone = 0;
         ctl->nclear = 0;

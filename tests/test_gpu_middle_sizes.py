@@ -54,3 +54,17 @@ def test_a_dense_step_above_the_resident_size_is_three_kernels():
         launches[n] = (b["launches"] - a["launches"] - 20 * (b["rebuilds"] - a["rebuilds"])) / 30
         s.close()
     assert launches[56_832] < 2.5 and 3.0 <= launches[56_900] < 4.5
+
+
+@pytest.mark.parametrize("skin,loop", [(1e-4, 1), (2e-4, 0)], ids=["thin", "thick"])
+def test_long_lists_leave_the_loop_with_fewer_contacts(skin, loop):
+    """Four particles per thread, between a 32nd and a 16th of them in contact: the several-per-thread loop
+    with less than one listed partner each, the three-kernel step with two."""
+    sc = _box(200_003, 0.98, skin)
+    sc.state.u[:] = 0.0
+    s = api.from_scenario(sc)
+    s.run_steps(30)
+    s.run_steps(10)
+    share = (s.particles.get("tng_count") > 0).mean()
+    assert 1 / 32 < share < 1 / 16
+    assert s.stats()["cooperative_loop"] == loop
