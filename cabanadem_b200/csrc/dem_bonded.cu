@@ -415,6 +415,7 @@ __global__ void __launch_bounds__(kBondBlock, 4) k_bond_step_tile(Particles P, B
         uint64_t *bar = &full[k % kBondRing];
         const long row = (long)k * cap + i0;
         bulk::bar_arrive_expect(bar, m * (9u * (uint32_t)sizeof(R) + 8u + 4u + 1u));
+        if (fc.drop_copies) return;   // testing the bounded waits: nothing will arrive
         bulk::copy_g2s(s + BT::IDX, B.idx + row, 4u * m, bar);
         bulk::copy_g2s(s + BT::BROKEN, B.broken + row, m, bar);
         bulk::copy_g2s(s + BT::LEN, B.init_len + row, 8u * m, bar);
@@ -451,9 +452,10 @@ __global__ void __launch_bounds__(kBondBlock, 4) k_bond_step_tile(Particles P, B
         const int j = reinterpret_cast<const int *>(s + BT::IDX)[threadIdx.x];
         return s[BT::BROKEN + threadIdx.x] ? -1 : j;
     };
+    const int limit = fc.wait_polls > 0 ? fc.wait_polls : kBondWaitLimit;
     int k = 0;
     for (; k < slots; ++k) {
-        ok = ok && bulk::bar_wait(&full[k % kBondRing], (k / kBondRing) & 1, kBondWaitLimit);
+        ok = ok && bulk::bar_wait(&full[k % kBondRing], (k / kBondRing) & 1, limit);
         const int j = ok ? partner_of(k) : -1;
         BondPartner q = {};
         if (j >= 0) q = bond_partner(pc, vc, wc, cap, j);
@@ -489,7 +491,7 @@ __global__ void __launch_bounds__(kBondBlock, 4) k_bond_step_tile(Particles P, B
     if (__syncthreads_or(ok ? 0 : 1)) {   // report, and let the copies in flight land before the block leaves
         if (threadIdx.x == 0) atomicOr(&ctl->status, DEM_ERR_TIMEOUT);
         for (int r = min(k, slots - 1); r < min(slots, k + kBondRing); ++r)
-            bulk::bar_wait(&full[r % kBondRing], (r / kBondRing) & 1, kBondWaitLimit);
+            bulk::bar_wait(&full[r % kBondRing], (r / kBondRing) & 1, limit);
         return;
     }
     if (have)
@@ -609,7 +611,7 @@ __global__ void __launch_bounds__(kBondBlock, 4) k_bond_loop(Particles P, Bonds 
         }
         unsigned long long big;
         int total;
-        ok = grid_step<kBondBlock>(bar, ctl, scratch, s, v2, 0, big, total);
+        ok = grid_step<kBondBlock>(bar, ctl, fc, scratch, s, v2, 0, big, total);
         if (!ok) break;
         disp = disp + fc.dt * sqrt(__longlong_as_double((long long)big)) * (1.0 + 1e-9);
         cur ^= 1;

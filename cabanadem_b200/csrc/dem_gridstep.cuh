@@ -48,11 +48,14 @@ __device__ __forceinline__ unsigned long long warp_max_bits(double v) {
 
 // Step k (0, 1, ... of the launch) ends: v2 >= 0 of the thread, count of the warp (the same in its
 // lanes).  Returns false when the wait gave up (DEM_ERR_TIMEOUT is set); else `big` holds the bits of
-// the grid's largest v2 and `total` the sum of the counts.
+// the grid's largest v2 and `total` the sum of the counts.  fc: the wait's limit, and whether blocks
+// leave out their arrival, for testing it (dem_solver_debug_stream_waits).
 template <int BLOCK>
-__device__ __forceinline__ bool grid_step(GridStep<BLOCK> &s, Ctl *ctl, unsigned long long *scratch, int k, double v2,
-                                          int count, unsigned long long &big, int &total) {
+__device__ __forceinline__ bool grid_step(GridStep<BLOCK> &s, Ctl *ctl, const ForceConsts &fc, unsigned long long *scratch,
+                                          int k, double v2, int count, unsigned long long &big, int &total) {
     constexpr int W = BLOCK / 32;
+    const unsigned long long one = fc.drop_copies ? 0ull : 1ull;
+    const int limit = fc.wait_polls > 0 ? fc.wait_polls : kGridStepPolls;
     const unsigned long long vb = warp_max_bits(v2);
     if ((threadIdx.x & 31) == 0) {
         s.vmax[threadIdx.x >> 5] = vb;
@@ -73,13 +76,13 @@ __device__ __forceinline__ bool grid_step(GridStep<BLOCK> &s, Ctl *ctl, unsigned
         }
         if (vm) atomicMax(&slot[1], vm);
         // the block's writes before its arrival
-        asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(slot), "l"(1ull + ((unsigned long long)c << 32))
+        asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(slot), "l"(one + ((unsigned long long)c << 32))
                      : "memory");
         unsigned long long arr, v;
         int p = 0;
         do ld_acquire_b128(slot, arr, v);
-        while ((unsigned)arr < gridDim.x && ++p < kGridStepPolls);
-        if (p == kGridStepPolls) {
+        while ((unsigned)arr < gridDim.x && ++p < limit);
+        if (p == limit) {
             atomicOr(&ctl->status, DEM_ERR_TIMEOUT);
             arr = ~0ull;
         }

@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_steps_live(Particles P, NbrList L
         const unsigned busy = __ballot_sync(0xffffffffu, full);
         if (status) atomicOr(&ctl->status, status);
         unsigned long long big;
-        ok = grid_step<kBlock>(bar, ctl, scratch, k, v2, __popc(busy), big, ncon);
+        ok = grid_step<kBlock>(bar, ctl, fc, scratch, k, v2, __popc(busy), big, ncon);
         if (!ok) break;
         double v = sqrt(__longlong_as_double((long long)big));
         if (quiet) v = fmax(v, vq + (k + 1) * fc.dt * ga * (1.0 + 1e-9));
@@ -499,7 +499,7 @@ __global__ void __launch_bounds__(kBlock, 3) k_steps_live_many(Particles P, NbrL
         }
         if (status) atomicOr(&ctl->status, status);
         unsigned long long big;
-        ok = grid_step<kBlock>(bar, ctl, scratch, k, vmax, busy, big, ncon);
+        ok = grid_step<kBlock>(bar, ctl, fc, scratch, k, vmax, busy, big, ncon);
         if (!ok) break;
         double v = sqrt(__longlong_as_double((long long)big));
         if (quiet) v = fmax(v, vq + (k + 1) * fc.dt * ga * (1.0 + 1e-9));

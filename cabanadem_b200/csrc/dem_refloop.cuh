@@ -79,7 +79,8 @@ __global__ void k_ref_enter(Particles P, const Ctl *ctl, RefTables R, unsigned l
 // Returns false when some block asked to stop before it, or when the wait gave up.  The low half
 // of the arrival word counts arrivals; bit 62 + (b & 1) is the stop request of barrier b (a block
 // may already be one barrier ahead of one that still polls, so the two need bits of their own).
-__device__ __forceinline__ bool ref_barrier(Ctl *ctl, unsigned long long *arrive, unsigned b, bool stop) {
+// fc: as for grid_step.
+__device__ __forceinline__ bool ref_barrier(Ctl *ctl, const ForceConsts &fc, unsigned long long *arrive, unsigned b, bool stop) {
     __shared__ int s_go;
     const int any = __syncthreads_or(stop ? 1 : 0);
     if (gridDim.x == 1) return !any;   // one block: its own barrier is the grid's
@@ -88,13 +89,15 @@ __device__ __forceinline__ bool ref_barrier(Ctl *ctl, unsigned long long *arrive
         const int bit = 62 + (int)(b & 1);
         unsigned long long v;
         if (any) atomicOr(arrive, 1ull << bit);
-        asm volatile("atom.release.gpu.global.add.u64 %0, [%1], 1;" : "=l"(v) : "l"(arrive) : "memory");
+        asm volatile("atom.release.gpu.global.add.u64 %0, [%1], %2;"
+                     : "=l"(v) : "l"(arrive), "l"(fc.drop_copies ? 0ull : 1ull) : "memory");
+        const int limit = fc.wait_polls > 0 ? fc.wait_polls : kCoopWaitPolls;
         int k = 0;
         do {
             asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(arrive) : "memory");
-        } while ((unsigned)v < want && ++k < kCoopWaitPolls);
+        } while ((unsigned)v < want && ++k < limit);
         int go = ((v >> bit) & 1) == 0;
-        if (k == kCoopWaitPolls) {
+        if (k == limit) {
             atomicOr(&ctl->status, DEM_ERR_TIMEOUT);
             go = 0;
         }
@@ -131,7 +134,7 @@ __global__ void __launch_bounds__(RefShape<NL>::block, RefShape<NL>::min_blocks)
     const int target = ctl->target;
     unsigned bar = 0;
     bool go = !(ctl->status & (kStopBits | DEM_ERR_NAN)) && !((*arrive >> 62) & 1);
-    go = ref_barrier(ctl, arrive, bar++, !go);
+    go = ref_barrier(ctl, fc, arrive, bar++, !go);
     int steps = 0, status = 0;
     // at most 2^31 - 1 arrivals per launch (the host goes on with another)
     const int kmax = min(max_steps, (int)(0x7fffffffu / gridDim.x) - 2);
@@ -259,7 +262,7 @@ __global__ void __launch_bounds__(RefShape<NL>::block, RefShape<NL>::min_blocks)
             }
             __syncwarp();
         }
-        go = ref_barrier(ctl, arrive, bar++, stop);
+        go = ref_barrier(ctl, fc, arrive, bar++, stop);
         cur ^= 1;
         vcur ^= 1;
         done += 1;

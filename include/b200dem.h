@@ -441,11 +441,12 @@ int dem_nn_status(dem_ctx *ctx, int *status);
  * and sets DEM_ERR_TIMEOUT in the word dem_nn_status returns.  The setting is per device and
  * process-wide; it takes effect for kernels queued after the call. */
 int dem_nn_debug_waits(dem_ctx *ctx, int poll_limit, int drop_mma);
-/* Bounds of the staged streaming kernel's waits (stream_split 4), for testing that a wait which
- * runs out stops the run with DEM_ERR_TIMEOUT and leaves the context usable (no reference
- * counterpart).  poll_limit: polls of a tile's copy barrier per wait (0 = the default, about
- * 260,000); drop_copies != 0: the kernel arms its barriers but issues no copy, so every wait
- * runs out with nothing in flight.  A run then returns DEM_ERR_TIMEOUT with its step
+/* Bounds of the waits of the staged kernels (streaming step with stream_split 4, bonded step) and of
+ * the cooperative step loops with static walls and no mesh, bonded runs among them, for testing that a
+ * wait which runs out stops the run with DEM_ERR_TIMEOUT and leaves the context usable (no reference
+ * counterpart).  poll_limit: polls per wait (0 = the defaults, 260,000 of a tile's copy barrier,
+ * millions of a grid barrier); drop_copies != 0: staged kernels arm their barriers but issue no copy,
+ * blocks of the loops do not arrive, so every wait runs out with nothing in flight.  A run then returns DEM_ERR_TIMEOUT with its step
  * unfinished (the particle state must be set again).  Calling with drop_copies = 0 also clears
  * the DEM_ERR_TIMEOUT bit of the solver's control word. */
 int dem_solver_debug_stream_waits(dem_solver *s, int poll_limit, int drop_copies);
