@@ -490,7 +490,8 @@ __global__ void __launch_bounds__(kBondBlock, 4) k_bond_step_tile(Particles P, B
     }
     if (__syncthreads_or(ok ? 0 : 1)) {   // report, and let the copies in flight land before the block leaves
         if (threadIdx.x == 0) atomicOr(&ctl->status, DEM_ERR_TIMEOUT);
-        for (int r = min(k, slots - 1); r < min(slots, k + kBondRing); ++r)
+        const int issued = min(slots, k + kBondRing);   // the last copies into each place of the ring
+        for (int r = max(0, issued - kBondRing); r < issued; ++r)
             bulk::bar_wait(&full[r % kBondRing], (r / kBondRing) & 1, limit);
         return;
     }
