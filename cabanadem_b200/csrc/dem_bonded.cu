@@ -743,16 +743,9 @@ void launch_bond_step(const Particles &P, const Bonds &B, Ctl *ctl, const ForceC
 }
 
 template <typename R>
-static int bond_loop_fit() {   // particles resident at once, per host thread
-    static thread_local int fit = 0;
-    if (!fit) {
-        int dev = 0, sms = 0, per = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void *)k_bond_loop<R>, kBondBlock, 0);
-        fit = (sms > 0 ? sms : 148) * (per > 0 ? per : 1) * (kBondBlock / 8);
-    }
-    return fit;
+static int bond_loop_fit() {   // particles resident at once
+    static thread_local PerDevice fit;
+    return resident_blocks(fit, (const void *)k_bond_loop<R>, kBondBlock) * (kBondBlock / 8);
 }
 int bond_loop_capacity(const Bonds &B, const BondConsts &bc, int slots) {
     if (slots > 8 || (bc.quirks & BQ10_INDEX_BY_J)) return 0;

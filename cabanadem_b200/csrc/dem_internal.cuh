@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include "b200dem.h"
+#include "dem_device.cuh"
 
 namespace b200dem {
 
@@ -271,6 +272,19 @@ struct BondConsts {
     unsigned quirks;
     double beta, radius_factor, kn, kt, break_strain;
 };
+
+// Blocks of `kernel` that the current device holds at once.  smem: dynamic shared memory, raised to it first.
+inline int resident_blocks(PerDevice &kept, const void *kernel, int block, int smem = 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return kept.get(dev, [&](int d) {
+        int sms = 0, per = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d);
+        if (smem > 0) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, block, smem);
+        return (sms > 0 ? sms : 148) * (per > 0 ? per : 1);
+    });
+}
 
 // ---- launchers (dem_bonded.cu) ----------------------------------------------------
 void launch_bond_setup(const Particles &P, const NbrList &L, const Bonds &B, Ctl *ctl, double factor, cudaStream_t s);

@@ -534,19 +534,11 @@ __global__ void __launch_bounds__(kBlock, 3) k_steps_live_many(Particles P, NbrL
     }
 }
 
-// Blocks resident at once, per host thread.
+// Blocks resident at once.
 template <bool MIXED>
 static int live_blocks(bool many) {
-    static thread_local int fit[2] = {0, 0};
-    if (!fit[many]) {
-        int dev = 0, sms = 0, per = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per, many ? (const void *)k_steps_live_many<MIXED> : (const void *)k_steps_live<MIXED>, kBlock, 0);
-        fit[many] = (sms > 0 ? sms : 148) * (per > 0 ? per : 1);
-    }
-    return fit[many];
+    static thread_local PerDevice fit[2];
+    return resident_blocks(fit[many], many ? (const void *)k_steps_live_many<MIXED> : (const void *)k_steps_live<MIXED>, kBlock);
 }
 
 template <bool MIXED>

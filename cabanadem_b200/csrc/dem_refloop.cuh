@@ -290,19 +290,11 @@ static cudaError_t steps_ref_t(const Particles &P, const NbrList &L, Ctl *ctl, c
                                const PairConst *pp, const PairConst *pw, const WallGeom *walls, const RefTables &R,
                                double delta, double skin, int max_steps, unsigned long long *arrive, cudaStream_t s) {
     const void *kernel = (const void *)k_steps_ref<NL, MIXED>;
-    static thread_local int fit = 0;   // resident blocks, per host thread
-    if (!fit) {
-        int dev = 0, sms = 0, per = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const int smem = (RefShape<NL>::block / NL) * (int)sizeof(RefGroup);
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, RefShape<NL>::block, smem);
-        fit = (sms > 0 ? sms : 148) * (per > 0 ? per : 1);
-    }
+    static thread_local PerDevice kept;
+    const int smem = (RefShape<NL>::block / NL) * (int)sizeof(RefGroup);
+    const int fit = resident_blocks(kept, kernel, RefShape<NL>::block, smem);
     const int need = (P.n + RefShape<NL>::block / NL - 1) / (RefShape<NL>::block / NL);
     const int grid = need < fit ? need : fit;
-    const int smem = (RefShape<NL>::block / NL) * (int)sizeof(RefGroup);
     cudaError_t e = cudaMemsetAsync(arrive, 0, sizeof(unsigned long long), s);
     if (e == cudaSuccess) e = cudaMemsetAsync(R.count, 0, sizeof(int) * 3 * (size_t)R.codes, s);
     if (e != cudaSuccess) return e;

@@ -737,20 +737,10 @@ constexpr int kBulkT = STREAM_BULK_T, kBulkS = STREAM_BULK_STAGES;
 // Persistent grid of the staged streaming kernel: every block the SMs hold at its shared
 // memory, at most one per tile.
 static int bulk_blocks(int n) {
-    static thread_local int per = -1, sms = 0;
-    if (per < 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms <= 0) sms = 148;
-        const int smem = kBulkS * BulkTile<kBulkT>::BYTES;
-        cudaFuncSetAttribute((const void *)k_stream_bulk<kBulkT, kBulkS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             smem);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_stream_bulk<kBulkT, kBulkS>, kBulkT, smem);
-        if (per <= 0) per = 1;
-    }
+    static thread_local PerDevice kept;
+    const int most = resident_blocks(kept, (const void *)k_stream_bulk<kBulkT, kBulkS>, kBulkT, kBulkS * BulkTile<kBulkT>::BYTES);
     const int tiles = (n + kBulkT - 1) / kBulkT;
-    return std::max(1, std::min(tiles, sms * per));
+    return std::max(1, std::min(tiles, most));
 }
 
 static int persistent_blocks(const void *kernel, int block, int n) {
@@ -881,16 +871,9 @@ static cudaError_t steps_coop_t(const Particles &P, const NbrList &L, Ctl *ctl, 
                                 unsigned long long *scratch, cudaStream_t s) {
     const bool lean = MESH && !fc.mwalls && !fc.mesh_moving && scratch;
     const void *kernel = lean ? (const void *)k_steps_coop_lean<MIXED> : (const void *)k_steps_coop<MIXED, MESH>;
-    static thread_local int fit[2] = {0, 0};   // resident blocks of each form, per host thread
-    if (!fit[lean]) {
-        int dev = 0, sms = 0, per = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, kBlock, 0);
-        fit[lean] = (sms > 0 ? sms : 148) * (per > 0 ? per : 1);
-    }
-    const int need = (P.n + kBlock - 1) / kBlock;
-    int grid = need < fit[lean] ? (need > 0 ? need : 1) : fit[lean];
+    static thread_local PerDevice kept[2];   // of each form
+    const int fit = resident_blocks(kept[lean], kernel, kBlock), need = (P.n + kBlock - 1) / kBlock;
+    int grid = need < fit ? (need > 0 ? need : 1) : fit;
     if (lean && grid > kCoopMaxBlocks) grid = kCoopMaxBlocks;   // the scratch holds that many slots
     Particles p = P;
     NbrList l = L;
