@@ -28,9 +28,9 @@ __device__ __forceinline__ int nth_high_bit(unsigned b, int r) {
     return 31 - __clz(b);
 }
 
-// Where a particle's list comes from: the solver's list arrays, read once through the read-only
-// path (a launch that does one step), or a list the group holds in shared memory, with the
-// particle's own arrays read by plain loads (a launch whose earlier steps wrote them).
+// Where a particle's list comes from: the solver's list arrays, with the particle's own state read once
+// through the read-only path (a launch that does one step), or a list the group holds in shared memory,
+// with the state the caller hands over (a launch whose earlier steps wrote the arrays).
 struct GlobalList {
     static constexpr bool kOneStep = true;
     const NbrList &L;
@@ -46,7 +46,7 @@ struct GroupList {
     __device__ __forceinline__ int at(int, int k) const { return list[k]; }
 };
 
-// A particle's own state where the caller has it already (every lane of the group): a round trip less.
+// A particle's own state, in every lane of the group: the caller has it already, a round trip less.
 struct CoopOwn {
     D4 p;
     double u[3], w[3], m, I;
@@ -65,7 +65,6 @@ __device__ __forceinline__ void particle_coop(const Particles &P, const LIST &li
                                               const int vcur, const int last, const int i, const int t,
                                               int *s_tidx, double *s_h, double *vn, double *wn, double &vmax2,
                                               int &status, D4 *pn_out = nullptr, const CoopOwn *own = nullptr) {
-    constexpr bool ONE = LIST::kOneStep;
     constexpr unsigned FULL = 0xffffffffu;
     constexpr unsigned GLOW = NL == 32 ? 0xffffffffu : ((1u << NL) - 1u);
     const int lane = threadIdx.x & 31, gl = lane % NL, gbase = lane - gl;
@@ -87,28 +86,28 @@ __device__ __forceinline__ void particle_coop(const Particles &P, const LIST &li
     double ui0 = 0., ui1 = 0., ui2 = 0., wi0 = 0., wi1 = 0., wi2 = 0.;
     double2 mIi = make_double2(0., 0.);
     int mi = 0, cs0 = 0, nn = 0;
-    if (act && own) {
-        pi = own->p;
-        ui0 = own->u[0];
-        ui1 = own->u[1];
-        ui2 = own->u[2];
-        wi0 = own->w[0];
-        wi1 = own->w[1];
-        wi2 = own->w[2];
-        mIi = make_double2(own->m, own->I);
-        cs0 = own->cs;
-        nn = list.count(i);
-        mi = fc.nmat > 1 ? (int)P.mat[i] : 0;
-    } else if (act) {
-        pi = ONE ? ld4_early(pc, i) : ld4(pc, i);
-        ui0 = ONE ? ld_early(vc + i) : vc[i];
-        ui1 = ONE ? ld_early(vc + cap + i) : vc[cap + i];
-        ui2 = ONE ? ld_early(vc + 2 * cap + i) : vc[2 * cap + i];
-        wi0 = ONE ? ld_early(wc + i) : wc[i];
-        wi1 = ONE ? ld_early(wc + cap + i) : wc[cap + i];
-        wi2 = ONE ? ld_early(wc + 2 * cap + i) : wc[2 * cap + i];
-        mIi = make_double2(ld_early(P.mI + i), ld_early(P.mI + cap + i));
-        cs0 = ONE ? ld_early_i(P.cstate + i) : P.cstate[i];
+    if (act) {
+        if constexpr (LIST::kOneStep) {
+            pi = ld4_early(pc, i);
+            ui0 = ld_early(vc + i);
+            ui1 = ld_early(vc + cap + i);
+            ui2 = ld_early(vc + 2 * cap + i);
+            wi0 = ld_early(wc + i);
+            wi1 = ld_early(wc + cap + i);
+            wi2 = ld_early(wc + 2 * cap + i);
+            mIi = make_double2(ld_early(P.mI + i), ld_early(P.mI + cap + i));
+            cs0 = ld_early_i(P.cstate + i);
+        } else {
+            pi = own->p;
+            ui0 = own->u[0];
+            ui1 = own->u[1];
+            ui2 = own->u[2];
+            wi0 = own->w[0];
+            wi1 = own->w[1];
+            wi2 = own->w[2];
+            mIi = make_double2(own->m, own->I);
+            cs0 = own->cs;
+        }
         nn = list.count(i);
         mi = fc.nmat > 1 ? (int)P.mat[i] : 0;
     }

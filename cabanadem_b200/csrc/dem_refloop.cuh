@@ -15,8 +15,9 @@
 // needed.  The grid is taken from the positions at the launch; a particle that leaves it counts to
 // the cell at the border (a clamped coordinate never separates two cells that touch, so no pair is
 // missed).  A full cell, a list over the solver's capacity or a position that is not finite ends
-// the launch at the step boundary, and the host goes on with the graph of build and step kernels,
-// which grows the lists or reports the error.  The run's last step writes the lists (all
+// the launch at the step boundary.  The host then makes the lists larger where that is what it takes, and
+// launches again on a fresh grid; a launch that can take no step hands the rest of the run to the graph
+// of build and step kernels, which reports the error if there is one.  The run's last step writes the lists (all
 // candidates within the cutoff) where the build kernels leave them.
 //
 // Measured (B200, FP64, us per step over 1,000 steps, graph / this loop): 2 spheres 37 / 4.2, a dense
