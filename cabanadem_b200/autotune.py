@@ -15,6 +15,9 @@ caller-index order, whatever its cutoff or the re-sort):
 * ``skin``              Verlet skin (0.5, 1, 2 or 4 times the scenario's), i.e. the rebuild cadence
                         against the listed neighbours a streaming pass checks
 
+A ``contact_lanes``, ``dense_form`` or ``stream_split`` other than 0 names the per-step kernels: above
+56,832 particles such a solver takes neither the resident loops nor the flights of quiet particles.
+
 ``tune`` times short runs of the caller's workload for each candidate, one setting at a time
 (coordinate search from the defaults), and caches the winner per size bucket (log2 of the
 particle count, precision, batched or single, and for a batch the scene-size bucket of its
