@@ -1204,6 +1204,9 @@ int build_with(dem_solver *s, bool resort, double delta, double skin) {
         // a solver's run list: with quiet classes (dem_flight.cuh) where those may pay
         ClassSpec cc;
         cc.gap = 0.5 * skin;
+        // for live_dense: an atomic per 256 particles on one word (counted at 2,000,000 too, a build and 1,000
+        // steps took 0.5 % longer)
+        cc.count_listed = s->p->P.n <= kLiveMany * live_capacity(s->fc.mixed != 0);
         bool quiet = false;
         if (resort && delta == s->sp.delta && skin == s->sp.skin && quiet_possible(s)) {
             quiet = s->quiet_wait == 0;

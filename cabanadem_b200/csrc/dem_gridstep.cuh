@@ -39,7 +39,8 @@ __device__ __forceinline__ void ld_acquire_b128(const void *p, unsigned long lon
 // that share the largest high word.  A NaN counts as 0, as in finish_step (its bits would be the largest
 // of all and end the displacement bound): the next list build reports it.
 __device__ __forceinline__ unsigned long long warp_max_bits(double v) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(fmax(v, 0.0));
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
+    const unsigned long long b = (unsigned)(bits >> 32) > 0x7ff00000u ? 0ull : bits;   // past infinity: a NaN
     const unsigned hi = (unsigned)(b >> 32);
     const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
     const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)b : 0u);

@@ -347,6 +347,7 @@ struct ClassSpec {
     double gap = 0.0;                 // a clear particle's listed neighbours all keep a larger gap
     const struct WallGeom *walls = nullptr;   // quiet classes: tracked contacts and near walls count too
     int nwall = 0, wps = 0;
+    bool count_listed = false;       // Ctl::listed too
 };
 void launch_build(const Particles &P, Particles &alt, const NbrList &L, BuildBuffers &B, Ctl *ctl, double delta,
                   double skin, bool resort, bool check_run, cudaStream_t s, const ClassSpec &cc = ClassSpec());

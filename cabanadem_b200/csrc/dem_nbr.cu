@@ -578,14 +578,14 @@ __global__ void __launch_bounds__(kPartBlock) k_part_list(Particles P, NbrList L
     if ((threadIdx.x & 31) == 0) {
         if (w0) atomicAdd(&cnt[0], w0);
         if (w1) atomicAdd(&cnt[1], w1);
-        if (w2) atomicAdd(&cnt[2], w2);
+        if (cc.count_listed && w2) atomicAdd(&cnt[2], w2);
     }
     atomicMax(&smax, count);
     __syncthreads();
     if (threadIdx.x < 2) sums[threadIdx.x * (nb + 1) + blockIdx.x] = cnt[threadIdx.x];
     if (threadIdx.x == 0) {
         atomicMax(&ctl->max_nbr, smax);
-        if (cnt[2]) atomicAdd(&ctl->listed, (unsigned long long)cnt[2]);
+        if (cc.count_listed && cnt[2]) atomicAdd(&ctl->listed, (unsigned long long)cnt[2]);
         if (smax > L.maxnb || smax > kMaxCand) atomicOr(&ctl->status, DEM_ERR_NEIGHBOR_OVERFLOW);
     }
 }
