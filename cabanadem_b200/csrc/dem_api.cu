@@ -108,6 +108,7 @@ struct dem_solver {
     bool quiet = false;                         // the current list's build found a quiet system
     int rest = 0;                               // its particles that are not quiet
     int quiet_wait = 0;                         // builds until quiet classes are tried again
+    int quiet_back = 16;                        // and how many that will be when classes end early (kQuietRetry)
     long quiet_from = 0;                        // total steps at the build that found it
     double quiet_left = 0.0;                    // steps the classes are expected to last from here
     bool live_off = false;                      // the last step was too dense for several particles per thread
@@ -1174,7 +1175,9 @@ constexpr int kQuietMinSteps = 64;   // steps the quiet particles' speed at a bu
 // with the largest speed of all particles at the build, and again when they are stale.  A build is 0.2 ms +
 // 0.45 ns per particle, the steps' gain 15 to 45 us (B200): some 10 to 20 steps.
 constexpr int kQuietLast = 24;
-constexpr int kQuietRetry = 16;      // builds until a system found not quiet is looked at again
+constexpr int kQuietRetry = 16;      // builds until a system found not quiet is looked at again; twice as many
+                                     // after each time that its classes then ended early, up to
+constexpr int kQuietRetryMost = 256; // this many (a packing of 120,000 flying apart: 1.5 % of a run otherwise)
 constexpr int kFlightSteps = 64;     // steps of the others per flight of the quiet ones
 constexpr int kFlightBatch = 16;     // most flights queued before the host reads the control word; fewer when
                                      // the classes are expected to be stale before
@@ -1910,7 +1913,12 @@ extern "C" int dem_solver_run(dem_solver *s, int nsteps) {
                 s->quiet_left = lasted > 0 ? (until - c.disp) * lasted / c.disp : s->quiet_left;
                 if (c.steps_done >= c.target) break;
                 if (s->quiet && !(c.disp < until)) {
-                    if (lasted < kQuietLast) s->quiet_wait = kQuietRetry;
+                    if (lasted < kQuietLast) {
+                        s->quiet_wait = s->quiet_back;
+                        s->quiet_back = std::min(2 * s->quiet_back, kQuietRetryMost);
+                    } else {
+                        s->quiet_back = kQuietRetry;
+                    }
                     int e = build_now(s, true);
                     if (e) return e;
                 }
