@@ -1096,14 +1096,16 @@ __global__ void k_clear_status(Ctl *ctl, int bits) {
 
 bool ref_mode(const dem_solver *s) { return s->sp.rebuild_every_step != 0; }
 
-// Largest system whose step is always one kernel: with static walls and no mesh the particles resident at
-// once (dem_live.cuh), since one more block of the kernel waits for a free place and doubles the step
-// (B200, 57,001 particles, FP64, device us per step, one kernel / three: packings with 24 % in contact 58.7 /
-// 43.6, with 59 % 74.7 / 44.5, a column of disks 48.4 / 30.2; FP32 forces 43.6 / 37.5, 56.4 / 43.7, 30.8 / 29.4).
-// A mesh, moving walls and the rebuild-every-step mode have cooperative loops of their own up to
-// kOneKernelMaxN.
+// Largest system whose step is always one kernel.  Where the resident loops take the sparse steps (dem_live.cuh)
+// the particles resident at once, since one more block of the kernel waits for a free place and doubles the
+// step (B200, 57,001 particles, FP64, device us per step, one kernel / three: packings with 24 % in contact
+// 58.7 / 43.6, with 59 % 74.7 / 44.5, a column of disks 48.4 / 30.2; FP32 forces 43.6 / 37.5, 56.4 / 43.7,
+// 30.8 / 29.4).  Elsewhere kOneKernelMaxN: a mesh, moving walls and the rebuild-every-step mode have
+// cooperative loops of their own, and a sparse step is the faster one in one kernel (graphs alone, FP32
+// forces, nothing in contact 13.6 / 18.3).
 int one_kernel_max(const dem_solver *s) {
-    const bool resident = !ref_mode(s) && !s->fc.mwalls && s->mesh_nt == 0 && s->sp.dense_form == 0 && s->sp.stream_split == 0;
+    const bool resident = s->loop && s->sp.cooperative_loop != 2 && !s->coop_refused && !ref_mode(s) && !s->fc.mwalls &&
+                          s->mesh_nt == 0 && s->sp.dense_form == 0 && s->sp.stream_split == 0;
     return resident ? std::min(live_capacity(s->fc.mixed != 0), kOneKernelMaxN) : kOneKernelMaxN;
 }
 

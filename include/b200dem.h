@@ -130,7 +130,8 @@ typedef struct dem_solver_params {
                             * copies.  Same results.                                           */
     int dense_form;        /* step of a dense flow (most particles in contact, contact_lanes 0):
                             * 0 = automatic (2 above the particles resident at once, 56,832 on
-                            * a B200; above 65,536 with a mesh or moving walls; else 1), 1 one kernel
+                            * a B200; above 65,536 with a mesh, moving walls or without the
+                            * cooperative loops; else 1), 1 one kernel
                             * with a thread per particle, 2 three kernels: contact search per
                             * particle, the pair law per contact, sums and integration per
                             * particle; 2 is also used at every density.  Same results.         */

@@ -44,16 +44,17 @@ def test_forms_agree(n, squeeze, skin, precision):
 
 def test_a_dense_step_above_the_resident_size_is_three_kernels():
     launches = {}
-    for n in (56_832, 56_900):
-        s = api.from_scenario(_box(n, 0.92), cooperative_loop=2)
+    for coop in (0, 2):
+        s = api.from_scenario(_box(56_900, 0.92), cooperative_loop=coop)
         s.run_steps(30)                      # the density is known after some steps
         a = s.stats()
         s.run_steps(30)
         b = s.stats()
+        assert b["cooperative_loop"] == 0
         # without the builds (20 kernels each), the run's two and the loop's control kernels
-        launches[n] = (b["launches"] - a["launches"] - 20 * (b["rebuilds"] - a["rebuilds"])) / 30
+        launches[coop] = (b["launches"] - a["launches"] - 20 * (b["rebuilds"] - a["rebuilds"])) / 30
         s.close()
-    assert launches[56_832] < 2.5 and 3.0 <= launches[56_900] < 4.5
+    assert 3.0 <= launches[0] < 4.5 and launches[2] < 2.5   # graphs alone stay with one kernel
 
 
 @pytest.mark.parametrize("skin,loop", [(1e-4, 1), (2e-4, 0)], ids=["thin", "thick"])
